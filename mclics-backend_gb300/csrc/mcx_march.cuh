@@ -4,6 +4,7 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include "mcx_packed.cuh"
 #include "mcx_pass.cuh"
 
 namespace mcx {
@@ -163,11 +164,13 @@ __device__ __forceinline__ void march_init(const PassArgs &a, const RepDev &R, i
 }
 
 // Resident CTAs per SM the compiler is asked for (measured best): the
-// unmasked Lebwohl-Lasher pass at about 96-113 registers per thread; the GHRL
-// and masked variants at 128 (they spill a little there, and still run 1.5x
-// faster than unconstrained at 160-206 registers, from the doubled occupancy).
+// unmasked Lebwohl-Lasher pass at 96 to 128 registers per thread (five CTAs of
+// 128: at six, 80 registers, the packed update spills 48 to 132 bytes and a
+// 16^3 block of 200 sweeps took 3.59 ms against 2.78); the GHRL and masked
+// variants at 128 (they spill a little there, and still run 1.5x faster than
+// unconstrained at 160-206 registers, from the doubled occupancy).
 #ifndef MCX_MARCH_LL128_BLOCKS
-#define MCX_MARCH_LL128_BLOCKS 6
+#define MCX_MARCH_LL128_BLOCKS 5
 #endif
 #ifndef MCX_MARCH_LL256_BLOCKS
 #define MCX_MARCH_LL256_BLOCKS 2
@@ -181,12 +184,57 @@ constexpr int march_min_blocks() {
                                 : (MCX_MARCH_MASK_REGS > 0 ? 65536 / (NT * MCX_MARCH_MASK_REGS) : 1);
 }
 
+// What a measured pass adds for one site with its final director (the
+// measured part of site_update): eb its bond sum to active neighbours.
+template <int POT, bool MASK, bool FIELD>
+__device__ __forceinline__ void measure_site(const RepDev &R, int c, float x, float y, float z, const float nb[6][3],
+                                             const float w[6], const float e[6], int pself, float sx, float sy,
+                                             float sz, float eb, float qs[kQ]) {
+  const int sid = pself - 2;
+  const bool surf = MASK && pself > 1 && sid < R.nsurf;
+  const float act = pself != 0 ? 1.f : 0.f;
+  if (pself != 0) {
+    qs[2] += x * x;
+    qs[3] += x * y;
+    qs[4] += x * z;
+    qs[5] += y * y;
+    qs[6] += y * z;
+  }
+  if (surf) {
+    const float es = surface_energy(R, sid, x, y, z, sx, sy, sz);
+    qs[0] += es;
+    qs[1] += es;
+  }
+  if (FIELD) {
+    const float ef = field_energy(R, x, y, z);
+    qs[0] += ef;
+    qs[1] += act * ef;
+  }
+  if (c == 1) {
+    if (pself != 0) {
+      const float ebs = bond_scale<POT>(R) * eb + bond_const<POT>(R, w);
+      qs[0] += 2.f * ebs;
+      qs[1] += 2.f * ebs;
+      if (MASK) {
+        float wi[6];
+#pragma unroll
+        for (int d = 0; d < 6; d++) wi[d] = e[d] - w[d];
+        qs[0] += bond_scale<POT>(R) * bond_sum<POT>(R, x, y, z, nb, wi) + bond_const<POT>(R, wi);
+      }
+    } else {
+      qs[0] += bond_scale<POT>(R) * bond_sum<POT>(R, x, y, z, nb, w) + bond_const<POT>(R, w);
+    }
+  }
+}
+
 // The update of one same-colour pair from its loaded neighbourhood (shared by
 // the z-march and its staged and prefetching forms): own directors (ax, ay,
 // az) in and out; o0 the opposite pair of the same row, yp / ym those of rows
 // y+1 / y-1, op / om those of the planes above / below (zp / zm: those bonds
 // exist), exv the extra x neighbour; s the parity of the own sites in this
-// row; rw the pair's Philox draw (pair_draw below).
+// row; rw the pair's Philox draw (pair_draw below).  Both sites run in packed
+// arithmetic (mcx_packed.cuh); a missing, phantom or inactive site's half is
+// computed and dropped.
 template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
 __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev &R, int c, int s, bool hasB_,
                                                  float ee0, float ee1, float eyp, float eym, const OPair &o0,
@@ -195,77 +243,144 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
                                                  const uint4 rw, long long ns_at, float ang, float invT, float2 &ax,
                                                  float2 &ay, float2 &az, unsigned &acc, float qs[kQ],
                                                  int tail = 0) {
-  float uA[3], uB[3];
-  pair_uniforms(rw, uA, uB);
-  auto wt = [&](float ee, uint8_t pp) { return MASK ? (ee != 0.f && pp != 0 ? 1.f : 0.f) : ee; };
-  // PER: every bond exists (all axes periodic, pairs always complete)
-  const float exe = PER ? 1.f : (s ? ee1 : ee0);
-  const float erz[4] = {PER ? 1.f : eyp, PER ? 1.f : eym, PER || zp ? 1.f : 0.f, PER || zm ? 1.f : 0.f};
+  constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
+  constexpr bool W = !PER;  // PER: every bond exists (all axes periodic, pairs always complete)
   const bool hasB = PER || hasB_;
-  const OPair *rows4[4] = {&yp, &ym, &op, &om};
-  const uint8_t lo = (uint8_t)(o0.pt & 0xFF), hi = (uint8_t)(o0.pt >> 8);
-  const int P = R.plane;
-  float nb[6][3], w[6], e[6];
-  // odd nx (masked only): a phantom in the last slot of an s = 1 row is
-  // skipped; the last site of an s = 0 row has no x+ bond
-  const bool skipA = MASK && s == 1 && tail == 1, skipB = MASK && s == 1 && tail == 2;
-  if (!skipA) {  // site A
-    if (s == 0) {
-      nb[0][0] = o0.v[0].x; nb[0][1] = o0.v[1].x; nb[0][2] = o0.v[2].x; e[0] = 1.f; w[0] = wt(1.f, lo);
-      nb[1][0] = exv[0]; nb[1][1] = exv[1]; nb[1][2] = exv[2]; e[1] = exe; w[1] = wt(exe, pex);
-    } else {
-      if (hasB) {
-        nb[0][0] = o0.v[0].y; nb[0][1] = o0.v[1].y; nb[0][2] = o0.v[2].y; e[0] = 1.f; w[0] = wt(1.f, hi);
-      } else {
-        nb[0][0] = exv[0]; nb[0][1] = exv[1]; nb[0][2] = exv[2]; e[0] = exe; w[0] = wt(exe, pex);
-      }
-      nb[1][0] = o0.v[0].x; nb[1][1] = o0.v[1].x; nb[1][2] = o0.v[2].x; e[1] = 1.f; w[1] = wt(1.f, lo);
-    }
-    if (MASK && s == 0 && tail == 1) e[0] = w[0] = 0.f;
+  // neighbour slots x+ x- y+ y- z+ z- of both sites
+  V2 nb[6];
+  f32x2 w[6];
+  {
+    f32x2 q0[3], q1[3];
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const OPair &o = *rows4[q];
-      nb[2 + q][0] = o.v[0].x; nb[2 + q][1] = o.v[1].x; nb[2 + q][2] = o.v[2].x;
-      e[2 + q] = erz[q];
-      w[2 + q] = wt(erz[q], MASK ? (uint8_t)(o.pt & 0xFF) : 1);
+    for (int q = 0; q < 3; q++) {
+      const float lo = o0.v[q].x, hi = o0.v[q].y, ex = exv[q];
+      q0[q] = pk(s ? (hasB ? hi : ex) : lo, s ? ex : hi);
+      q1[q] = pk(s ? lo : ex, s ? hi : lo);
     }
-    const int ps = MASK ? (pself & 0xFF) : 1;
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    if (MASK && ps > 1) {
-      const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * P + ns_at;
-      sx = __ldg(nsb);
-      sy = __ldg(nsb + P);
-      sz = __ldg(nsb + 2 * P);
-    }
-    acc += site_update<POT, MASK, FIELD, MODE>(R, a, c, ax.x, ay.x, az.x, nb, w, e, ps, sx, sy, sz, uA, ang, invT,
-                                               0u, qs);
+    nb[0] = {q0[0], q0[1], q0[2]};
+    nb[1] = {q1[0], q1[1], q1[2]};
+    nb[2] = {pk(yp.v[0]), pk(yp.v[1]), pk(yp.v[2])};
+    nb[3] = {pk(ym.v[0]), pk(ym.v[1]), pk(ym.v[2])};
+    nb[4] = {pk(op.v[0]), pk(op.v[1]), pk(op.v[2])};
+    nb[5] = {pk(om.v[0]), pk(om.v[1]), pk(om.v[2])};
   }
-  if (hasB && !skipB) {  // site B
-    if (s == 0) {
-      nb[0][0] = o0.v[0].y; nb[0][1] = o0.v[1].y; nb[0][2] = o0.v[2].y; e[0] = 1.f; w[0] = wt(1.f, hi);
-      nb[1][0] = o0.v[0].x; nb[1][1] = o0.v[1].x; nb[1][2] = o0.v[2].x; e[1] = 1.f; w[1] = wt(1.f, lo);
-      if (MASK && tail == 2) e[0] = w[0] = 0.f;
+  // bonds present (e) and present to an active neighbour (w), per site
+  float eA[6], eB[6], wA[6], wB[6];
+  if (W) {
+    const float exe = s ? ee1 : ee0;
+    const float erz[4] = {eyp, eym, zp ? 1.f : 0.f, zm ? 1.f : 0.f};
+    eA[0] = s && !hasB ? exe : 1.f;
+    eB[0] = s ? exe : 1.f;
+    eA[1] = s ? 1.f : exe;
+    eB[1] = 1.f;
+    // odd nx (masked only): the last site of an s = 0 row has no x+ bond
+    if (MASK && s == 0 && tail == 1) eA[0] = 0.f;
+    if (MASK && s == 0 && tail == 2) eB[0] = 0.f;
+#pragma unroll
+    for (int q = 0; q < 4; q++) eA[2 + q] = eB[2 + q] = erz[q];
+    if (MASK) {
+      const uint8_t lo = (uint8_t)(o0.pt & 0xFF), hi = (uint8_t)(o0.pt >> 8);
+      const uint16_t pr[4] = {yp.pt, ym.pt, op.pt, om.pt};
+      auto wt = [](float e, uint8_t p) { return e != 0.f && p != 0 ? 1.f : 0.f; };
+      wA[0] = wt(eA[0], s ? (hasB ? hi : pex) : lo);
+      wB[0] = wt(eB[0], s ? pex : hi);
+      wA[1] = wt(eA[1], s ? lo : pex);
+      wB[1] = wt(eB[1], s ? hi : lo);
+#pragma unroll
+      for (int q = 0; q < 4; q++) {
+        wA[2 + q] = wt(erz[q], (uint8_t)(pr[q] & 0xFF));
+        wB[2 + q] = wt(erz[q], (uint8_t)(pr[q] >> 8));
+      }
     } else {
-      nb[0][0] = exv[0]; nb[0][1] = exv[1]; nb[0][2] = exv[2]; e[0] = exe; w[0] = wt(exe, pex);
-      nb[1][0] = o0.v[0].y; nb[1][1] = o0.v[1].y; nb[1][2] = o0.v[2].y; e[1] = 1.f; w[1] = wt(1.f, hi);
+#pragma unroll
+      for (int d = 0; d < 6; d++) {
+        wA[d] = eA[d];
+        wB[d] = eB[d];
+      }
     }
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const OPair &o = *rows4[q];
-      nb[2 + q][0] = o.v[0].y; nb[2 + q][1] = o.v[1].y; nb[2 + q][2] = o.v[2].y;
-      e[2 + q] = erz[q];
-      w[2 + q] = wt(erz[q], MASK ? (uint8_t)(o.pt >> 8) : 1);
+    for (int d = 0; d < 6; d++) w[d] = pk(wA[d], wB[d]);
+  } else {
+#pragma unroll
+    for (int d = 0; d < 6; d++) eA[d] = eB[d] = wA[d] = wB[d] = 1.f;
+  }
+  // odd nx (masked only): a phantom in the last slot of an s = 1 row is skipped
+  const bool hereA = !(MASK && s == 1 && tail == 1), hereB = hasB && !(MASK && s == 1 && tail == 2);
+  const int psA = MASK ? (pself & 0xFF) : 1, psB = MASK ? (pself >> 8) : 1;
+  const bool actA = hereA && psA != 0, actB = hereB && psB != 0;
+  const V2 n = {pk(ax), pk(ay), pk(az)};
+  const V2 p = propose2(n, rw, ang);
+  f32x2 e_old, e_new;
+  bond_sums<POT, W>(R, n, p, nb, w, e_old, e_new);
+  // every rounding of dE is the scalar update's (site_update)
+  f32x2 dE = sub2(e_new, e_old);
+  if (POT == POT_LL) dE = mul2(pk1(bond_scale<POT>(R)), dE);
+  float sn[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+  if (MASK && (psA > 1 || psB > 1)) {  // surface sites
+    const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
+    float2 d = unpk(dE);
+    const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * R.plane + ns_at;
+    if (psA > 1) {
+#pragma unroll
+      for (int q = 0; q < 3; q++) sn[0][q] = __ldg(nsb + q * R.plane);
+      if (psA - 2 < R.nsurf)
+        d.x = __fadd_rn(d.x, __fsub_rn(surface_energy(R, psA - 2, px.x, py.x, pz.x, sn[0][0], sn[0][1], sn[0][2]),
+                                       surface_energy(R, psA - 2, ax.x, ay.x, az.x, sn[0][0], sn[0][1], sn[0][2])));
     }
-    const int ps = MASK ? (pself >> 8) : 1;
-    float sx = 0.f, sy = 0.f, sz = 0.f;
-    if (MASK && ps > 1) {
-      const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * P + ns_at + 1;
-      sx = __ldg(nsb);
-      sy = __ldg(nsb + P);
-      sz = __ldg(nsb + 2 * P);
+    if (psB > 1) {
+#pragma unroll
+      for (int q = 0; q < 3; q++) sn[1][q] = __ldg(nsb + q * R.plane + 1);
+      if (psB - 2 < R.nsurf)
+        d.y = __fadd_rn(d.y, __fsub_rn(surface_energy(R, psB - 2, px.y, py.y, pz.y, sn[1][0], sn[1][1], sn[1][2]),
+                                       surface_energy(R, psB - 2, ax.y, ay.y, az.y, sn[1][0], sn[1][1], sn[1][2])));
     }
-    acc += site_update<POT, MASK, FIELD, MODE>(R, a, c, ax.y, ay.y, az.y, nb, w, e, ps, sx, sy, sz, uB, ang, invT,
-                                               0u, qs);
+    dE = pk(d);
+  }
+  if (FIELD) {
+    const V2 ef = {pk1(R.ex), pk1(R.ey), pk1(R.ez)};
+    const f32x2 E = pk1(R.elecE), mA = pk1(-R.elecA);
+    const f32x2 dn = mul2(E, dot2(p, ef)), dold = mul2(E, dot2(n, ef));
+    dE = add2(dE, sub2(mul2(mul2(mA, dn), dn), mul2(mul2(mA, dold), dold)));
+  }
+  // src/evolve.cpp:160: accept when u < exp(-(E_new - E_old)/T)
+  const float2 arg = unpk(mul2(dE, pk1(-invT))), u2 = accept_uniforms(rw);
+  const bool accA = actA && u2.x < __expf(arg.x), accB = actB && u2.y < __expf(arg.y);
+  const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
+  if (accA) {
+    ax.x = px.x;
+    ay.x = py.x;
+    az.x = pz.x;
+    acc++;
+  }
+  if (accB) {
+    ax.y = px.y;
+    ay.y = py.y;
+    az.y = pz.y;
+    acc++;
+  }
+  if (MEAS) {
+    const float2 eo = unpk(e_old), en = unpk(e_new);
+    float nbs[6][3];
+    if (hereA) {
+#pragma unroll
+      for (int d = 0; d < 6; d++) {
+        nbs[d][0] = unpk(nb[d].x).x;
+        nbs[d][1] = unpk(nb[d].y).x;
+        nbs[d][2] = unpk(nb[d].z).x;
+      }
+      measure_site<POT, MASK, FIELD>(R, c, ax.x, ay.x, az.x, nbs, wA, eA, psA, sn[0][0], sn[0][1], sn[0][2],
+                                     accA ? en.x : eo.x, qs);
+    }
+    if (hereB) {
+#pragma unroll
+      for (int d = 0; d < 6; d++) {
+        nbs[d][0] = unpk(nb[d].x).y;
+        nbs[d][1] = unpk(nb[d].y).y;
+        nbs[d][2] = unpk(nb[d].z).y;
+      }
+      measure_site<POT, MASK, FIELD>(R, c, ax.y, ay.y, az.y, nbs, wB, eB, psB, sn[1][0], sn[1][1], sn[1][2],
+                                     accB ? en.y : eo.y, qs);
+    }
   }
 }
 
