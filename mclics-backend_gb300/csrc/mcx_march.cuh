@@ -317,24 +317,42 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
   if (POT == POT_LL) dE = mul2(pk1(bond_scale<POT>(R)), dE);
   float sn[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
   if (MASK && (psA > 1 || psB > 1)) {  // surface sites
-    const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
-    float2 d = unpk(dE);
     const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * R.plane + ns_at;
-    if (psA > 1) {
+    // the quadratic anchorings W (n.v)^2 of both sites in packed arithmetic
+    // (surface_energy's operations): v the surface normal or the easy axis, k
+    // its signed strength, 0 for a site without one
+    float v[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}, k[2] = {0.f, 0.f};
+    bool form[2] = {false, false};  // a GHRL-form anchoring: the general function
 #pragma unroll
-      for (int q = 0; q < 3; q++) sn[0][q] = __ldg(nsb + q * R.plane);
-      if (psA - 2 < R.nsurf)
+    for (int b = 0; b < 2; b++) {
+      const int sid = (b ? psB : psA) - 2;
+      if (sid < 0) continue;
+#pragma unroll
+      for (int q = 0; q < 3; q++) sn[b][q] = __ldg(nsb + q * R.plane + b);
+      if (sid >= R.nsurf) continue;
+      const int kind = R.anch[sid];
+      form[b] = kind == ANCH_HOMEOTROPIC_GHRL || kind == ANCH_FG_GHRL || kind == ANCH_RP_GHRL;
+      if (form[b]) continue;
+      const bool normal = kind == ANCH_HOMEOTROPIC || kind == ANCH_FG;
+      k[b] = kind == ANCH_FG ? R.W[sid] : -R.W[sid];
+      v[b][0] = normal ? sn[b][0] : R.dx[sid];
+      v[b][1] = normal ? sn[b][1] : R.dy[sid];
+      v[b][2] = normal ? sn[b][2] : R.dz[sid];
+    }
+    const V2 vv = {pk(v[0][0], v[1][0]), pk(v[0][1], v[1][1]), pk(v[0][2], v[1][2])};
+    const f32x2 kk = pk(k[0], k[1]), cn = dot2(p, vv), co = dot2(n, vv);
+    dE = add2(dE, sub2(mul2(mul2(kk, cn), cn), mul2(mul2(kk, co), co)));
+    if (form[0] || form[1]) {
+      const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
+      float2 d = unpk(dE);
+      if (form[0])
         d.x = __fadd_rn(d.x, __fsub_rn(surface_energy(R, psA - 2, px.x, py.x, pz.x, sn[0][0], sn[0][1], sn[0][2]),
                                        surface_energy(R, psA - 2, ax.x, ay.x, az.x, sn[0][0], sn[0][1], sn[0][2])));
-    }
-    if (psB > 1) {
-#pragma unroll
-      for (int q = 0; q < 3; q++) sn[1][q] = __ldg(nsb + q * R.plane + 1);
-      if (psB - 2 < R.nsurf)
+      if (form[1])
         d.y = __fadd_rn(d.y, __fsub_rn(surface_energy(R, psB - 2, px.y, py.y, pz.y, sn[1][0], sn[1][1], sn[1][2]),
                                        surface_energy(R, psB - 2, ax.y, ay.y, az.y, sn[1][0], sn[1][1], sn[1][2])));
+      dE = pk(d);
     }
-    dE = pk(d);
   }
   if (FIELD) {
     const V2 ef = {pk1(R.ex), pk1(R.ey), pk1(R.ez)};
