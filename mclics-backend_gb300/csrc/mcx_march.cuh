@@ -340,7 +340,10 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
       v[b][2] = normal ? sn[b][2] : R.dz[sid];
     }
     const V2 vv = {pk(v[0][0], v[1][0]), pk(v[0][1], v[1][1]), pk(v[0][2], v[1][2])};
-    const f32x2 kk = pk(k[0], k[1]), cn = dot2(p, vv), co = dot2(n, vv);
+    const f32x2 kk = pk(k[0], k[1]);
+    // n.v with the fusions the compiler gives surface_energy: x fused onto y
+    const f32x2 cn = fma2(p.z, vv.z, fma2(p.x, vv.x, mul2(p.y, vv.y)));
+    const f32x2 co = fma2(n.z, vv.z, fma2(n.x, vv.x, mul2(n.y, vv.y)));
     dE = add2(dE, sub2(mul2(mul2(kk, cn), cn), mul2(mul2(kk, co), co)));
     if (form[0] || form[1]) {
       const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
