@@ -55,9 +55,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_amar
   const RepDev &R = a.reps[r];
   const RepState *S = a.st + r;
   unsigned acc = 0;
-  float qs[kQ];
-#pragma unroll
-  for (int q = 0; q < kQ; q++) qs[q] = 0.f;
+  PairSums<false> sums;
+  sums.clear();
   const int p = u.y + (int)threadIdx.x;
   if (p < R.hp * R.ny) {
     const int nz = R.nz;
@@ -110,10 +109,9 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_amar
       const uint4 rw_next = pair_draw(m.pid + m.dpid, c, sw, seed, stream);  // unused after the last plane
       update_pair_draw<POT, false, FIELD, MODE, PER>(a, R, c, m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, o0, yp, ym, op,
                                                      om, exv, 0x0101, 1, zp, zm, rw, m.off, ang, invT, ax, ay, az, acc,
-                                                     qs);
+                                                     sums);
       if (MODE == MODE_SWEEP_MEASURE && a.meas_both && c == 1) {  // the colour-0 pair of this row (PassArgs::meas_both)
-        measure_opposite<FIELD>(R, o0.v[0].x, o0.v[1].x, o0.v[2].x, qs);
-        if (m.hasB) measure_opposite<FIELD>(R, o0.v[0].y, o0.v[1].y, o0.v[2].y, qs);
+        measure_opposite<FIELD, PER>(R, o0.v[0], o0.v[1], o0.v[2], m.hasB, sums);
       }
       rw = rw_next;
       *reinterpret_cast<float2 *>(m.A0 + m.off) = ax;
@@ -131,6 +129,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_amar
   }
   grid_dependency_wait();    // threads without a pair reach here without having waited
   grid_launch_dependents();  // the next pass may start its set-up now
+  float qs[kQ];
+  sums.fold(qs);
   flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, false);
 }
 

@@ -1003,7 +1003,23 @@ static bool persistent(const mcx_engine *e) {
   return e->pmarch && e->march && !e->staged && e->proposal == MCX_PROPOSAL_PLAIN;
 }
 
+// Whether the sweeps' kernels leave the inactive sites' field energy to
+// k_idle_field: the plain z-march and resident sweeps of a masked batch.
+static bool idle_field(const mcx_engine *e) {
+  return e->var.mask && e->var.field && e->march && !e->staged && e->proposal == MCX_PROPOSAL_PLAIN;
+}
+
 static mcx_status run_sweeps(mcx_engine *e, int n, int m) {
+  if (m && n > 0 && idle_field(e)) {
+    int plane = 0;
+    for (const RepDev &R : e->rep) plane = std::max(plane, R.plane);
+    // a replica per grid row: batches of more replicas than a grid has rows in parts
+    for (int r = 0; r < e->nrep; r += 32768)
+      launch_idle_field(e->d_rep + r, e->d_st + r, e->d_pt, e->d_dir,
+                        e->d_ring + (size_t)r * (e->ring_cap + 1) * kLanes * kQ, e->ring_cap,
+                        std::min(32768, e->nrep - r), plane, n, e->stream);
+    e->launches += 1;
+  }
   if (persistent(e) && pmarch_fits(e)) {  // otherwise the register march below (the same update)
     PassArgs pa = pass_args(e);
     for (int done = 0; done < n;) {

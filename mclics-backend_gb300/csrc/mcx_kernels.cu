@@ -819,6 +819,52 @@ void launch_flush(const FlushArgs &f, int nrep, cudaStream_t st) {
   k_flush<<<nrep, kFlushThreads, 0, st>>>(f);
 }
 
+// Field energy of the inactive sites of replica blockIdx.y (the all-site
+// energy counts it, energy_calculator, src/evolve.cpp:27-62), added to the
+// ring slots of its next n measured sweeps.  Inactive sites never move, so a
+// run of sweeps needs the sum once: adding it site by site in every measured
+// sweep made the units outside a droplet read their directors each time (8
+// droplets of 96^3: a measured pass took 100 us, an unmeasured one 56).
+constexpr int kIdleThreads = 256, kIdleSites = 8;  // sites per thread and colour
+__global__ void __launch_bounds__(kIdleThreads) k_idle_field(const RepDev *reps, const RepState *rst,
+                                                             const uint8_t *__restrict__ pt,
+                                                             const float *__restrict__ dir, double *ring, int ring_cap,
+                                                             int n) {
+  __shared__ double s_sum[kIdleThreads / 32];
+  const int r = blockIdx.y;
+  const RepDev &R = reps[r];
+  float sum = 0.f;
+  for (int q = 0; q < kIdleSites; q++) {
+    const int at = (blockIdx.x * kIdleSites + q) * kIdleThreads + threadIdx.x;
+    if (at >= R.plane) break;
+    const int row = at / R.hs, h = at - row * R.hs, jk = row % R.ny + row / R.ny;
+#pragma unroll
+    for (int c = 0; c < 2; c++) {
+      if (2 * h + ((c + jk) & 1) >= R.nx || pt[R.pt_off + (long long)c * R.pplane + (long long)row * R.hps + h] != 0)
+        continue;
+      const float *d = dir + R.dir_off + (long long)(3 * c) * R.plane + at;
+      sum += field_energy(R, d[0], d[R.plane], d[2 * R.plane]);
+    }
+  }
+  double v = sum;
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = v;
+  __syncthreads();
+  v = 0.0;
+  for (int w = 0; w < kIdleThreads / 32; w++) v += s_sum[w];
+  if (v == 0.0) return;
+  const unsigned long long first = rst[r].meas;
+  for (int s = threadIdx.x; s < n; s += kIdleThreads)
+    atomicAdd(ring + (((size_t)r * (ring_cap + 1) + (size_t)((first + s) % (unsigned long long)ring_cap)) * kLanes +
+                      blockIdx.x % kLanes) * kQ, v);
+}
+
+void launch_idle_field(const RepDev *reps, const RepState *st, const uint8_t *pt, const float *dir, double *ring,
+                       int ring_cap, int nrep, int max_plane, int n, cudaStream_t s) {
+  const int per = kIdleThreads * kIdleSites;
+  k_idle_field<<<dim3((max_plane + per - 1) / per, nrep), kIdleThreads, 0, s>>>(reps, st, pt, dir, ring, ring_cap, n);
+}
+
 void launch_measure_out(const RepDev *reps, double *ring, int ring_cap, int nrep, double *out, cudaStream_t st) {
   k_measure_out<<<(nrep + 127) / 128, 128, 0, st>>>(reps, ring, ring_cap, nrep, out);
 }

@@ -153,6 +153,11 @@ void launch_tpass(const Variant &v, int mode, const PassArgs &a, int grid, cudaS
 // per SM it reaches (0 if it cannot run).
 int tpass_smem_bytes(int stage_bytes);
 int tpass_blocks_per_sm(const Variant &v, int mode, int stage_bytes);
+// Adds the field energy of a masked batch's inactive sites, which no sweep
+// changes, to the ring slots of the next n measured sweeps (the z-march and
+// resident sweeps measure active sites only).
+void launch_idle_field(const RepDev *reps, const RepState *st, const uint8_t *pt, const float *dir, double *ring,
+                       int ring_cap, int nrep, int max_plane, int n, cudaStream_t s);
 void launch_flush(const FlushArgs &f, int nrep, cudaStream_t st);
 void launch_measure_out(const RepDev *reps, double *ring, int ring_cap, int nrep, double *out, cudaStream_t st);
 void launch_aos_to_split(const RepDev &R, const float *aos, float *dir, cudaStream_t st);

@@ -177,9 +177,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_tmar
     tm_issue(R, Ob, Ag, kb - 1, kb + 1, kb, kb, jA0, jA1, sl, &bars[0]);
   }
   unsigned acc = 0;
-  float qs[kQ];
-#pragma unroll
-  for (int q = 0; q < kQ; q++) qs[q] = 0.f;
+  PairSums<false> sums;
+  sums.clear();
   for (int t = 0; t < L; t++) {
     const int k = kb + t;
     // copies for the next step: A plane k+1, O plane k+2
@@ -220,7 +219,7 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_tmar
       update_pair<POT, false, FIELD, MODE, PER>(a, R, c, s, hasB, ee0, ee1, eyp, eym, o0, yp, ym, op, om, exv, 0x0101,
                                                 1, zp, zm, (uint32_t)row * (uint32_t)hp + (uint32_t)(h0 >> 1),
                                                 (long long)row * hs + h0, seed, stream, sw, ang, invT, ax, ay, az,
-                                                acc, qs);
+                                                acc, sums);
       float *g = Ag + (size_t)row * hs + h0;
       *reinterpret_cast<float2 *>(g) = ax;
       *reinterpret_cast<float2 *>(g + R.plane) = ay;
@@ -229,6 +228,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_tmar
     __syncthreads();  // the slots of this step may be refilled from here on
   }
   grid_launch_dependents();
+  float qs[kQ];
+  sums.fold(qs);
   flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, false);
 }
 

@@ -30,19 +30,17 @@ __device__ __forceinline__ float ldo1(const float *p) { return __ldcg(p); }
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" :::); }
 
-// What a measured pass adds for an active site of an unmasked lattice other
-// than its bonds (site_update): its Q-tensor products and field energy.
-template <bool FIELD>
-__device__ __forceinline__ void measure_opposite(const RepDev &R, float x, float y, float z, float qs[kQ]) {
-  qs[2] += x * x;
-  qs[3] += x * y;
-  qs[4] += x * z;
-  qs[5] += y * y;
-  qs[6] += y * z;
+// What a measured pass adds for the opposite pair of an unmasked lattice: its
+// Q-tensor products and field energy (its bonds are the own sites').
+template <bool FIELD, bool PER, class Q>
+__device__ __forceinline__ void measure_opposite(const RepDev &R, const float2 &x, const float2 &y, const float2 &z,
+                                                 bool hasB, Q &sums) {
+  const V2 n = {pk(x), pk(y), pk(z)};
+  const f32x2 m = pk(1.f, hasB ? 1.f : 0.f);
+  add_q<PER>(sums, n, m);
   if (FIELD) {
-    const float ef = field_energy(R, x, y, z);
-    qs[0] += ef;
-    qs[1] += ef;
+    const f32x2 ef = field_energy2(R, n);
+    sums.add(0, PER ? ef : mul2(ef, m));
   }
 }
 
@@ -82,7 +80,7 @@ __device__ __forceinline__ void grid_dependency_wait(March &m) {
                : "memory");
 }
 
-// A dead unit (kUnitDead) of a masked lattice: in measured sweeps with a
+// A dead unit (kUnitDead) of the learned pass: in measured sweeps with a
 // field, each own (inactive) site adds its field energy, in the order the
 // full update adds it; nothing else.
 // The slot of a phantom site (odd nx, a row whose own sites are odd) is
@@ -184,49 +182,6 @@ constexpr int march_min_blocks() {
                                 : (MCX_MARCH_MASK_REGS > 0 ? 65536 / (NT * MCX_MARCH_MASK_REGS) : 1);
 }
 
-// What a measured pass adds for one site with its final director (the
-// measured part of site_update): eb its bond sum to active neighbours.
-template <int POT, bool MASK, bool FIELD>
-__device__ __forceinline__ void measure_site(const RepDev &R, int c, float x, float y, float z, const float nb[6][3],
-                                             const float w[6], const float e[6], int pself, float sx, float sy,
-                                             float sz, float eb, float qs[kQ]) {
-  const int sid = pself - 2;
-  const bool surf = MASK && pself > 1 && sid < R.nsurf;
-  const float act = pself != 0 ? 1.f : 0.f;
-  if (pself != 0) {
-    qs[2] += x * x;
-    qs[3] += x * y;
-    qs[4] += x * z;
-    qs[5] += y * y;
-    qs[6] += y * z;
-  }
-  if (surf) {
-    const float es = surface_energy(R, sid, x, y, z, sx, sy, sz);
-    qs[0] += es;
-    qs[1] += es;
-  }
-  if (FIELD) {
-    const float ef = field_energy(R, x, y, z);
-    qs[0] += ef;
-    qs[1] += act * ef;
-  }
-  if (c == 1) {
-    if (pself != 0) {
-      const float ebs = bond_scale<POT>(R) * eb + bond_const<POT>(R, w);
-      qs[0] += 2.f * ebs;
-      qs[1] += 2.f * ebs;
-      if (MASK) {
-        float wi[6];
-#pragma unroll
-        for (int d = 0; d < 6; d++) wi[d] = e[d] - w[d];
-        qs[0] += bond_scale<POT>(R) * bond_sum<POT>(R, x, y, z, nb, wi) + bond_const<POT>(R, wi);
-      }
-    } else {
-      qs[0] += bond_scale<POT>(R) * bond_sum<POT>(R, x, y, z, nb, w) + bond_const<POT>(R, w);
-    }
-  }
-}
-
 // The update of one same-colour pair from its loaded neighbourhood (shared by
 // the z-march and its staged and prefetching forms): own directors (ax, ay,
 // az) in and out; o0 the opposite pair of the same row, yp / ym those of rows
@@ -235,13 +190,13 @@ __device__ __forceinline__ void measure_site(const RepDev &R, int c, float x, fl
 // row; rw the pair's Philox draw (pair_draw below).  Both sites run in packed
 // arithmetic (mcx_packed.cuh); a missing, phantom or inactive site's half is
 // computed and dropped.
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
 __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev &R, int c, int s, bool hasB_,
                                                  float ee0, float ee1, float eyp, float eym, const OPair &o0,
                                                  const OPair &yp, const OPair &ym, const OPair &op, const OPair &om,
                                                  const float exv[3], uint16_t pself, uint8_t pex, bool zp, bool zm,
                                                  const uint4 rw, long long ns_at, float ang, float invT, float2 &ax,
-                                                 float2 &ay, float2 &az, unsigned &acc, float qs[kQ],
+                                                 float2 &ay, float2 &az, unsigned &acc, Q &sums,
                                                  int tail = 0) {
   constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
   constexpr bool W = !PER;  // PER: every bond exists (all axes periodic, pairs always complete)
@@ -310,18 +265,23 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
   const bool actA = hereA && psA != 0, actB = hereB && psB != 0;
   const V2 n = {pk(ax), pk(ay), pk(az)};
   const V2 p = propose2(n, rw, ang);
-  f32x2 e_old, e_new;
-  bond_sums<POT, W>(R, n, p, nb, w, e_old, e_new);
+  f32x2 e_old, e_new, x[6], x_old = 0ull, x_new = 0ull;
+  if (MASK && MEAS) {  // bonds of active sites to inactive ones
+#pragma unroll
+    for (int d = 0; d < 6; d++) x[d] = pk(actA ? eA[d] - wA[d] : 0.f, actB ? eB[d] - wB[d] : 0.f);
+  }
+  bond_sums<POT, W, MASK && MEAS>(R, n, p, nb, w, e_old, e_new, x, x_old, x_new);
   // every rounding of dE is the scalar update's (site_update)
   f32x2 dE = sub2(e_new, e_old);
   if (POT == POT_LL) dE = mul2(pk1(bond_scale<POT>(R)), dE);
-  float sn[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+  f32x2 s_old = 0ull, s_new = 0ull, f_old = 0ull, f_new = 0ull;  // anchoring and field energies
   if (MASK && (psA > 1 || psB > 1)) {  // surface sites
     const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * R.plane + ns_at;
     // the quadratic anchorings W (n.v)^2 of both sites in packed arithmetic
     // (surface_energy's operations): v the surface normal or the easy axis, k
     // its signed strength, 0 for a site without one
-    float v[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}, k[2] = {0.f, 0.f};
+    float sn[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}}, v[2][3] = {{0.f, 0.f, 0.f}, {0.f, 0.f, 0.f}};
+    float k[2] = {0.f, 0.f};
     bool form[2] = {false, false};  // a GHRL-form anchoring: the general function
 #pragma unroll
     for (int b = 0; b < 2; b++) {
@@ -344,24 +304,28 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
     // n.v with the fusions the compiler gives surface_energy: x fused onto y
     const f32x2 cn = fma2(p.z, vv.z, fma2(p.x, vv.x, mul2(p.y, vv.y)));
     const f32x2 co = fma2(n.z, vv.z, fma2(n.x, vv.x, mul2(n.y, vv.y)));
-    dE = add2(dE, sub2(mul2(mul2(kk, cn), cn), mul2(mul2(kk, co), co)));
+    s_new = mul2(mul2(kk, cn), cn);
+    s_old = mul2(mul2(kk, co), co);
     if (form[0] || form[1]) {
       const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
-      float2 d = unpk(dE);
-      if (form[0])
-        d.x = __fadd_rn(d.x, __fsub_rn(surface_energy(R, psA - 2, px.x, py.x, pz.x, sn[0][0], sn[0][1], sn[0][2]),
-                                       surface_energy(R, psA - 2, ax.x, ay.x, az.x, sn[0][0], sn[0][1], sn[0][2])));
-      if (form[1])
-        d.y = __fadd_rn(d.y, __fsub_rn(surface_energy(R, psB - 2, px.y, py.y, pz.y, sn[1][0], sn[1][1], sn[1][2]),
-                                       surface_energy(R, psB - 2, ax.y, ay.y, az.y, sn[1][0], sn[1][1], sn[1][2])));
-      dE = pk(d);
+      float2 en = unpk(s_new), eo = unpk(s_old);
+      if (form[0]) {
+        en.x = surface_energy(R, psA - 2, px.x, py.x, pz.x, sn[0][0], sn[0][1], sn[0][2]);
+        eo.x = surface_energy(R, psA - 2, ax.x, ay.x, az.x, sn[0][0], sn[0][1], sn[0][2]);
+      }
+      if (form[1]) {
+        en.y = surface_energy(R, psB - 2, px.y, py.y, pz.y, sn[1][0], sn[1][1], sn[1][2]);
+        eo.y = surface_energy(R, psB - 2, ax.y, ay.y, az.y, sn[1][0], sn[1][1], sn[1][2]);
+      }
+      s_new = pk(en);
+      s_old = pk(eo);
     }
+    dE = add2(dE, sub2(s_new, s_old));
   }
   if (FIELD) {
-    const V2 ef = {pk1(R.ex), pk1(R.ey), pk1(R.ez)};
-    const f32x2 E = pk1(R.elecE), mA = pk1(-R.elecA);
-    const f32x2 dn = mul2(E, dot2(p, ef)), dold = mul2(E, dot2(n, ef));
-    dE = add2(dE, sub2(mul2(mul2(mA, dn), dn), mul2(mul2(mA, dold), dold)));
+    f_new = field_energy2(R, p);
+    f_old = field_energy2(R, n);
+    dE = add2(dE, sub2(f_new, f_old));
   }
   // src/evolve.cpp:160: accept when u < exp(-(E_new - E_old)/T)
   const float2 arg = unpk(mul2(dE, pk1(-invT))), u2 = accept_uniforms(rw);
@@ -380,28 +344,39 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
     acc++;
   }
   if (MEAS) {
-    const float2 eo = unpk(e_old), en = unpk(e_new);
-    float nbs[6][3];
-    if (hereA) {
-#pragma unroll
-      for (int d = 0; d < 6; d++) {
-        nbs[d][0] = unpk(nb[d].x).x;
-        nbs[d][1] = unpk(nb[d].y).x;
-        nbs[d][2] = unpk(nb[d].z).x;
+    // the final directors and their energies.  Each bond counts in the local
+    // energy of each active end, from the colour-1 side; the all-site energy
+    // also counts inactive sites' bonds to active ones.  (The field energy of
+    // inactive sites is k_idle_field's.)
+    constexpr bool ALL = PER;  // both sites count
+    const V2 nf = {pk(ax), pk(ay), pk(az)};
+    const f32x2 m = pk(actA ? 1.f : 0.f, actB ? 1.f : 0.f);
+    add_q<ALL>(sums, nf, m);
+    f32x2 site = 0ull;
+    if (MASK) site = pick2(accA, accB, s_new, s_old);
+    if (FIELD) site = add2(site, pick2(accA, accB, f_new, f_old));
+    if ((MASK || FIELD) && !ALL) site = mul2(site, m);
+    f32x2 all = site, valid = site;
+    if (c == 1) {
+      f32x2 eb = pick2(accA, accB, e_new, e_old);
+      if (POT == POT_LL) eb = mul2(pk1(bond_scale<POT>(R)), eb);
+      eb = add_bond_const<POT, W>(R, w, eb);
+      if (ALL) {
+        all = fma2(pk1(2.f), eb, all);
+      } else {
+        const f32x2 k2 = pk(actA ? 2.f : (hereA ? 1.f : 0.f), actB ? 2.f : (hereB ? 1.f : 0.f));
+        all = fma2(k2, eb, all);
+        if (MASK) {
+          valid = fma2(mul2(pk1(2.f), m), eb, valid);
+          f32x2 xb = pick2(accA, accB, x_new, x_old);
+          if (POT == POT_LL) xb = mul2(pk1(bond_scale<POT>(R)), xb);
+          all = add2(all, add_bond_const<POT, true>(R, x, xb));
+        }
       }
-      measure_site<POT, MASK, FIELD>(R, c, ax.x, ay.x, az.x, nbs, wA, eA, psA, sn[0][0], sn[0][1], sn[0][2],
-                                     accA ? en.x : eo.x, qs);
     }
-    if (hereB) {
-#pragma unroll
-      for (int d = 0; d < 6; d++) {
-        nbs[d][0] = unpk(nb[d].x).y;
-        nbs[d][1] = unpk(nb[d].y).y;
-        nbs[d][2] = unpk(nb[d].z).y;
-      }
-      measure_site<POT, MASK, FIELD>(R, c, ax.y, ay.y, az.y, nbs, wB, eB, psB, sn[1][0], sn[1][1], sn[1][2],
-                                     accB ? en.y : eo.y, qs);
-    }
+    if (MASK || FIELD || c == 1) sums.add(0, all);
+    if (MASK) sums.add(1, valid);
+    else if (Q::kMasked && (FIELD || c == 1)) sums.add(1, all);  // a masked batch's bulk sites
   }
 }
 
@@ -411,17 +386,17 @@ __device__ __forceinline__ uint4 pair_draw(uint32_t pid, int c, unsigned long lo
   return philox4x32_10(make_uint4(pid, (uint32_t)sw, (uint32_t)(sw >> 32), TAG_PLAIN | (uint32_t)c), seed, stream);
 }
 
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
 __device__ __forceinline__ void update_pair(const PassArgs &a, const RepDev &R, int c, int s, bool hasB_, float ee0,
                                             float ee1, float eyp, float eym, const OPair &o0, const OPair &yp,
                                             const OPair &ym, const OPair &op, const OPair &om, const float exv[3],
                                             uint16_t pself, uint8_t pex, bool zp, bool zm, uint32_t pid,
                                             long long ns_at, uint32_t seed, uint32_t stream, unsigned long long sw,
                                             float ang, float invT, float2 &ax, float2 &ay, float2 &az, unsigned &acc,
-                                            float qs[kQ], int tail = 0) {
+                                            Q &sums, int tail = 0) {
   update_pair_draw<POT, MASK, FIELD, MODE, PER>(a, R, c, s, hasB_, ee0, ee1, eyp, eym, o0, yp, ym, op, om, exv, pself,
                                                 pex, zp, zm, pair_draw(pid, c, sw, seed, stream), ns_at, ang, invT, ax,
-                                                ay, az, acc, qs, tail);
+                                                ay, az, acc, sums, tail);
 }
 
 }  // namespace mcx

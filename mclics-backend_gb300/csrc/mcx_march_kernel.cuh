@@ -12,11 +12,11 @@ namespace mcx {
 
 // One plane of the march: loads (first, so that the Philox rounds overlap
 // them), the pair update, the stores.
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
 __device__ __forceinline__ void march_plane(const PassArgs &a, const RepDev &R, int c, const March &m,
                                             const OPair &om, const OPair &o0, const OPair &op, bool zp, bool zm,
                                             uint32_t seed, uint32_t stream, unsigned long long sw, float ang,
-                                            float invT, unsigned &acc, float qs[kQ]) {
+                                            float invT, unsigned &acc, Q &sums) {
   float2 ax = *reinterpret_cast<const float2 *>(m.A0 + m.off);
   float2 ay = *reinterpret_cast<const float2 *>(m.A1 + m.off);
   float2 az = *reinterpret_cast<const float2 *>(m.A2 + m.off);
@@ -30,18 +30,17 @@ __device__ __forceinline__ void march_plane(const PassArgs &a, const RepDev &R, 
   if (MASK) {
     pself = __ldg(reinterpret_cast<const uint16_t *>(m.PA + m.offp));
     pex = __ldg(m.PO + m.offp + dx);
-    // two inactive sites: nothing moves, and an unmeasured sweep adds nothing
-    // (a warp of such pairs skips the draw and the arithmetic)
-    if (MODE == MODE_SWEEP && pself == 0) return;
+    // two inactive sites: nothing moves, and a measured sweep adds only the
+    // colour-1 sites' bonds to active ones (a warp of such pairs skips the draw
+    // and the arithmetic)
+    if (pself == 0 && (MODE == MODE_SWEEP || c == 0 || (o0.pt | yp.pt | ym.pt | op.pt | om.pt | pex) == 0)) return;
   }
   update_pair<POT, MASK, FIELD, MODE, PER>(a, R, c, m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, o0, yp, ym, op, om, exv,
                                            pself, pex, zp, zm, m.pid, m.off, seed, stream, sw, ang, invT, ax, ay, az,
-                                           acc, qs, m.tail);
+                                           acc, sums, m.tail);
   if (!MASK && MODE == MODE_SWEEP_MEASURE && a.meas_both && c == 1) {
-    // the colour-0 pair of this row (final: its pass is done), as the colour-0
-    // pass's site_update would measure it
-    measure_opposite<FIELD>(R, o0.v[0].x, o0.v[1].x, o0.v[2].x, qs);
-    if (m.hasB) measure_opposite<FIELD>(R, o0.v[0].y, o0.v[1].y, o0.v[2].y, qs);
+    // the colour-0 pair of this row (final: its pass is done)
+    measure_opposite<FIELD, PER>(R, o0.v[0], o0.v[1], o0.v[2], m.hasB, sums);
   }
   *reinterpret_cast<float2 *>(m.A0 + m.off) = ax;
   *reinterpret_cast<float2 *>(m.A1 + m.off) = ay;
@@ -50,9 +49,9 @@ __device__ __forceinline__ void march_plane(const PassArgs &a, const RepDev &R, 
 
 // The march of one unit's chunk of planes kb..ke-1 (everything after the
 // dependency wait).
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
 __device__ __forceinline__ void march_chunk(const PassArgs &a, const RepDev &R, int c, March &m, int kb, int ke,
-                                            const RepState *S, unsigned &acc, float qs[kQ]) {
+                                            const RepState *S, unsigned &acc, Q &sums) {
   const int nz = R.nz;
   const bool zper = R.zb == BOUND_PERIODIC;
   const uint32_t seed = R.seed, stream = R.stream;
@@ -72,7 +71,8 @@ __device__ __forceinline__ void march_chunk(const PassArgs &a, const RepDev &R, 
     const bool zp = k + 1 < nz || zper;
     const int up = k + 1 < nz ? 1 : 1 - nz;
     load_opair_at<MASK>(m, m.off + up * m.dz, m.offp + up * m.dzp, zp, op);
-    march_plane<POT, MASK, FIELD, MODE, PER>(a, R, c, m, om, o0, op, zp, zm, seed, stream, sw, ang, invT, acc, qs);
+    march_plane<POT, MASK, FIELD, MODE, PER>(a, R, c, m, om, o0, op, zp, zm, seed, stream, sw, ang, invT, acc,
+                                               sums);
     om = o0;
     o0 = op;
     zm = true;
@@ -92,9 +92,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>()) k_march
   const RepDev &R = a.reps[r];
   const RepState *S = a.st + r;
   unsigned acc = 0;
-  float qs[kQ];
-#pragma unroll
-  for (int q = 0; q < kQ; q++) qs[q] = 0.f;
+  PairSums<MASK> sums;
+  sums.clear();
   int slot = -1;  // the sweep's ring slot (measured passes)
   int p = u.y + (int)threadIdx.x;
   bool live = p < R.hp * R.ny;
@@ -115,15 +114,17 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>()) k_march
     // the ring slot read here, off the CTA's tail (headline lattice +0.8%);
     // not in the masked field build, where the live register cost it 1.1%
     if (MODE == MODE_SWEEP_MEASURE && !(MASK && FIELD) && threadIdx.x < kQ) slot = ring_slot(a, S);
-    if (MASK && (u.w & kUnitDead))
-      dead_unit<FIELD, MODE>(R, m, kb, ke, qs);
-    else if (MASK && (u.w & kUnitBulk))  // only bulk sites around: the unmasked update
-      march_chunk<POT, false, FIELD, MODE, false>(a, R, c, m, kb, ke, S, acc, qs);
+    if (MASK && (u.w & kUnitDead)) {
+      // no active site in or next to the unit: nothing to update or to measure
+    } else if (MASK && (u.w & kUnitBulk))  // only bulk sites around: the unmasked update
+      march_chunk<POT, false, FIELD, MODE, false>(a, R, c, m, kb, ke, S, acc, sums);
     else
-      march_chunk<POT, MASK, FIELD, MODE, PER>(a, R, c, m, kb, ke, S, acc, qs);
+      march_chunk<POT, MASK, FIELD, MODE, PER>(a, R, c, m, kb, ke, S, acc, sums);
   }
   grid_dependency_wait();    // threads without a pair reach here without having waited
   grid_launch_dependents();  // the next pass may start its set-up now
+  float qs[kQ];
+  sums.fold(qs);
   flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, MASK, -1, slot);
 }
 

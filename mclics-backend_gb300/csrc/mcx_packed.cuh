@@ -138,10 +138,12 @@ __device__ __forceinline__ f32x2 add_chiral(float sigma, const V2 &n, const V2 &
 
 // Slot D's bond (bond<POT, D>) of the old and of the new directors, added to
 // the running sums eo and en with weight w (W: some weights are not 1; they
-// are 0 or 1).
-template <int POT, int D, bool W>
+// are 0 or 1), and with X to xo and xn with weight x (a measured masked pass:
+// bonds to inactive neighbours).
+template <int POT, int D, bool W, bool X_>
 __device__ __forceinline__ void add_bonds(const PairConst<POT> &K, bool chiral, const DirTerms<POT> &o,
-                                          const DirTerms<POT> &n, const V2 &b, f32x2 w, f32x2 &eo, f32x2 &en) {
+                                          const DirTerms<POT> &n, const V2 &b, f32x2 w, f32x2 &eo, f32x2 &en, f32x2 x,
+                                          f32x2 &xo, f32x2 &xn) {
   constexpr int X = D >> 1;
   f32x2 no = dot2(o.n, b), nn = dot2(n.n, b);
   f32x2 vo, vn;
@@ -155,6 +157,10 @@ __device__ __forceinline__ void add_bonds(const PairConst<POT> &K, bool chiral, 
     } else {
       eo = fma2(W ? mul2(no, w) : no, no, eo);
       en = fma2(W ? mul2(nn, w) : nn, nn, en);
+    }
+    if (X_) {
+      xo = D == 0 ? mul2(mul2(no, x), no) : fma2(mul2(no, x), no, xo);
+      xn = D == 0 ? mul2(mul2(nn, x), nn) : fma2(mul2(nn, x), nn, xn);
     }
     return;
   } else if (POT == POT_PEAR) {
@@ -186,31 +192,42 @@ __device__ __forceinline__ void add_bonds(const PairConst<POT> &K, bool chiral, 
     eo = W ? fma2(w, vo, eo) : add2(vo, eo);
     en = W ? fma2(w, vn, en) : add2(vn, en);
   }
+  if (X_) {
+    xo = D == 0 ? mul2(x, vo) : fma2(x, vo, xo);
+    xn = D == 0 ? mul2(x, vn) : fma2(x, vn, xn);
+  }
 }
 
-// Bond sums of the old and the new directors over the six slots.
-template <int POT, bool W>
-__device__ __forceinline__ void bond_sums(const RepDev &R, const V2 &o, const V2 &n, const V2 nb[6], const f32x2 w[6],
-                                          f32x2 &eo, f32x2 &en) {
+// Bond sums of the old and the new directors over the six slots (X: also with
+// the weights x, into xo and xn).
+template <int POT, bool W, bool X>
+__device__ __forceinline__ void bond_sums_c(const RepDev &R, bool chiral, const V2 &o, const V2 &n, const V2 nb[6],
+                                            const f32x2 w[6], f32x2 &eo, f32x2 &en, const f32x2 x[6], f32x2 &xo,
+                                            f32x2 &xn) {
   const PairConst<POT> K(R);
-  const bool chiral = POT == POT_GHRL && R.sigma != 0.f;  // uniform: a CTA serves one replica
-  if (chiral) {
-    const DirTerms<POT> O(o, true), N(n, true);
-    add_bonds<POT, 0, W>(K, true, O, N, nb[0], w[0], eo, en);
-    add_bonds<POT, 1, W>(K, true, O, N, nb[1], w[1], eo, en);
-    add_bonds<POT, 2, W>(K, true, O, N, nb[2], w[2], eo, en);
-    add_bonds<POT, 3, W>(K, true, O, N, nb[3], w[3], eo, en);
-    add_bonds<POT, 4, W>(K, true, O, N, nb[4], w[4], eo, en);
-    add_bonds<POT, 5, W>(K, true, O, N, nb[5], w[5], eo, en);
-  } else {
-    const DirTerms<POT> O(o, false), N(n, false);
-    add_bonds<POT, 0, W>(K, false, O, N, nb[0], w[0], eo, en);
-    add_bonds<POT, 1, W>(K, false, O, N, nb[1], w[1], eo, en);
-    add_bonds<POT, 2, W>(K, false, O, N, nb[2], w[2], eo, en);
-    add_bonds<POT, 3, W>(K, false, O, N, nb[3], w[3], eo, en);
-    add_bonds<POT, 4, W>(K, false, O, N, nb[4], w[4], eo, en);
-    add_bonds<POT, 5, W>(K, false, O, N, nb[5], w[5], eo, en);
-  }
+  const DirTerms<POT> O(o, chiral), N(n, chiral);
+  add_bonds<POT, 0, W, X>(K, chiral, O, N, nb[0], w[0], eo, en, x[0], xo, xn);
+  add_bonds<POT, 1, W, X>(K, chiral, O, N, nb[1], w[1], eo, en, x[1], xo, xn);
+  add_bonds<POT, 2, W, X>(K, chiral, O, N, nb[2], w[2], eo, en, x[2], xo, xn);
+  add_bonds<POT, 3, W, X>(K, chiral, O, N, nb[3], w[3], eo, en, x[3], xo, xn);
+  add_bonds<POT, 4, W, X>(K, chiral, O, N, nb[4], w[4], eo, en, x[4], xo, xn);
+  add_bonds<POT, 5, W, X>(K, chiral, O, N, nb[5], w[5], eo, en, x[5], xo, xn);
+}
+
+template <int POT, bool W, bool X>
+__device__ __forceinline__ void bond_sums(const RepDev &R, const V2 &o, const V2 &n, const V2 nb[6], const f32x2 w[6],
+                                          f32x2 &eo, f32x2 &en, const f32x2 x[6], f32x2 &xo, f32x2 &xn) {
+  // uniform: a CTA serves one replica
+  if (POT == POT_GHRL && R.sigma != 0.f) bond_sums_c<POT, W, X>(R, true, o, n, nb, w, eo, en, x, xo, xn);
+  else bond_sums_c<POT, W, X>(R, false, o, n, nb, w, eo, en, x, xo, xn);
+}
+
+// The constant the GHRL bond leaves out (ghrl_bond_var), per weighted bond.
+template <int POT, bool W>
+__device__ __forceinline__ f32x2 add_bond_const(const RepDev &R, const f32x2 w[6], f32x2 e) {
+  if (POT != POT_GHRL) return e;
+  if (!W) return fma2(pk1(R.gconst), pk1(6.f), e);
+  return fma2(pk1(R.gconst), add2(add2(add2(w[0], w[1]), add2(w[2], w[3])), add2(w[4], w[5])), e);
 }
 
 // The pair's uniforms (pair_uniforms) as the packed update uses them: f0 and
@@ -256,6 +273,52 @@ __device__ __forceinline__ V2 propose2(const V2 &n, const uint4 &w, float ang) {
 __device__ __forceinline__ float2 accept_uniforms(const uint4 &w) {
   const uint32_t a = (w.z >> 9) & 0x7FFFFCu, b = ((w.z & 0x7FFu) << 12) | ((w.w & 0x3FFu) << 2);
   return unpk(add2(pk(one_plus(a), one_plus(b)), pk1(-1.f)));
+}
+
+// Sums of a measured pass (kQ quantities) over a thread's pairs, both sites of
+// a pair in the halves of a value.  MASKED: the energy of active sites is a sum
+// of its own.
+template <bool MASKED>
+struct PairSums {
+  static constexpr bool kMasked = MASKED;
+  f32x2 v[kQ];
+  __device__ __forceinline__ void clear() {
+#pragma unroll
+    for (int q = 0; q < kQ; q++) v[q] = 0ull;
+  }
+  __device__ __forceinline__ void add(int q, f32x2 t) { v[q] = add2(v[q], t); }
+  __device__ __forceinline__ void add_product(int q, f32x2 a, f32x2 b) { v[q] = fma2(a, b, v[q]); }
+  __device__ __forceinline__ void fold(float out[kQ]) const {
+#pragma unroll
+    for (int q = 0; q < kQ; q++) {
+      const float2 u = unpk(v[q]);
+      out[q] = u.x + u.y;
+    }
+  }
+};
+
+// The Q-tensor products of a pair of sites, m 1 for sites that count and 0 for
+// others.
+template <bool ALL, class Q>
+__device__ __forceinline__ void add_q(Q &sums, const V2 &n, f32x2 m) {
+  const f32x2 x = ALL ? n.x : mul2(n.x, m), y = ALL ? n.y : mul2(n.y, m), z = ALL ? n.z : mul2(n.z, m);
+  sums.add_product(2, x, n.x);
+  sums.add_product(3, x, n.y);
+  sums.add_product(4, x, n.z);
+  sums.add_product(5, y, n.y);
+  sums.add_product(6, y, n.z);
+}
+
+// Electric term of both sites (field_energy).
+__device__ __forceinline__ f32x2 field_energy2(const RepDev &R, const V2 &n) {
+  const V2 e = {pk1(R.ex), pk1(R.ey), pk1(R.ez)};
+  const f32x2 d = mul2(pk1(R.elecE), dot2(n, e));
+  return mul2(mul2(pk1(-R.elecA), d), d);
+}
+
+__device__ __forceinline__ f32x2 pick2(bool a, bool b, f32x2 yes, f32x2 no) {
+  const float2 y = unpk(yes), n = unpk(no);
+  return pk(a ? y.x : n.x, b ? y.y : n.y);
 }
 
 }  // namespace mcx

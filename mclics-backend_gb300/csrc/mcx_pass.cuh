@@ -21,6 +21,7 @@
 #include "mcx_device.cuh"
 #include "mcx_kernels.cuh"
 #include "mcx_mlp.cuh"
+#include "mcx_step.h"
 
 // Threads and CTAs per SM the direct pass kernel is compiled for.
 constexpr int kPB = 128;
@@ -241,6 +242,28 @@ __device__ __forceinline__ int ring_slot(const PassArgs &a, const RepState *S) {
   return (int)(__ldcg(&S->meas) % (unsigned long long)a.ring_cap);
 }
 
+// A warp's sums of its lanes' kQ quantities: quantity q ends in lane 4 q.
+// Lanes exchange halves of the values instead of every value with every step
+// (9 shuffles for 35); each sum is added in the order of a butterfly from lane
+// distance 16 down to 1.
+__device__ __forceinline__ float warp_sums(const float qs[kQ]) {
+  const int lane = threadIdx.x & 31;
+  float v[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) v[q] = q < kQ ? qs[q] : 0.f;
+#pragma unroll
+  for (int h = 4; h > 0; h >>= 1) {
+    const bool up = lane & (4 * h);
+#pragma unroll
+    for (int q = 0; q < h; q++) {
+      const float keep = up ? v[q + h] : v[q], give = up ? v[q] : v[q + h];
+      v[q] = keep + __shfl_xor_sync(0xffffffffu, give, 4 * h);
+    }
+  }
+  v[0] += __shfl_xor_sync(0xffffffffu, v[0], 2);
+  return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
+}
+
 // slot_pre: the ring slot if the caller read it early (ring_slot; -1: read
 // it here, at the end of the CTA, where its latency is exposed).
 template <int NT, int MODE>
@@ -270,13 +293,8 @@ __device__ __forceinline__ void flush_replica(const PassArgs &a, int r, int unit
     if (lane == 0) s_acc[wid] = wa;
   }
   if (MEAS) {
-#pragma unroll
-    for (int q = 0; q < kQ; q++) {
-      float v = qs[q];
-#pragma unroll
-      for (int o2 = 16; o2 > 0; o2 >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o2);
-      if (lane == 0) s_q[wid][q] = v;
-    }
+    const float v = warp_sums(qs);
+    if ((lane & 3) == 0 && lane < 4 * kQ) s_q[wid][lane >> 2] = v;
   }
   __syncthreads();
   if (MEAS && threadIdx.x < kQ) {
@@ -304,17 +322,7 @@ __device__ __forceinline__ void flush_replica(const PassArgs &a, int r, int unit
       if ((unsigned)(old >> 32) + (unsigned)units == total) {  // the replica's last unit of the sweep
         const unsigned sweep_acc = (unsigned)old + tot;
         S->cnt = 0ull;
-        // src/evolve.cpp:169-178 with the reference's float/double rounding
-        float av = av0;
-        const double ratio = 1.0 * (double)sweep_acc / (double)R.valid;
-        if (frozen0) {
-        } else if (ratio < 0.5) {
-          av = (float)((double)av * 0.99);
-          if ((double)av < 0.01) av = (float)0.01;
-        } else if (ratio > 0.5) {
-          av = (float)((double)av / 0.99);
-          if ((double)av > 1.0) av = (float)((double)av - 0.5);
-        }
+        const float av = frozen0 ? av0 : next_step(av0, sweep_acc, (unsigned)R.valid);  // src/evolve.cpp:169-178
         S->ang_var = av;
         const unsigned long long sweep = sweep0 + 1;
         S->sweep = sweep;

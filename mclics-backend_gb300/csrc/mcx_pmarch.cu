@@ -79,11 +79,11 @@ __device__ __forceinline__ void pm_load_opair(const March &m, int off, int offp,
 }
 
 // One plane: k_march's march_plane with L2 loads of the directors.
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
 __device__ __forceinline__ void pm_plane(const PassArgs &a, const RepDev &R, int c, const March &m, const OPair &om,
                                          const OPair &o0, const OPair &op, bool zp, bool zm, uint32_t seed,
                                          uint32_t stream, unsigned long long sw, float ang, float invT, unsigned &acc,
-                                         float qs[kQ]) {
+                                         Q &sums) {
   float2 ax = ldcg2(m.A0 + m.off);
   float2 ay = ldcg2(m.A1 + m.off);
   float2 az = ldcg2(m.A2 + m.off);
@@ -100,7 +100,7 @@ __device__ __forceinline__ void pm_plane(const PassArgs &a, const RepDev &R, int
   }
   update_pair<POT, MASK, FIELD, MODE, PER>(a, R, c, m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, o0, yp, ym, op, om, exv,
                                            pself, pex, zp, zm, m.pid, m.off, seed, stream, sw, ang, invT, ax, ay, az,
-                                           acc, qs, m.tail);
+                                           acc, sums, m.tail);
   *reinterpret_cast<float2 *>(m.A0 + m.off) = ax;
   *reinterpret_cast<float2 *>(m.A1 + m.off) = ay;
   *reinterpret_cast<float2 *>(m.A2 + m.off) = az;
@@ -126,14 +126,9 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>())
   for (int pass = 0; pass < 2 * nsweeps; pass++) {
     const int c = pass & 1;
     unsigned acc = 0;
-    float qs[kQ];
-#pragma unroll
-    for (int q = 0; q < kQ; q++) qs[q] = 0.f;
-    if (has_pair && dead) {
-      March m;
-      march_init<MASK>(a, R, c, p, kb, m);
-      dead_unit<FIELD, MODE>(R, m, kb, ke, qs);
-    } else if (has_pair) {
+    PairSums<MASK> sums;
+    sums.clear();
+    if (has_pair && !dead) {
       March m;
       march_init<MASK>(a, R, c, p, kb, m);
       const unsigned long long sw = __ldcg(&S->sweep);
@@ -151,7 +146,7 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>())
         const bool zp = k + 1 < nz || zper;
         const int up = k + 1 < nz ? 1 : 1 - nz;
         pm_load_opair<MASK>(m, m.off + up * m.dz, m.offp + up * m.dzp, zp, op);
-        pm_plane<POT, MASK, FIELD, MODE, PER>(a, R, c, m, om, o0, op, zp, zm, seed, stream, sw, ang, invT, acc, qs);
+        pm_plane<POT, MASK, FIELD, MODE, PER>(a, R, c, m, om, o0, op, zp, zm, seed, stream, sw, ang, invT, acc, sums);
         om = o0;
         o0 = op;
         zm = true;
@@ -162,6 +157,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>())
         m.s ^= 1;
       }
     }
+    float qs[kQ];
+    sums.fold(qs);
     flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, MASK, c);
     target += gridDim.x;
     if (!pm_barrier(bar, target, a.err)) return;

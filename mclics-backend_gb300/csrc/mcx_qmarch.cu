@@ -81,9 +81,8 @@ __global__ void __launch_bounds__(NT, qmarch_min_blocks<NT>()) k_qmarch(PassArgs
   const RepDev &R = a.reps[r];
   const RepState *S = a.st + r;
   unsigned acc = 0;
-  float qs[kQ];
-#pragma unroll
-  for (int q = 0; q < kQ; q++) qs[q] = 0.f;
+  PairSums<false> sums;
+  sums.clear();
   // the thread's pairs: p and p + 1 of the plane (row-major), the same row
   // because a row holds an even number of pairs
   const int p = u.y + 2 * (int)threadIdx.x;
@@ -158,15 +157,14 @@ __global__ void __launch_bounds__(NT, qmarch_min_blocks<NT>()) k_qmarch(PassArgs
       float2 axB = make_float2(ax.z, ax.w), ayB = make_float2(ay.z, ay.w), azB = make_float2(az.z, az.w);
       update_pair_draw<POT, false, FIELD, MODE, PER>(a, R, c, s, true, ee0, 1.f, eyp, eym, lo_pair(o0), lo_pair(yp),
                                                      lo_pair(ym), lo_pair(op), lo_pair(om), xA, 0x0101, 1, zp, zm,
-                                                     rwA, off, ang, invT, axA, ayA, azA, acc, qs);
+                                                     rwA, off, ang, invT, axA, ayA, azA, acc, sums);
       update_pair_draw<POT, false, FIELD, MODE, PER>(a, R, c, s, true, 1.f, ee1, eyp, eym, hi_pair(o0), hi_pair(yp),
                                                      hi_pair(ym), hi_pair(op), hi_pair(om), xB, 0x0101, 1, zp, zm,
-                                                     rwB, off + 2, ang, invT, axB, ayB, azB, acc, qs);
+                                                     rwB, off + 2, ang, invT, axB, ayB, azB, acc, sums);
       if (MODE == MODE_SWEEP_MEASURE && a.meas_both && c == 1) {  // the colour-0 quad of this row (PassArgs::meas_both)
-        measure_opposite<FIELD>(R, o0.v[0].x, o0.v[1].x, o0.v[2].x, qs);
-        measure_opposite<FIELD>(R, o0.v[0].y, o0.v[1].y, o0.v[2].y, qs);
-        measure_opposite<FIELD>(R, o0.v[0].z, o0.v[1].z, o0.v[2].z, qs);
-        measure_opposite<FIELD>(R, o0.v[0].w, o0.v[1].w, o0.v[2].w, qs);
+        const OPair lo = lo_pair(o0), hi = hi_pair(o0);
+        measure_opposite<FIELD, true>(R, lo.v[0], lo.v[1], lo.v[2], true, sums);
+        measure_opposite<FIELD, true>(R, hi.v[0], hi.v[1], hi.v[2], true, sums);
       }
       *reinterpret_cast<float4 *>(A0 + off) = make_float4(axA.x, axA.y, axB.x, axB.y);
       *reinterpret_cast<float4 *>(A1 + off) = make_float4(ayA.x, ayA.y, ayB.x, ayB.y);
@@ -181,6 +179,8 @@ __global__ void __launch_bounds__(NT, qmarch_min_blocks<NT>()) k_qmarch(PassArgs
   }
   grid_dependency_wait();    // threads without pairs reach here without having waited
   grid_launch_dependents();  // the next pass may start its set-up now
+  float qs[kQ];
+  sums.fold(qs);
   flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, false);
 }
 
