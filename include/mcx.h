@@ -221,7 +221,7 @@ int mcx_get_staged(const mcx_engine *eng);
  * summation order): the autotuner's choice changes the speed, never the
  * trajectory.
  *
- *   MCX_PASS_MARCH   the default: a CTA marches a block of same-colour site
+ *   MCX_PASS_MARCH   the default of larger lattices: a CTA marches a block of same-colour site
  *                    pairs of one z-plane through a chunk of planes, keeping
  *                    the z neighbours in registers;
  *   MCX_PASS_DIRECT  persistent CTAs, each pair's neighbourhood loaded by
@@ -239,7 +239,14 @@ int mcx_get_staged(const mcx_engine *eng);
  *                    of 128 or 256 threads; one wave of units);
  *   MCX_PASS_MARCH_QUAD  the z-march with four same-colour sites (two pairs)
  *                    per thread and 16-byte loads (unmasked batches with nx a
- *                    multiple of 8).
+ *                    multiple of 8);
+ *   MCX_PASS_RESIDENT  a run of sweeps as one launch, every replica resident
+ *                    in the shared memory of a cluster of 1 to 16 CTAs
+ *                    (replicas up to about 40^3; MCX_ERR_UNSUPPORTED
+ *                    otherwise).  The default of engines whose replicas are
+ *                    small enough that it is estimated faster;
+ *                    mcx_set_march_shape returns to MCX_PASS_MARCH, which also
+ *                    runs the single passes of mcx_pass_timing.
  * No counterpart in the reference. */
 typedef enum {
   MCX_PASS_MARCH = 0,
@@ -248,7 +255,8 @@ typedef enum {
   MCX_PASS_MARCH_TMA = 3,
   MCX_PASS_MARCH_ASYNC = 4,
   MCX_PASS_MARCH_PERSISTENT = 5,
-  MCX_PASS_MARCH_QUAD = 6
+  MCX_PASS_MARCH_QUAD = 6,
+  MCX_PASS_RESIDENT = 7
 } mcx_pass_kind;
 mcx_status mcx_set_pass(mcx_engine *eng, int kind);
 int mcx_get_pass(const mcx_engine *eng);
@@ -257,12 +265,14 @@ int mcx_get_pass(const mcx_engine *eng);
  * so that the work units fill max(1, -planes) waves of the CTAs the GPU holds
  * at once).  Default 128 x 8. */
 mcx_status mcx_set_march_shape(mcx_engine *eng, int block, int planes);
-/* Autotuner: times the z-march pass (register and, for unmasked batches,
- * TMA-staged forms) for block sizes {64, 128, 256} and chunk
+/* Autotuner: times the z-march pass (register form and, for unmasked batches,
+ * the prefetching and four-site forms) for block sizes {64, 128, 256} and chunk
  * depths {1, 2, 4, ..., 32} (up to the deepest lattice) and balanced chunks
- * over 1 to 4 waves (planes 0, -2, -3, -4) on a scratch copy of
- * the engine's state (the state itself is untouched), keeps the fastest and
- * reports it (any output may be NULL).  Synchronous. */
+ * over 1 to 4 waves (planes 0, -2, -3, -4), and the resident form where it
+ * runs, on a scratch copy of the engine's state (the state itself is
+ * untouched), keeps the fastest and reports it (any output may be NULL; the
+ * resident form reports the z-march shape that its short runs use).
+ * Synchronous. */
 mcx_status mcx_autotune(mcx_engine *eng, int *block, int *planes, float *pass_us);
 
 /* Learned proposal (no counterpart in the reference).  A small network reads

@@ -3,6 +3,7 @@
 // per-sweep sequence (pass 0, pass 1, [measure], epilogue) captured once into
 // CUDA graphs of kChunk sweeps and replayed.
 #include <cuda_runtime.h>
+#include <math.h>
 #include <stdarg.h>
 #include <stdlib.h>
 #include <stdio.h>
@@ -76,6 +77,11 @@ struct mcx_engine {
   bool amarch = false;  // the z-march with a per-thread cp.async prefetch (unmasked LL / GHRL)
   bool pmarch = false;  // the z-march as one cooperative launch per run of sweeps (grid barriers)
   bool qmarch = false;  // the z-march with four sites per thread (unmasked, nx a multiple of 8)
+  bool resident = false;  // runs of sweeps with every replica resident in a cluster's shared memory
+  int res_c = 0, res_nt = 0, res_smem = 0;  // its clusters' CTAs, threads and shared memory (0: cannot run)
+  std::vector<int> res_cut;                 // [nrep][res_c + 2]: rows of its CTAs (launch_resident)
+  int *d_cut = nullptr;
+  std::vector<std::vector<int>> rowcnt;     // active sites per row of a masked replica (empty: all)
   // per replica of a masked batch, row j + ny * k: 0 no active site, 1 only
   // bulk sites (point type 1), 2 anything else (empty: unknown)
   std::vector<std::vector<uint8_t>> rowact;
@@ -110,6 +116,8 @@ static PassArgs pass_args(mcx_engine *e);
 static bool use_tmarch(mcx_engine *e, bool on);
 static bool qmarch_ok(const mcx_engine *e);
 static mcx_status apply_march_shape(mcx_engine *e, int nt, int k);
+static double plan_resident(mcx_engine *e);
+static double march_estimate(const mcx_engine *e);
 
 static mcx_status fail(mcx_engine *e, mcx_status st, const char *fmt, ...) {
   char buf[512];
@@ -216,6 +224,7 @@ static void free_engine(mcx_engine *e) {
   cudaFree(e->d_mlp);
   cudaFree(e->d_units);
   cudaFree(e->d_lunits);
+  cudaFree(e->d_cut);
   cudaFree(e->d_w);
   cudaFree(e->d_am);
   cudaFree(e->d_av);
@@ -481,6 +490,7 @@ extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engin
   e->rep.resize(n);
   e->rowact.resize(n);
   e->segact.resize(n);
+  e->rowcnt.resize(n);
   e->tiled.assign(n, 0);
   for (int r = 0; r < n; r++) {
     mcx_replica_desc &d = e->desc[r];
@@ -697,6 +707,11 @@ extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engin
       return st;
     }
   }
+  // small lattices: resident where that is estimated faster than the z-march
+  if (e->march && !e->staged) {
+    const double t = plan_resident(e);
+    e->resident = t > 0.0 && t < march_estimate(e);
+  }
   CKC(cudaStreamSynchronize(e->stream));
 #undef CKC
   *out = e;
@@ -793,11 +808,14 @@ extern "C" mcx_status mcx_set_mask(mcx_engine *e, int r, const int *pt, const fl
   // which rows hold an active site: z-march units far from every one skip their updates
   std::vector<uint8_t> &act = e->rowact[r];
   act.assign((size_t)R.ny * R.nz, 0);
+  std::vector<int> &cnt = e->rowcnt[r];
+  cnt.assign((size_t)R.ny * R.nz, 0);
   for (long row = 0; row < (long)R.ny * R.nz; row++) {
     bool any = false, bulk = true;
     for (int i = 0; i < R.nx; i++) {
       any |= pt[row * R.nx + i] != 0;
       bulk &= pt[row * R.nx + i] == 1;
+      cnt[row] += pt[row * R.nx + i] != 0;
     }
     // an odd-nx row also holds a padding slot (inactive): never a bulk row
     act[row] = bulk && R.nx % 2 == 0 ? 1 : (any ? 2 : 0);
@@ -1003,6 +1021,126 @@ static bool persistent(const mcx_engine *e) {
   return e->pmarch && e->march && !e->staged && e->proposal == MCX_PROPOSAL_PLAIN;
 }
 
+// Sweeps per launch of the resident form (bounds a launch to some milliseconds).
+// Runs of any length use it: one sweep takes 13 to 31 us through it, loading
+// and storing the lattice included, and 13 to 30 us as two z-march passes (16^3
+// to 16 x 25^3); two sweeps are faster everywhere.
+constexpr int kResidentSweeps = 4096;
+static bool use_resident(const mcx_engine *e) {
+  return e->resident && e->march && !e->staged && e->proposal == MCX_PROPOSAL_PLAIN;
+}
+
+// Cuts replica r's rows into C shares of near-equal work (active sites of a
+// masked replica, whose idle rows still cost a little), each at least one
+// plane: out[0 .. C] the first rows, out[C + 1] the largest share.  Returns the
+// largest share's work in sites.
+static int cut_rows(const mcx_engine *e, int r, int C, int *out) {
+  const RepDev &R = e->rep[r];
+  const int rows = R.ny * R.nz;
+  const std::vector<int> &cnt = e->rowcnt[r];
+  auto weight = [&](int row) { return cnt.empty() ? (long long)R.nx : 1 + (long long)cnt[row]; };
+  long long total = 0;
+  for (int q = 0; q < rows; q++) total += weight(q);
+  out[0] = 0;
+  long long sum = 0, worst = 0, share = 0;
+  int row = 0, widest = 0;
+  for (int q = 0; q < C; q++) {
+    const long long goal = total * (q + 1) / C;
+    share = 0;
+    const int hi = rows - (C - 1 - q) * R.ny;  // leaves a plane for every share after this one
+    const int lo = std::min(hi, out[q] + R.ny);
+    while (row < hi && (row < lo || q == C - 1 || sum + weight(row) / 2 < goal)) {
+      sum += weight(row);
+      share += weight(row);
+      row++;
+    }
+    out[q + 1] = row;
+    worst = std::max(worst, share);
+    widest = std::max(widest, row - out[q]);
+  }
+  out[C + 1] = widest;
+  return (int)worst;
+}
+
+// Estimated microseconds per pass of the resident form for one shape, fitted
+// to measurements of 16^3 to 40^3 lattices, 1 to 300 replicas, clusters of 1
+// to 16 CTAs of 128 to 512 threads (within 15% of most): a pass costs 0.4 for
+// the exchange, and per pair and thread a latency plus the issue time of the
+// warps that share a scheduler.
+static double resident_estimate(const mcx_engine *e, int pairs, int C, int nt, int live, int nsm) {
+  const double lat = e->var.pot == POT_LL ? 0.20 : (e->var.pot == POT_PEAR ? 0.25 : 0.27);
+  const double issue = e->var.pot == POT_LL ? 0.19 : (e->var.pot == POT_PEAR ? 0.25 : 0.32);
+  const double waves = std::ceil((double)e->nrep / live);
+  const double per_sm = std::ceil(std::min(e->nrep, live) * (double)C / nsm);
+  const double it = std::ceil((double)pairs / nt);
+  return waves * (0.4 + it * (e->var.mask ? 1.5 : 1.0) * (lat + issue * per_sm * nt / 128.0));
+}
+
+// The z-march's estimated microseconds per pass at its best shape (launch,
+// ramp and drain, then its rate), for the choice between the two.
+static double march_estimate(const mcx_engine *e) {
+  double sites = 0;
+  for (const RepDev &R : e->rep) sites += (double)R.valid;
+  const double rate = e->var.pot == POT_LL ? 1.0e5 : (e->var.pot == POT_PEAR ? 8.0e4 : 6.2e4);
+  return 2.3 + (e->var.mask ? 1.5 : 1.0) * 0.5 * sites / rate;
+}
+
+// Chooses the resident form's cluster size and CTA size: the shape with the
+// least estimated time per pass.  Returns the estimate, 0 when no shape runs
+// this batch (a replica's rows do not fit a cluster's shared memory).
+static double plan_resident(mcx_engine *e) {
+  e->res_c = 0;
+  int minz = 1 << 30, dev = 0, nsm = 0;
+  for (const RepDev &R : e->rep) minz = std::min(minz, R.nz);
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+  double best = 1e30;
+  std::vector<int> cut;
+  for (int C : {1, 2, 4, 8, 16}) {
+    if (C > minz) break;  // a CTA's rows span at least one plane
+    long long smem = 0;
+    int sites = 0;
+    // the replicas of one shape are cut alike; look at the memory first
+    for (const RepDev &R : e->rep)
+      smem = std::max(smem, resident_smem_bytes(R, e->var.mask, (R.ny * R.nz + C - 1) / C));
+    if (smem > kResidentSmem) continue;
+    cut.assign((size_t)e->nrep * (C + 2), 0);
+    for (int r = 0; r < e->nrep; r++) {
+      int *c = cut.data() + (size_t)r * (C + 2);
+      sites = std::max(sites, cut_rows(e, r, C, c));
+      smem = std::max(smem, resident_smem_bytes(e->rep[r], e->var.mask, c[C + 1]));
+    }
+    if (smem > kResidentSmem) continue;
+    const int pairs = (sites + 3) / 4;  // of one colour
+    int last = 0;
+    for (int cap = 128; cap <= resident_max_threads(); cap *= 2) {
+      const int it = (pairs + cap - 1) / cap, nt = std::max(64, ((pairs + it - 1) / it + 31) / 32 * 32);
+      if (nt == last) continue;
+      last = nt;
+      const int live = resident_clusters(e->var, C, nt, (int)smem);
+      if (live <= 0) continue;
+      const double est = resident_estimate(e, pairs, C, nt, live, nsm);
+      if (est < best) {
+        best = est;
+        e->res_c = C;
+        e->res_nt = nt;
+        e->res_smem = (int)smem;
+        e->res_cut = cut;
+      }
+    }
+  }
+  if (e->res_c == 0) return 0.0;
+  cudaFree(e->d_cut);
+  e->d_cut = nullptr;
+  if (cudaMalloc(&e->d_cut, sizeof(int) * e->res_cut.size()) != cudaSuccess ||
+      cudaMemcpy(e->d_cut, e->res_cut.data(), sizeof(int) * e->res_cut.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+    cudaGetLastError();
+    e->res_c = 0;
+    return 0.0;
+  }
+  return best;
+}
+
 // Whether the sweeps' kernels leave the inactive sites' field energy to
 // k_idle_field: the plain z-march and resident sweeps of a masked batch.
 static bool idle_field(const mcx_engine *e) {
@@ -1019,6 +1157,17 @@ static mcx_status run_sweeps(mcx_engine *e, int n, int m) {
                         e->d_ring + (size_t)r * (e->ring_cap + 1) * kLanes * kQ, e->ring_cap,
                         std::min(32768, e->nrep - r), plane, n, e->stream);
     e->launches += 1;
+  }
+  if (use_resident(e)) {
+    PassArgs pa = pass_args(e);
+    for (int done = 0; done < n;) {
+      const int k = std::min(n - done, kResidentSweeps);
+      CK(e, launch_resident(e->var, m ? MODE_SWEEP_MEASURE : MODE_SWEEP, pa, e->d_cut, e->nrep, k, e->res_c, e->res_nt,
+                            e->res_smem, e->stream));
+      e->launches += 1;
+      done += k;
+    }
+    return MCX_OK;
   }
   if (persistent(e) && pmarch_fits(e)) {  // otherwise the register march below (the same update)
     PassArgs pa = pass_args(e);
@@ -1070,6 +1219,8 @@ static mcx_status check_err_flag(mcx_engine *e) {
     CK(e, cudaMemset(e->d_err, 0, sizeof f));
     if (f & 2u)
       return fail(e, MCX_ERR_CUDA, "persistent z-march: a grid barrier was not reached in time; results are invalid");
+    if (f & 8u)
+      return fail(e, MCX_ERR_CUDA, "resident sweeps: a neighbouring CTA's rows did not arrive in time; results are invalid");
     if (f & 4u)
       return fail(e, MCX_ERR_CUDA, "tensor-core network: an MMA did not complete in time; results are invalid");
     return fail(e, MCX_ERR_CUDA, "staged pass: a shared-memory tile copy did not complete in time; results are invalid");
@@ -1085,7 +1236,7 @@ extern "C" mcx_status mcx_sync(mcx_engine *e) {
 
 extern "C" mcx_status mcx_set_pass(mcx_engine *e, int kind) {
   if (!e) return fail(nullptr, MCX_ERR_INVALID, "null engine");
-  if (kind < MCX_PASS_MARCH || kind > MCX_PASS_MARCH_QUAD)
+  if (kind < MCX_PASS_MARCH || kind > MCX_PASS_RESIDENT)
     return fail(e, MCX_ERR_INVALID, "unknown pass kernel %d", kind);
   if (kind == MCX_PASS_STAGED && !e->can_stage)
     return fail(e, MCX_ERR_UNSUPPORTED, "a replica's rows do not fit the staged pass's shared memory");
@@ -1098,13 +1249,16 @@ extern "C" mcx_status mcx_set_pass(mcx_engine *e, int kind) {
     return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march runs blocks of 128 or 256 threads");
   if (kind == MCX_PASS_MARCH_QUAD && !qmarch_ok(e))
     return fail(e, MCX_ERR_UNSUPPORTED, "the four-site z-march needs an unmasked batch with nx a multiple of 8");
+  if (kind == MCX_PASS_RESIDENT && plan_resident(e) == 0.0)
+    return fail(e, MCX_ERR_UNSUPPORTED, "the resident form needs every replica to fit the shared memory of one cluster");
   if (kind != MCX_PASS_MARCH_TMA) e->tmarch = false;
+  e->resident = kind == MCX_PASS_RESIDENT;
   e->amarch = kind == MCX_PASS_MARCH_ASYNC;
   e->qmarch = kind == MCX_PASS_MARCH_QUAD;
   e->pmarch = kind == MCX_PASS_MARCH_PERSISTENT;
   e->staged = kind == MCX_PASS_STAGED;
   e->march = kind == MCX_PASS_MARCH || kind == MCX_PASS_MARCH_TMA || kind == MCX_PASS_MARCH_ASYNC ||
-             kind == MCX_PASS_MARCH_PERSISTENT || kind == MCX_PASS_MARCH_QUAD;
+             kind == MCX_PASS_MARCH_PERSISTENT || kind == MCX_PASS_MARCH_QUAD || kind == MCX_PASS_RESIDENT;
   if (e->march) {
     if (mcx_status st = apply_march_shape(e, e->march_nt, e->march_k)) return st;  // chunks follow the form's residency
     if (e->pmarch && !pmarch_fits(e)) {
@@ -1122,6 +1276,7 @@ extern "C" int mcx_get_pass(const mcx_engine *e) {
   if (!e) return -1;
   if (e->staged) return MCX_PASS_STAGED;
   if (!e->march) return MCX_PASS_DIRECT;
+  if (e->resident) return MCX_PASS_RESIDENT;
   if (e->pmarch) return MCX_PASS_MARCH_PERSISTENT;
   if (e->qmarch) return MCX_PASS_MARCH_QUAD;
   return e->tmarch ? MCX_PASS_MARCH_TMA : (e->amarch ? MCX_PASS_MARCH_ASYNC : MCX_PASS_MARCH);
@@ -1225,12 +1380,12 @@ extern "C" mcx_status mcx_set_march_shape(mcx_engine *e, int block, int planes) 
   if (e->pmarch && !pmarch_block_ok(block))
     return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march runs blocks of 128 or 256 threads");
   CK(e, cudaStreamSynchronize(e->stream));
+  e->resident = false;  // a shape is asked for: the z-march runs it
   return apply_march_shape(e, block, planes);
 }
 
 static void launch_march_form(mcx_engine *e, int form, const PassArgs &pa, int nt) {
-  if (form == 1) launch_tmarch(e->var, MODE_SWEEP, pa, nt, e->pdl, e->stream);
-  else if (form == 2) launch_amarch(e->var, MODE_SWEEP, pa, nt, e->pdl, e->stream);
+  if (form == 2) launch_amarch(e->var, MODE_SWEEP, pa, nt, e->pdl, e->stream);
   else if (form == 4) launch_qmarch(e->var, MODE_SWEEP, pa, nt, e->pdl, e->stream);
   else launch_march(e->var, MODE_SWEEP, pa, nt, e->pdl, e->stream);
 }
@@ -1250,8 +1405,9 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
   cudaEvent_t t0, t1;
   mcx_status st = MCX_OK;
   int best_nt = e->march_nt, best_k = e->march_k,
-      best_form = e->pmarch ? 3 : (e->tmarch ? 1 : (e->amarch ? 2 : (e->qmarch ? 4 : 0)));
+      best_form = e->resident ? 5 : (e->pmarch ? 3 : (e->tmarch ? 1 : (e->amarch ? 2 : (e->qmarch ? 4 : 0))));
   float best = 1e30f;
+  e->resident = false;
 #define CKA(call)                                                                                    \
   do {                                                                                               \
     cudaError_t _r = (call);                                                                         \
@@ -1271,34 +1427,26 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
   {
     const int nts[3] = {64, 128, 256};
     const int ks[10] = {1, 2, 4, 8, 16, 32, 0, -2, -3, -4};  // fixed depths, then balanced over 1..4 waves
-    // forms: 0 the register march, 1 rows staged by bulk copies, 2 the per-thread prefetch,
-    // 3 one cooperative launch per run of sweeps (one wave of units: a single shape per block size),
-    // 4 four sites per thread
-    for (int form = 0; form < 5; form++)
+    // forms: 0 the register march, 2 the per-thread prefetch, 4 four sites per
+    // thread (the TMA-staged form, 1, and the persistent one, 3, measured slower
+    // than these on every lattice and are not timed)
+    for (int form : {0, 2, 4})
     for (int a = 0; a < 3; a++)
       for (int ki = 0; ki < 10; ki++) {
         const int k = ks[ki];
         if (k > maxnz && k > 1) continue;
-        if (form == 3 && (k != 0 || !pmarch_block_ok(nts[a]) || pmarch_blocks_per_sm(e->var, nts[a]) == 0)) continue;
-        e->tmarch = form == 1;
+        e->tmarch = e->pmarch = false;
         e->amarch = form == 2;
-        e->pmarch = form == 3;
         e->qmarch = form == 4;
         if ((st = apply_march_shape(e, nts[a], k))) goto done;
-        if ((form == 1 && !e->tmarch) || (form == 2 && !e->amarch) || (form == 3 && !pmarch_fits(e)) ||
-            (form == 4 && !e->qmarch))
-          continue;  // the form cannot run this batch
+        if ((form == 2 && !e->amarch) || (form == 4 && !e->qmarch)) continue;  // the form cannot run this batch
         PassArgs pa = pass_args(e);
         pa.dir = d_dir;
         pa.st = d_st;
         pa.stats = d_stats;
         pa.ring = d_ring;
         const int reps = 8;
-        if (form == 3) {
-          CKA(launch_pmarch(e->var, MODE_SWEEP, pa, nts[a], 2, e->d_err + 1, e->stream));
-          CKA(cudaEventRecord(t0, e->stream));
-          CKA(launch_pmarch(e->var, MODE_SWEEP, pa, nts[a], reps, e->d_err + 1, e->stream));
-        } else {
+        {
           for (int w = 0; w < 2; w++)
             for (int c = 0; c < 2; c++) {
               pa.colour = c;
@@ -1325,7 +1473,32 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
           best_form = form;
         }
       }
+    // the resident form at its planned shape (its time includes a run's load
+    // and store of the lattice, over as many sweeps as above)
+    if (plan_resident(e) > 0.0) {
+      PassArgs pa = pass_args(e);
+      pa.dir = d_dir;
+      pa.st = d_st;
+      pa.stats = d_stats;
+      pa.ring = d_ring;
+      const int reps = 32;
+      for (int w = 0; w < 2; w++) {
+        CKA(cudaEventRecord(t0, e->stream));
+        CKA(launch_resident(e->var, MODE_SWEEP, pa, e->d_cut, e->nrep, reps, e->res_c, e->res_nt, e->res_smem, e->stream));
+        CKA(cudaEventRecord(t1, e->stream));
+        CKA(cudaEventSynchronize(t1));
+        e->launches++;
+      }
+      float ms = 0.f;
+      CKA(cudaEventElapsedTime(&ms, t0, t1));
+      const float us = ms * 1e3f / (2 * reps);
+      if (us < best) {
+        best = us;
+        best_form = 5;
+      }
+    }
   }
+  e->resident = best_form == 5;
   e->tmarch = best_form == 1;
   e->amarch = best_form == 2;
   e->pmarch = best_form == 3;

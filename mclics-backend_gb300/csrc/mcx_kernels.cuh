@@ -134,6 +134,16 @@ bool pmarch_block_ok(int nt);
 int pmarch_blocks_per_sm(const Variant &v, int nt);
 cudaError_t launch_pmarch(const Variant &v, int mode, const PassArgs &a, int nt, int nsweeps, unsigned *bar,
                           cudaStream_t st, unsigned extra = 0);
+// The sweeps of small lattices resident in shared memory, one cluster of C
+// CTAs per replica and one launch per run of sweeps (mcx_resident.cu).
+// cut: per replica the first row (j + ny k) of each of its C CTAs, the row
+// count and the largest share; every share spans at least one plane.
+long long resident_smem_bytes(const RepDev &R, bool mask, int n);
+int resident_max_threads();
+constexpr int kResidentSmem = 220 * 1024;  // dynamic shared memory of a CTA, below the 227 KB limit
+int resident_clusters(const Variant &v, int C, int nt, int smem);
+cudaError_t launch_resident(const Variant &v, int mode, const PassArgs &a, const int *cut, int nrep, int nsweeps,
+                            int C, int nt, int smem, cudaStream_t st);
 // The learned-proposal z-march (mcx_lmarch.cu): units of lmarch_block_threads()
 // pairs; lmarch_prepare sets its shared memory and checks residency.  tc: the
 // network on the tcgen05 tensor cores (else the warp-level mma.sync code).

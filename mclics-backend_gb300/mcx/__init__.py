@@ -31,7 +31,7 @@ ANCHORINGS = {"homeotropic": 0, "fg": 1, "rp": 2, "strong": 3, "homeotropic_ghrl
               "strong_ghrl": 7}
 PROPOSALS = {"plain": 0, "vmf_mlp": 1}
 PASSES = {"march": 0, "direct": 1, "staged": 2, "march_tma": 3, "march_async": 4, "march_persistent": 5,
-          "march_quad": 6}
+          "march_quad": 6, "resident": 7}
 MLP_PARAMS = 6792
 SAMPLE_FLOATS = 24
 AUG_FLIP, AUG_ROTATE = 1, 2
