@@ -10,6 +10,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <functional>
 #include <string>
 #include <vector>
 
@@ -1142,9 +1143,11 @@ static double plan_resident(mcx_engine *e) {
 }
 
 // Whether the sweeps' kernels leave the inactive sites' field energy to
-// k_idle_field: the plain z-march and resident sweeps of a masked batch.
+// k_idle_field: the z-march (plain or learned) and resident sweeps of a masked
+// batch.
 static bool idle_field(const mcx_engine *e) {
-  return e->var.mask && e->var.field && e->march && !e->staged && e->proposal == MCX_PROPOSAL_PLAIN;
+  return e->var.mask && e->var.field && e->march &&
+         (e->proposal == MCX_PROPOSAL_PLAIN ? !e->staged : e->lmarch_ok);
 }
 
 static mcx_status run_sweeps(mcx_engine *e, int n, int m) {
@@ -1288,24 +1291,66 @@ extern "C" mcx_status mcx_set_staged(mcx_engine *e, int on) {
 
 extern "C" int mcx_get_staged(const mcx_engine *e) { return e && e->staged ? 1 : 0; }
 
-// Re-plans the z-march units for a block size and chunk depth and uploads
-// them with the replicas' CTA counts.
+// Chunk depth of the learned z-march: the one whose units, dealt in launch
+// order to the CTAs the GPU holds at once, finish first (a unit costs its
+// planes and about a third of a plane for its weights and set-up; a unit
+// without an active site nothing).  A fixed depth of 8 left the second of two
+// waves 58% idle on 4 x 96^3.
+static int learn_depth(const mcx_engine *e, int nt, int slots) {
+  int maxnz = 1;
+  for (const RepDev &R : e->rep) maxnz = std::max(maxnz, R.nz);
+  double best = 1e300;
+  int best_d = 1;
+  std::vector<double> busy;
+  for (int n = 1; n <= std::min(maxnz, 32); n++) {
+    const int d = (maxnz + n - 1) / n;
+    if (n > 1 && d == (maxnz + n - 2) / (n - 1)) continue;
+    // slots as a heap of the times they fall free (the earliest first)
+    busy.assign(slots, 0.0);
+    double end = 0.0;
+    for (int r = 0; r < e->nrep; r++) {
+      const RepDev &R = e->rep[r];
+      const int npp = R.hp * R.ny, chunks = (R.nz + d - 1) / d;
+      for (int q = 0; q < chunks; q++) {
+        const int k0 = (int)((long long)q * R.nz / chunks), k1 = (int)((long long)(q + 1) * R.nz / chunks);
+        for (int p0 = 0; p0 < npp; p0 += nt) {
+          if (e->var.mask && unit_class(e, make_int4(r, p0, k0, k1 - k0), nt) == kUnitDead) continue;
+          std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+          busy.back() += (k1 - k0) + 0.3;
+          end = std::max(end, busy.back());
+          std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+        }
+      }
+    }
+    if (end < best) {
+      best = end;
+      best_d = d;
+    }
+  }
+  return best_d;
+}
+
 // Units of the learned-proposal z-march: per replica, blocks of its CTA size
-// of a plane's pairs times chunks of kLearnPlanes planes; uploads them and the
-// replicas' CTA counts.
-constexpr int kLearnPlanes = 8;
+// of a plane's pairs times chunks of near-equal depth (learn_depth); uploads
+// them and the replicas' CTA counts.
 static mcx_status plan_lmarch(mcx_engine *e) {
   e->lunits.clear();
   const int nt = lmarch_block_threads();
+  int dev = 0, nsm = 0;
+  CK(e, cudaGetDevice(&dev));
+  CK(e, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+  const int d = learn_depth(e, nt, std::max(1, nsm * lmarch_blocks_per_sm(e->var, e->ltc)));
   for (int r = 0; r < e->nrep; r++) {
     RepDev &R = e->rep[r];
-    const int npp = R.hp * R.ny, K = std::min(kLearnPlanes, R.nz);
+    const int npp = R.hp * R.ny, chunks = (R.nz + d - 1) / d;
     R.lcta = 0;
-    for (int k0 = 0; k0 < R.nz; k0 += K)
+    for (int q = 0; q < chunks; q++) {
+      const int k0 = (int)((long long)q * R.nz / chunks), k1 = (int)((long long)(q + 1) * R.nz / chunks);
       for (int p0 = 0; p0 < npp; p0 += nt) {
-        e->lunits.push_back(make_int4(r, p0, k0, std::min(K, R.nz - k0)));
+        e->lunits.push_back(make_int4(r, p0, k0, k1 - k0));
         R.lcta++;
       }
+    }
   }
   for (int4 &u : e->lunits) u.w |= unit_class(e, u, nt) == kUnitDead ? kUnitDead : 0;
   cudaFree(e->d_lunits);

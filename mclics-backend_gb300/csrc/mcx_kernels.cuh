@@ -148,6 +148,7 @@ cudaError_t launch_resident(const Variant &v, int mode, const PassArgs &a, const
 // pairs; lmarch_prepare sets its shared memory and checks residency.  tc: the
 // network on the tcgen05 tensor cores (else the warp-level mma.sync code).
 int lmarch_block_threads();
+int lmarch_blocks_per_sm(const Variant &v, bool tc);
 bool lmarch_prepare(const Variant &v, bool tc);
 void launch_lmarch(const Variant &v, int mode, const PassArgs &a, bool pdl, bool tc, cudaStream_t st);
 // The direct pass with the learned proposal (mcx_learned.cu).

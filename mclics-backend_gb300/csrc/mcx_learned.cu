@@ -99,6 +99,13 @@ void pack_mlp_weights(const float *flat, uint8_t *out) {
   memcpy(out + kMlpB1, b1, kMlpH * 4);
   memcpy(out + kMlpB2, b2, kMlpH * 4);
   memcpy(out + kMlpB3, b3, kMlpOut * 4);
+  for (int nt = 0; nt < 8; nt++)
+    for (int tg = 0; tg < 4; tg++)
+      for (int r = 0; r < 4; r++) {
+        const size_t at = ((size_t)(nt * 4 + tg) * 4 + r) * 4;
+        memcpy(out + kMlpC1 + at, b1 + nt * 8 + 2 * tg + (r & 1), 4);
+        memcpy(out + kMlpC2 + at, b2 + nt * 8 + 2 * tg + (r & 1), 4);
+      }
 }
 
 }  // namespace mcx

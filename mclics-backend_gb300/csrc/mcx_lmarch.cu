@@ -2,17 +2,26 @@
 // the reference).
 //
 //   k_lmarch  the z-march of mcx_march.cu with the learned proposal: per
-//             plane every thread loads its pair's neighbourhood into
-//             registers (the z neighbours come from the march), writes the two
-//             sites' network inputs as rows 2*lane and 2*lane+1 of its warp's
+//             plane every thread loads its pair's neighbourhood, writes the two
+//             sites' network inputs as rows lane and lane+32 of its warp's
 //             64-row tile, the warp evaluates the network on the tensor cores
-//             (mlp_warp, mcx_mlp.cuh), and each thread draws and accepts its
-//             sites' moves (site_update_learned, mcx_pass.cuh).  The network is
-//             warp-synchronous, so every lane runs every plane: a thread past
-//             the end of the plane contributes zero rows and updates nothing.
-//             No shared-memory staging of neighbourhoods: 40 KB per CTA
-//             (weights and one input/output tile per warp), four CTAs of 128
-//             threads per SM at 128 registers.
+//             (mlp_warp, mcx_mlp.cuh), and each thread loads the neighbourhood
+//             again, draws and accepts its sites' moves
+//             (update_pair_learned).  The network is warp-synchronous, so every
+//             lane runs every plane: a thread past the end of the plane
+//             contributes zero rows and updates nothing.  41 KB of shared memory
+//             per CTA (weights and one input/output tile per warp), four CTAs of
+//             128 threads per SM at 128 registers.
+//
+//             What bounded it: shared-memory wavefronts (60% of peak, the
+//             network's weight fragments) and the issue of 44 warp instructions
+//             per site.  Two row tiles now share each weight fragment; for their
+//             registers the neighbourhood is not held across the network but
+//             read a second time (L2, 7% busy).  Bonds and energies run packed
+//             (mcx_packed.cuh).  4 x LL 96^3: 123.5 -> 112.4 us a pass (37
+//             instructions per site, wavefronts 41%); 6 droplets of 64^3, whose
+//             chunks of 8 planes also left the last wave idle (learn_depth,
+//             mcx_engine.cu): 85 -> 50 us, measured 100 -> 55.
 //
 //             With TC the network runs on the 5th-generation tensor cores
 //             instead (tc_mlp, mcx_tcmlp.cuh): per plane the CTA's 128
@@ -22,11 +31,9 @@
 //             columns of the CTA and every thread reads back its own rows.
 //             63 KB of shared memory per CTA (three CTAs per SM).
 //
-// It computes what the learned direct pass (k_pass<LEARN>) computes: the
-// same rows reach the network, the same per-site Philox counters drive the
-// draws.  Results agree bit for bit except where a decision lies within an
-// ulp of its threshold: the compiler fuses multiply-adds per kernel, so such
-// a decision (about one in 10^7-10^8 updates) can go the other way.
+// It computes what the learned direct pass (k_pass<LEARN>) computes, bit for
+// bit: the same rows reach the network, the same per-site Philox counters drive
+// the draws, and the energies keep the scalar update's roundings.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
@@ -44,10 +51,105 @@ constexpr uint32_t kLmarchTcCols = 128;  // two tiles of 64 FP32 accumulator col
 #define MCX_LMARCH_MIN_BLOCKS 4
 #endif
 
+// A pair's neighbourhood as loaded for plane k.
+struct Hood {
+  OPair o0, yp, ym, op, om;
+  float ex[3];
+  uint8_t pex;
+};
+
+template <bool MASK>
+__device__ __forceinline__ void load_hood(const March &m, int up, int down, bool zp, bool zm, Hood &h) {
+  const int dx = m.s ? m.dx1 : m.dx0;
+  load_opair_at<MASK>(m, m.off, m.offp, true, h.o0);
+  load_opair_at<MASK>(m, m.off + m.dyp, m.offp + m.dypp, true, h.yp);
+  load_opair_at<MASK>(m, m.off + m.dym, m.offp + m.dymp, true, h.ym);
+  load_opair_at<MASK>(m, m.off + up * m.dz, m.offp + up * m.dzp, zp, h.op);
+  load_opair_at<MASK>(m, m.off - down * m.dz, m.offp - down * m.dzp, zm, h.om);
+  h.ex[0] = ldo1(m.O0 + m.off + dx);
+  h.ex[1] = ldo1(m.O1 + m.off + dx);
+  h.ex[2] = ldo1(m.O2 + m.off + dx);
+  h.pex = 1;
+  if (MASK) h.pex = __ldg(m.PO + m.offp + dx);
+}
+
+template <bool MASK, bool PER>
+__device__ __forceinline__ PairSlots hood_slots(const March &m, const Hood &h, uint16_t pself, bool zp, bool zm) {
+  return pair_slots<MASK, PER>(m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, h.o0, h.yp, h.ym, h.op, h.om, h.ex, pself,
+                               h.pex, zp, zm, m.tail);
+}
+
+// The network input rows of both sites (feature_words): the six neighbours
+// (absent or inactive ones as zero vectors), T and a zero, as BF16 pairs; zero
+// rows for sites that are not there.
+__device__ __forceinline__ void pair_features(const PairSlots &S, float T, bool liveA, bool liveB, uint32_t rA[16],
+                                              uint32_t rB[16]) {
+  float fA[20], fB[20];
+  const f32x2 live = pk(liveA ? 1.f : 0.f, liveB ? 1.f : 0.f);
+#pragma unroll
+  for (int d = 0; d < 6; d++) {
+    const f32x2 w = pk(liveA ? S.wA[d] : 0.f, liveB ? S.wB[d] : 0.f);
+    const float2 x = unpk(mul2(S.nb[d].x, w)), y = unpk(mul2(S.nb[d].y, w)), z = unpk(mul2(S.nb[d].z, w));
+    fA[3 * d] = x.x; fA[3 * d + 1] = y.x; fA[3 * d + 2] = z.x;
+    fB[3 * d] = x.y; fB[3 * d + 1] = y.y; fB[3 * d + 2] = z.y;
+  }
+  const float2 t = unpk(mul2(live, pk1(T)));
+  fA[18] = t.x;
+  fB[18] = t.y;
+  fA[19] = fB[19] = 0.f;
+#pragma unroll
+  for (int q = 0; q < 10; q++) {
+    rA[q] = pack_bf16(fA[2 * q], fA[2 * q + 1]);
+    rB[q] = pack_bf16(fB[2 * q], fB[2 * q + 1]);
+  }
+#pragma unroll
+  for (int q = 10; q < 16; q++) rA[q] = rB[q] = 0u;
+}
+
+// One site's draw from the network's mixture.
+struct Drawn {
+  float mu[3], kappa, v[3], u;
+};
+__device__ __forceinline__ void draw_site(const RepDev &R, const float4 &y4, uint32_t nat, unsigned long long sw,
+                                          Drawn &d) {
+  const float y[4] = {y4.x, y4.y, y4.z, y4.w};
+  const uint4 r = philox4x32_10(make_uint4(nat, (uint32_t)sw, (uint32_t)(sw >> 32), TAG_VMF), R.seed, R.stream);
+  vmf_params(y, d.mu, d.kappa);
+  vmf_sample(d.mu, d.kappa, u01(r.x), u01(r.y), u01(r.z), d.v);
+  d.u = u01(r.w);
+}
+
+// The learned update of a pair (site_update_learned for both sites): the draws
+// site by site, everything between them in packed arithmetic with the scalar
+// update's roundings.
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
+__device__ __forceinline__ void update_pair_learned(const PassArgs &a, const RepDev &R, int c, const PairSlots &S,
+                                                    const float4 &yA, const float4 &yB, uint32_t nat, long long ns_at,
+                                                    unsigned long long sw, float invT, float2 &ax, float2 &ay,
+                                                    float2 &az, unsigned &acc, Q &sums) {
+  constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
+  const V2 n = {pk(ax), pk(ay), pk(az)};
+  Drawn A = {{0.f, 0.f, 1.f}, 0.f, {0.f, 0.f, 1.f}, 1.f}, B = A;
+  if (!MASK || S.actA) draw_site(R, yA, nat, sw, A);
+  if (!MASK || S.actB) draw_site(R, yB, nat + 2u, sw, B);
+  const V2 p = {pk(A.v[0], B.v[0]), pk(A.v[1], B.v[1]), pk(A.v[2], B.v[2])};
+  const V2 mu = {pk(A.mu[0], B.mu[0]), pk(A.mu[1], B.mu[1]), pk(A.mu[2], B.mu[2])};
+  const PairEnergy E = pair_energy<POT, MASK, FIELD, MEAS, PER>(a, R, c, ns_at, S, n, p, ax, ay, az);
+  const f32x2 kap = pk(A.kappa, B.kappa);
+  const float2 co = unpk(mul2(kap, dot2(mu, n))), cn = unpk(mul2(kap, dot2(mu, p)));
+  const f32x2 lo = pk(log_cosh_shift(co.x), log_cosh_shift(co.y));
+  const f32x2 ln = pk(log_cosh_shift(cn.x), log_cosh_shift(cn.y));
+  const float2 lr = unpk(sub2(fma2(E.dE, pk1(-invT), lo), ln));
+  const bool accA = S.actA && A.u < __expf(lr.x), accB = S.actB && B.u < __expf(lr.y);
+  accept_pair(accA, accB, p, ax, ay, az);
+  acc += (accA ? 1u : 0u) + (accB ? 1u : 0u);
+  if (MEAS) measure_pair<POT, MASK, FIELD, PER>(R, c, S, E, accA, accB, ax, ay, az, sums);
+}
+
 // the tensor-core form holds 63 KB of shared memory: three CTAs per SM, so
 // each thread may use up to 170 registers.  ODD: the batch holds an odd nx
 // (phantom slots, odd_tail); built only for masked batches that need it.
-template <int POT, bool MASK, bool FIELD, int MODE, bool TC, bool ODD>
+template <int POT, bool MASK, bool FIELD, int MODE, bool TC, bool ODD, bool PER>
 __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch(PassArgs a) {
   static_assert(MODE == MODE_SWEEP || MODE == MODE_SWEEP_MEASURE, "sweep modes only");
   extern __shared__ __align__(1024) uint8_t dyn[];
@@ -74,6 +176,7 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
   } else {
     for (int i = threadIdx.x; i < kMlpBytes / 16; i += kLPB)
       reinterpret_cast<int4 *>(W)[i] = reinterpret_cast<const int4 *>(a.mlp)[i];
+    clear_row_tails(X, lane);
   }
   const int4 u = a.units[blockIdx.x];
   const int r = u.x, c = a.colour;
@@ -88,165 +191,83 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
   const bool zper = R.zb == BOUND_PERIODIC;
   const int kb = u.z, ke = u.z + (u.w & kUnitPlanes);
   unsigned acc = 0;
-  float qs[kQ];
-#pragma unroll
-  for (int q = 0; q < kQ; q++) qs[q] = 0.f;
+  PairSums<MASK> sums;
+  sums.clear();
   __syncthreads();  // weights in shared memory
   if (TC) {
     tc_fence_after();
     tmem = *tslot;
   }
   grid_dependency_wait(m);
-  if (MASK && (u.w & kUnitDead)) {  // no active site in or next to the unit: field energies only
-    if (valid) dead_unit<FIELD, MODE>(R, m, kb, ke, qs);
-  } else {
-  const unsigned long long sw = S->sweep;
-  const float T = S->T, invT = 1.0f / S->T;
-  OPair om, o0, op;
-  const bool zm0 = kb > 0 || zper;
-  {
-    const int wrap = kb == 0 ? nz : 0;
-    load_opair_at<MASK>(m, m.off + (wrap - 1) * m.dz, m.offp + (wrap - 1) * m.dzp, zm0, om);
-    load_opair_at<MASK>(m, m.off, m.offp, true, o0);
-  }
-  bool zm = zm0;
-  auto wt = [&](float ee, uint8_t pp) { return MASK ? (ee != 0.f && pp != 0 ? 1.f : 0.f) : ee; };
+  if (!(MASK && (u.w & kUnitDead))) {  // a dead unit: no active site in or next to it
+    const unsigned long long sw = S->sweep;
+    const float T = S->T, invT = 1.0f / S->T;
 #pragma unroll 1
-  for (int k = kb; k < ke; k++) {
-    const bool zp = k + 1 < nz || zper;
-    const int up = k + 1 < nz ? 1 : 1 - nz;
-    load_opair_at<MASK>(m, m.off + up * m.dz, m.offp + up * m.dzp, zp, op);
-    const int dx = m.s ? m.dx1 : m.dx0;
-    uint16_t pself = 0x0101;
-    if (MASK) pself = __ldg(reinterpret_cast<const uint16_t *>(m.PA + m.offp));
-    // a warp whose 64 sites are all inactive: nothing moves, so it needs no
-    // network, and in an unmeasured sweep nothing is measured either, so it
-    // skips the updates too (the tensor-core form evaluates the network per
-    // CTA and does not skip)
-    const bool idle = !TC && MASK && __all_sync(0xffffffffu, !valid || pself == 0);
-    const bool skip = idle && MODE == MODE_SWEEP;
-    if (!skip) {
-    float2 ax = *reinterpret_cast<const float2 *>(m.A0 + m.off);
-    float2 ay = *reinterpret_cast<const float2 *>(m.A1 + m.off);
-    float2 az = *reinterpret_cast<const float2 *>(m.A2 + m.off);
-    const float exv[3] = {ldo1(m.O0 + m.off + dx), ldo1(m.O1 + m.off + dx), ldo1(m.O2 + m.off + dx)};
-    OPair yp, ym;
-    load_opair_at<MASK>(m, m.off + m.dyp, m.offp + m.dypp, true, yp);
-    load_opair_at<MASK>(m, m.off + m.dym, m.offp + m.dymp, true, ym);
-    uint8_t pex = 1;
-    if (MASK) pex = __ldg(m.PO + m.offp + dx);
-    const int s = m.s;
-    const float exe = s ? m.ee1 : m.ee0;
-    const float erz[4] = {m.eyp, m.eym, zp ? 1.f : 0.f, zm ? 1.f : 0.f};
-    const OPair *rows4[4] = {&yp, &ym, &op, &om};
-    const uint8_t lo = (uint8_t)(o0.pt & 0xFF), hi = (uint8_t)(o0.pt >> 8);
-    // neighbour slots x+ x- y+ y- z+ z- of both sites (as update_pair)
-    float nbA[6][3], wA[6], eA[6], nbB[6][3], wB[6], eB[6];
-    if (s == 0) {
-      nbA[0][0] = o0.v[0].x; nbA[0][1] = o0.v[1].x; nbA[0][2] = o0.v[2].x; eA[0] = 1.f; wA[0] = wt(1.f, lo);
-      nbA[1][0] = exv[0]; nbA[1][1] = exv[1]; nbA[1][2] = exv[2]; eA[1] = exe; wA[1] = wt(exe, pex);
-      nbB[0][0] = o0.v[0].y; nbB[0][1] = o0.v[1].y; nbB[0][2] = o0.v[2].y; eB[0] = 1.f; wB[0] = wt(1.f, hi);
-      nbB[1][0] = o0.v[0].x; nbB[1][1] = o0.v[1].x; nbB[1][2] = o0.v[2].x; eB[1] = 1.f; wB[1] = wt(1.f, lo);
-      // odd nx: the row's last site has no x+ bond (odd_tail, mcx_pass.cuh)
-      if (MASK && m.tail == 1) eA[0] = wA[0] = 0.f;
-      if (MASK && m.tail == 2) eB[0] = wB[0] = 0.f;
-    } else {
-      if (m.hasB) {
-        nbA[0][0] = o0.v[0].y; nbA[0][1] = o0.v[1].y; nbA[0][2] = o0.v[2].y; eA[0] = 1.f; wA[0] = wt(1.f, hi);
-      } else {
-        nbA[0][0] = exv[0]; nbA[0][1] = exv[1]; nbA[0][2] = exv[2]; eA[0] = exe; wA[0] = wt(exe, pex);
-      }
-      nbA[1][0] = o0.v[0].x; nbA[1][1] = o0.v[1].x; nbA[1][2] = o0.v[2].x; eA[1] = 1.f; wA[1] = wt(1.f, lo);
-      nbB[0][0] = exv[0]; nbB[0][1] = exv[1]; nbB[0][2] = exv[2]; eB[0] = exe; wB[0] = wt(exe, pex);
-      nbB[1][0] = o0.v[0].y; nbB[1][1] = o0.v[1].y; nbB[1][2] = o0.v[2].y; eB[1] = 1.f; wB[1] = wt(1.f, hi);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; q++) {
-      const OPair &o = *rows4[q];
-      nbA[2 + q][0] = o.v[0].x; nbA[2 + q][1] = o.v[1].x; nbA[2 + q][2] = o.v[2].x;
-      nbB[2 + q][0] = o.v[0].y; nbB[2 + q][1] = o.v[1].y; nbB[2 + q][2] = o.v[2].y;
-      eA[2 + q] = eB[2 + q] = erz[q];
-      wA[2 + q] = wt(erz[q], MASK ? (uint8_t)(o.pt & 0xFF) : 1);
-      wB[2 + q] = wt(erz[q], MASK ? (uint8_t)(o.pt >> 8) : 1);
-    }
-    const int psA = MASK ? (pself & 0xFF) : 1, psB = MASK ? (pself >> 8) : 1;
-    float yA[4], yB[4];
-    if (TC) {
-      // the network for the CTA's 256 sites: two M = 128 tiles on the tensor cores
-      uint32_t fw[16];
-      feature_words(nbA, wA, T, valid, fw);
-      tc_store_row32(TX, threadIdx.x, fw);
-      feature_words(nbB, wB, T, valid && m.hasB, fw);
-      tc_store_row32(TX + kTcXBytes, threadIdx.x, fw);
-      fence_proxy_async();
-      __syncthreads();
-      float y[2][4];
-      if (!tc_mlp(W, TX, TH, 2, tmem, tbar, tphase, y, a.err)) break;  // uniform: every thread saw the same waits
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        yA[q] = y[0][q];
-        yB[q] = y[1][q];
-      }
-    } else if (idle) {  // no active site: the outputs are never read
-#pragma unroll
-      for (int q = 0; q < 4; q++) yA[q] = yB[q] = 0.f;
-    } else {
-      // the network for the warp's 64 sites
-      __syncwarp();
-      write_features(X + (size_t)(2 * lane) * kXs, nbA, wA, T, valid);
-      write_features(X + (size_t)(2 * lane + 1) * kXs, nbB, wB, T, valid && m.hasB);
-      __syncwarp();
-      mlp_warp(W, X, Y);
-      __syncwarp();
-#pragma unroll
-      for (int q = 0; q < 4; q++) {
-        yA[q] = Y[(2 * lane) * 4 + q];
-        yB[q] = Y[(2 * lane + 1) * 4 + q];
-      }
-    }
-    if (valid) {
-      // odd nx: the phantom in the last slot of an s = 1 row is skipped
-      const bool skipA = MASK && s == 1 && m.tail == 1, skipB = MASK && s == 1 && m.tail == 2;
-      if (!skipA) {
-        float sx = 0.f, sy = 0.f, sz = 0.f;
-        if (MASK && psA > 1) {
-          const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * R.plane + m.off;
-          sx = __ldg(nsb);
-          sy = __ldg(nsb + R.plane);
-          sz = __ldg(nsb + 2 * R.plane);
+    for (int k = kb; k < ke; k++) {
+      const bool zp = k + 1 < nz || zper, zm = k > 0 || zper;
+      const int up = k + 1 < nz ? 1 : 1 - nz, down = k > 0 ? 1 : 1 - nz;
+      uint16_t pself = 0x0101;
+      if (MASK) pself = __ldg(reinterpret_cast<const uint16_t *>(m.PA + m.offp));
+      // a warp whose 64 sites are all inactive: nothing moves, so it needs no
+      // network, and only the colour-1 sites' bonds to active ones are measured
+      // (the tensor-core form evaluates the network per CTA and does not skip)
+      const bool idle = !TC && MASK && __all_sync(0xffffffffu, !valid || pself == 0);
+      if (!(idle && (MODE == MODE_SWEEP || c == 0))) {
+        float4 yA = make_float4(0.f, 0.f, 0.f, 0.f), yB = yA;
+        if (!idle) {
+          Hood h;
+          load_hood<MASK>(m, up, down, zp, zm, h);
+          const PairSlots sl = hood_slots<MASK, PER>(m, h, pself, zp, zm);
+          uint32_t rA[16], rB[16];
+          pair_features(sl, T, valid, valid && (PER || m.hasB), rA, rB);
+          if (TC) {
+            // the network for the CTA's 256 sites: two M = 128 tiles on the tensor cores
+            tc_store_row32(TX, threadIdx.x, rA);
+            tc_store_row32(TX + kTcXBytes, threadIdx.x, rB);
+            fence_proxy_async();
+            __syncthreads();
+            float y[2][4];
+            if (!tc_mlp(W, TX, TH, 2, tmem, tbar, tphase, y, a.err)) break;  // uniform: every thread saw the same waits
+            yA = make_float4(y[0][0], y[0][1], y[0][2], y[0][3]);
+            yB = make_float4(y[1][0], y[1][1], y[1][2], y[1][3]);
+          } else {
+            // the network for the warp's 64 sites
+            __syncwarp();
+            store_row(X, site_row(lane, 0), rA);  // words 10..15 are zeros that clear_row_tails wrote
+            store_row(X, site_row(lane, 1), rB);
+            __syncwarp();
+            mlp_warp(W, X, Y);
+            __syncwarp();
+            yA = reinterpret_cast<const float4 *>(Y)[site_row(lane, 0)];
+            yB = reinterpret_cast<const float4 *>(Y)[site_row(lane, 1)];
+          }
         }
-        const uint32_t nat = (uint32_t)(2 * m.h0 + s) + (uint32_t)nx * (uint32_t)m.row;
-        acc += site_update_learned<POT, MASK, FIELD, MODE>(R, a, c, ax.x, ay.x, az.x, nbA, wA, eA, psA, sx, sy, sz,
-                                                           yA, invT, nat, sw, qs);
-      }
-      if (m.hasB && !skipB) {
-        float sx = 0.f, sy = 0.f, sz = 0.f;
-        if (MASK && psB > 1) {
-          const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * R.plane + m.off + 1;
-          sx = __ldg(nsb);
-          sy = __ldg(nsb + R.plane);
-          sz = __ldg(nsb + 2 * R.plane);
+        if (valid) {
+          // the neighbourhood again: held in registers across the network it
+          // would cost the network its second row tile (spills)
+          Hood h;
+          load_hood<MASK>(m, up, down, zp, zm, h);
+          float2 ax = *reinterpret_cast<const float2 *>(m.A0 + m.off);
+          float2 ay = *reinterpret_cast<const float2 *>(m.A1 + m.off);
+          float2 az = *reinterpret_cast<const float2 *>(m.A2 + m.off);
+          const PairSlots sl = hood_slots<MASK, PER>(m, h, pself, zp, zm);
+          const uint32_t nat = (uint32_t)(2 * m.h0 + m.s) + (uint32_t)nx * (uint32_t)m.row;
+          update_pair_learned<POT, MASK, FIELD, MODE, PER>(a, R, c, sl, yA, yB, nat, m.off, sw, invT, ax, ay, az, acc,
+                                                           sums);
+          *reinterpret_cast<float2 *>(m.A0 + m.off) = ax;
+          *reinterpret_cast<float2 *>(m.A1 + m.off) = ay;
+          *reinterpret_cast<float2 *>(m.A2 + m.off) = az;
         }
-        const uint32_t nat = (uint32_t)(2 * m.h0 + 2 + s) + (uint32_t)nx * (uint32_t)m.row;
-        acc += site_update_learned<POT, MASK, FIELD, MODE>(R, a, c, ax.y, ay.y, az.y, nbB, wB, eB, psB, sx, sy, sz,
-                                                           yB, invT, nat, sw, qs);
       }
-      *reinterpret_cast<float2 *>(m.A0 + m.off) = ax;
-      *reinterpret_cast<float2 *>(m.A1 + m.off) = ay;
-      *reinterpret_cast<float2 *>(m.A2 + m.off) = az;
+      m.off += m.dz;
+      m.offp += m.dzp;
+      m.row += R.ny;
+      m.s ^= 1;
     }
-    }  // !skip
-    om = o0;
-    o0 = op;
-    zm = true;
-    m.off += m.dz;
-    m.offp += m.dzp;
-    m.pid += m.dpid;
-    m.row += R.ny;
-    m.s ^= 1;
-  }
   }
   grid_launch_dependents();
+  float qs[kQ];
+  sums.fold(qs);
   flush_replica<kLPB, MODE>(a, r, 1, (unsigned)R.lcta, acc, qs, MASK);
   if (TC) {  // every TMEM read is done (tc_mlp ends on a fenced barrier; flush_replica syncs again)
     tc_fence_after();
@@ -254,26 +275,23 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
   }
 }
 
-template <int POT, bool MASK, bool FIELD, bool TC, bool ODD = false>
+template <int POT, bool MASK, bool FIELD, bool TC, bool ODD, bool PER>
 static const void *lmarch_fn(int mode) {
-  return mode == MODE_SWEEP_MEASURE ? (const void *)k_lmarch<POT, MASK, FIELD, MODE_SWEEP_MEASURE, TC, ODD>
-                                    : (const void *)k_lmarch<POT, MASK, FIELD, MODE_SWEEP, TC, ODD>;
+  return mode == MODE_SWEEP_MEASURE ? (const void *)k_lmarch<POT, MASK, FIELD, MODE_SWEEP_MEASURE, TC, ODD, PER>
+                                    : (const void *)k_lmarch<POT, MASK, FIELD, MODE_SWEEP, TC, ODD, PER>;
 }
 
 template <int POT, bool FIELD, bool TC>
-static const void *lmarch_fn_masked(const Variant &v, int mode) {
-  return v.odd ? lmarch_fn<POT, true, FIELD, TC, true>(mode) : lmarch_fn<POT, true, FIELD, TC, false>(mode);
+static const void *lmarch_fn_v(const Variant &v, int mode) {
+  if (v.mask)
+    return v.odd ? lmarch_fn<POT, true, FIELD, TC, true, false>(mode) : lmarch_fn<POT, true, FIELD, TC, false, false>(mode);
+  return v.per ? lmarch_fn<POT, false, FIELD, TC, false, true>(mode) : lmarch_fn<POT, false, FIELD, TC, false, false>(mode);
 }
 
 template <bool TC>
 static const void *lmarch_kernel_tc(const Variant &v, int mode) {
-  if (v.pot == POT_LL) {
-    if (v.mask) return v.field ? lmarch_fn_masked<POT_LL, true, TC>(v, mode) : lmarch_fn_masked<POT_LL, false, TC>(v, mode);
-    return v.field ? lmarch_fn<POT_LL, false, true, TC>(mode) : lmarch_fn<POT_LL, false, false, TC>(mode);
-  }
-  if (v.mask)
-    return v.field ? lmarch_fn_masked<POT_GHRL, true, TC>(v, mode) : lmarch_fn_masked<POT_GHRL, false, TC>(v, mode);
-  return v.field ? lmarch_fn<POT_GHRL, false, true, TC>(mode) : lmarch_fn<POT_GHRL, false, false, TC>(mode);
+  if (v.pot == POT_LL) return v.field ? lmarch_fn_v<POT_LL, true, TC>(v, mode) : lmarch_fn_v<POT_LL, false, TC>(v, mode);
+  return v.field ? lmarch_fn_v<POT_GHRL, true, TC>(v, mode) : lmarch_fn_v<POT_GHRL, false, TC>(v, mode);
 }
 
 static const void *lmarch_kernel(const Variant &v, int mode, bool tc) {
@@ -283,6 +301,14 @@ static const void *lmarch_kernel(const Variant &v, int mode, bool tc) {
 static int lmarch_smem(bool tc) { return tc ? kLmarchTcSmem : kLmarchSmem; }
 
 int lmarch_block_threads() { return kLPB; }
+
+int lmarch_blocks_per_sm(const Variant &v, bool tc) {
+  int n = 0;
+  if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lmarch_kernel(v, MODE_SWEEP, tc), kLPB, lmarch_smem(tc)) !=
+      cudaSuccess)
+    return 0;
+  return n;
+}
 
 bool lmarch_prepare(const Variant &v, bool tc) {
   if (v.pot == POT_PEAR) return false;

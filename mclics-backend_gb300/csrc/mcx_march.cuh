@@ -80,27 +80,6 @@ __device__ __forceinline__ void grid_dependency_wait(March &m) {
                : "memory");
 }
 
-// A dead unit (kUnitDead) of the learned pass: in measured sweeps with a
-// field, each own (inactive) site adds its field energy, in the order the
-// full update adds it; nothing else.
-// The slot of a phantom site (odd nx, a row whose own sites are odd) is
-// skipped.
-template <bool FIELD, int MODE>
-__device__ __forceinline__ void dead_unit(const RepDev &R, March &m, int kb, int ke, float qs[kQ]) {
-  if (!(FIELD && MODE == MODE_SWEEP_MEASURE)) return;
-  int s = m.s;
-#pragma unroll 1
-  for (int k = kb; k < ke; k++) {
-    const float2 x = *reinterpret_cast<const float2 *>(m.A0 + m.off);
-    const float2 y = *reinterpret_cast<const float2 *>(m.A1 + m.off);
-    const float2 z = *reinterpret_cast<const float2 *>(m.A2 + m.off);
-    if (!(s && m.tail == 1)) qs[0] += field_energy(R, x.x, y.x, z.x);
-    if (m.hasB && !(s && m.tail == 2)) qs[0] += field_energy(R, x.y, y.y, z.y);
-    m.off += m.dz;
-    s ^= 1;
-  }
-}
-
 template <bool MASK>
 __device__ __forceinline__ void load_opair_at(const March &m, int off, int offp, bool on, OPair &o) {
   if (on) {
@@ -182,28 +161,29 @@ constexpr int march_min_blocks() {
                                 : (MCX_MARCH_MASK_REGS > 0 ? 65536 / (NT * MCX_MARCH_MASK_REGS) : 1);
 }
 
-// The update of one same-colour pair from its loaded neighbourhood (shared by
-// the z-march and its staged and prefetching forms): own directors (ax, ay,
-// az) in and out; o0 the opposite pair of the same row, yp / ym those of rows
-// y+1 / y-1, op / om those of the planes above / below (zp / zm: those bonds
-// exist), exv the extra x neighbour; s the parity of the own sites in this
-// row; rw the pair's Philox draw (pair_draw below).  Both sites run in packed
-// arithmetic (mcx_packed.cuh); a missing, phantom or inactive site's half is
-// computed and dropped.
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
-__device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev &R, int c, int s, bool hasB_,
-                                                 float ee0, float ee1, float eyp, float eym, const OPair &o0,
-                                                 const OPair &yp, const OPair &ym, const OPair &op, const OPair &om,
-                                                 const float exv[3], uint16_t pself, uint8_t pex, bool zp, bool zm,
-                                                 const uint4 rw, long long ns_at, float ang, float invT, float2 &ax,
-                                                 float2 &ay, float2 &az, unsigned &acc, Q &sums,
-                                                 int tail = 0) {
-  constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
+// The neighbourhood of a pair as the update uses it: the neighbours in slots
+// x+ x- y+ y- z+ z- of both sites, which bonds exist (e) and exist to an active
+// neighbour (w), and which of the two sites are there and active.
+struct PairSlots {
+  V2 nb[6];
+  f32x2 w[6];
+  float eA[6], eB[6], wA[6], wB[6];
+  bool hereA, hereB, actA, actB;
+  int psA, psB;
+};
+
+// Own parity s of the row; o0 the opposite pair of the same row, yp / ym those
+// of rows y+1 / y-1, op / om those of the planes above / below (zp / zm: those
+// bonds exist), exv the extra x neighbour.
+template <bool MASK, bool PER>
+__device__ __forceinline__ PairSlots pair_slots(int s, bool hasB_, float ee0, float ee1, float eyp, float eym,
+                                                const OPair &o0, const OPair &yp, const OPair &ym, const OPair &op,
+                                                const OPair &om, const float exv[3], uint16_t pself, uint8_t pex,
+                                                bool zp, bool zm, int tail) {
   constexpr bool W = !PER;  // PER: every bond exists (all axes periodic, pairs always complete)
   const bool hasB = PER || hasB_;
   // neighbour slots x+ x- y+ y- z+ z- of both sites
-  V2 nb[6];
-  f32x2 w[6];
+  PairSlots S;
   {
     f32x2 q0[3], q1[3];
 #pragma unroll
@@ -212,70 +192,86 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
       q0[q] = pk(s ? (hasB ? hi : ex) : lo, s ? ex : hi);
       q1[q] = pk(s ? lo : ex, s ? hi : lo);
     }
-    nb[0] = {q0[0], q0[1], q0[2]};
-    nb[1] = {q1[0], q1[1], q1[2]};
-    nb[2] = {pk(yp.v[0]), pk(yp.v[1]), pk(yp.v[2])};
-    nb[3] = {pk(ym.v[0]), pk(ym.v[1]), pk(ym.v[2])};
-    nb[4] = {pk(op.v[0]), pk(op.v[1]), pk(op.v[2])};
-    nb[5] = {pk(om.v[0]), pk(om.v[1]), pk(om.v[2])};
+    S.nb[0] = {q0[0], q0[1], q0[2]};
+    S.nb[1] = {q1[0], q1[1], q1[2]};
+    S.nb[2] = {pk(yp.v[0]), pk(yp.v[1]), pk(yp.v[2])};
+    S.nb[3] = {pk(ym.v[0]), pk(ym.v[1]), pk(ym.v[2])};
+    S.nb[4] = {pk(op.v[0]), pk(op.v[1]), pk(op.v[2])};
+    S.nb[5] = {pk(om.v[0]), pk(om.v[1]), pk(om.v[2])};
   }
   // bonds present (e) and present to an active neighbour (w), per site
-  float eA[6], eB[6], wA[6], wB[6];
   if (W) {
     const float exe = s ? ee1 : ee0;
     const float erz[4] = {eyp, eym, zp ? 1.f : 0.f, zm ? 1.f : 0.f};
-    eA[0] = s && !hasB ? exe : 1.f;
-    eB[0] = s ? exe : 1.f;
-    eA[1] = s ? 1.f : exe;
-    eB[1] = 1.f;
+    S.eA[0] = s && !hasB ? exe : 1.f;
+    S.eB[0] = s ? exe : 1.f;
+    S.eA[1] = s ? 1.f : exe;
+    S.eB[1] = 1.f;
     // odd nx (masked only): the last site of an s = 0 row has no x+ bond
-    if (MASK && s == 0 && tail == 1) eA[0] = 0.f;
-    if (MASK && s == 0 && tail == 2) eB[0] = 0.f;
+    if (MASK && s == 0 && tail == 1) S.eA[0] = 0.f;
+    if (MASK && s == 0 && tail == 2) S.eB[0] = 0.f;
 #pragma unroll
-    for (int q = 0; q < 4; q++) eA[2 + q] = eB[2 + q] = erz[q];
+    for (int q = 0; q < 4; q++) S.eA[2 + q] = S.eB[2 + q] = erz[q];
     if (MASK) {
       const uint8_t lo = (uint8_t)(o0.pt & 0xFF), hi = (uint8_t)(o0.pt >> 8);
       const uint16_t pr[4] = {yp.pt, ym.pt, op.pt, om.pt};
       auto wt = [](float e, uint8_t p) { return e != 0.f && p != 0 ? 1.f : 0.f; };
-      wA[0] = wt(eA[0], s ? (hasB ? hi : pex) : lo);
-      wB[0] = wt(eB[0], s ? pex : hi);
-      wA[1] = wt(eA[1], s ? lo : pex);
-      wB[1] = wt(eB[1], s ? hi : lo);
+      S.wA[0] = wt(S.eA[0], s ? (hasB ? hi : pex) : lo);
+      S.wB[0] = wt(S.eB[0], s ? pex : hi);
+      S.wA[1] = wt(S.eA[1], s ? lo : pex);
+      S.wB[1] = wt(S.eB[1], s ? hi : lo);
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        wA[2 + q] = wt(erz[q], (uint8_t)(pr[q] & 0xFF));
-        wB[2 + q] = wt(erz[q], (uint8_t)(pr[q] >> 8));
+        S.wA[2 + q] = wt(erz[q], (uint8_t)(pr[q] & 0xFF));
+        S.wB[2 + q] = wt(erz[q], (uint8_t)(pr[q] >> 8));
       }
     } else {
 #pragma unroll
       for (int d = 0; d < 6; d++) {
-        wA[d] = eA[d];
-        wB[d] = eB[d];
+        S.wA[d] = S.eA[d];
+        S.wB[d] = S.eB[d];
       }
     }
 #pragma unroll
-    for (int d = 0; d < 6; d++) w[d] = pk(wA[d], wB[d]);
+    for (int d = 0; d < 6; d++) S.w[d] = pk(S.wA[d], S.wB[d]);
   } else {
 #pragma unroll
-    for (int d = 0; d < 6; d++) eA[d] = eB[d] = wA[d] = wB[d] = 1.f;
+    for (int d = 0; d < 6; d++) S.eA[d] = S.eB[d] = S.wA[d] = S.wB[d] = 1.f;
   }
   // odd nx (masked only): a phantom in the last slot of an s = 1 row is skipped
-  const bool hereA = !(MASK && s == 1 && tail == 1), hereB = hasB && !(MASK && s == 1 && tail == 2);
-  const int psA = MASK ? (pself & 0xFF) : 1, psB = MASK ? (pself >> 8) : 1;
-  const bool actA = hereA && psA != 0, actB = hereB && psB != 0;
-  const V2 n = {pk(ax), pk(ay), pk(az)};
-  const V2 p = propose2(n, rw, ang);
-  f32x2 e_old, e_new, x[6], x_old = 0ull, x_new = 0ull;
+  S.hereA = !(MASK && s == 1 && tail == 1);
+  S.hereB = hasB && !(MASK && s == 1 && tail == 2);
+  S.psA = MASK ? (pself & 0xFF) : 1;
+  S.psB = MASK ? (pself >> 8) : 1;
+  S.actA = S.hereA && S.psA != 0;
+  S.actB = S.hereB && S.psB != 0;
+  return S;
+}
+
+// Energies of a pair's old and new directors: bond sums to active neighbours
+// (e; unscaled for LL), for a measured masked pass to inactive ones (x, weights
+// x[6]), anchoring (s) and field (f), and the energy change dE with every
+// rounding the scalar update's (site_update).
+struct PairEnergy {
+  f32x2 dE, e_old, e_new, x[6], x_old, x_new, s_old, s_new, f_old, f_new;
+};
+
+template <int POT, bool MASK, bool FIELD, bool MEAS, bool PER>
+__device__ __forceinline__ PairEnergy pair_energy(const PassArgs &a, const RepDev &R, int c, long long ns_at,
+                                                  const PairSlots &S, const V2 &n, const V2 &p, const float2 &ax,
+                                                  const float2 &ay, const float2 &az) {
+  PairEnergy E;
+  E.x_old = E.x_new = 0ull;
   if (MASK && MEAS) {  // bonds of active sites to inactive ones
 #pragma unroll
-    for (int d = 0; d < 6; d++) x[d] = pk(actA ? eA[d] - wA[d] : 0.f, actB ? eB[d] - wB[d] : 0.f);
+    for (int d = 0; d < 6; d++) E.x[d] = pk(S.actA ? S.eA[d] - S.wA[d] : 0.f, S.actB ? S.eB[d] - S.wB[d] : 0.f);
   }
-  bond_sums<POT, W, MASK && MEAS>(R, n, p, nb, w, e_old, e_new, x, x_old, x_new);
+  bond_sums<POT, !PER, MASK && MEAS>(R, n, p, S.nb, S.w, E.e_old, E.e_new, E.x, E.x_old, E.x_new);
   // every rounding of dE is the scalar update's (site_update)
-  f32x2 dE = sub2(e_new, e_old);
-  if (POT == POT_LL) dE = mul2(pk1(bond_scale<POT>(R)), dE);
-  f32x2 s_old = 0ull, s_new = 0ull, f_old = 0ull, f_new = 0ull;  // anchoring and field energies
-  if (MASK && (psA > 1 || psB > 1)) {  // surface sites
+  E.dE = sub2(E.e_new, E.e_old);
+  if (POT == POT_LL) E.dE = mul2(pk1(bond_scale<POT>(R)), E.dE);
+  E.s_old = E.s_new = E.f_old = E.f_new = 0ull;
+  if (MASK && (S.psA > 1 || S.psB > 1)) {  // surface sites
     const float *nsb = a.ns + R.ns_off + (long long)(c * 3) * R.plane + ns_at;
     // the quadratic anchorings W (n.v)^2 of both sites in packed arithmetic
     // (surface_energy's operations): v the surface normal or the easy axis, k
@@ -285,7 +281,7 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
     bool form[2] = {false, false};  // a GHRL-form anchoring: the general function
 #pragma unroll
     for (int b = 0; b < 2; b++) {
-      const int sid = (b ? psB : psA) - 2;
+      const int sid = (b ? S.psB : S.psA) - 2;
       if (sid < 0) continue;
 #pragma unroll
       for (int q = 0; q < 3; q++) sn[b][q] = __ldg(nsb + q * R.plane + b);
@@ -304,80 +300,111 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
     // n.v with the fusions the compiler gives surface_energy: x fused onto y
     const f32x2 cn = fma2(p.z, vv.z, fma2(p.x, vv.x, mul2(p.y, vv.y)));
     const f32x2 co = fma2(n.z, vv.z, fma2(n.x, vv.x, mul2(n.y, vv.y)));
-    s_new = mul2(mul2(kk, cn), cn);
-    s_old = mul2(mul2(kk, co), co);
+    E.s_new = mul2(mul2(kk, cn), cn);
+    E.s_old = mul2(mul2(kk, co), co);
     if (form[0] || form[1]) {
       const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
-      float2 en = unpk(s_new), eo = unpk(s_old);
+      float2 en = unpk(E.s_new), eo = unpk(E.s_old);
       if (form[0]) {
-        en.x = surface_energy(R, psA - 2, px.x, py.x, pz.x, sn[0][0], sn[0][1], sn[0][2]);
-        eo.x = surface_energy(R, psA - 2, ax.x, ay.x, az.x, sn[0][0], sn[0][1], sn[0][2]);
+        en.x = surface_energy(R, S.psA - 2, px.x, py.x, pz.x, sn[0][0], sn[0][1], sn[0][2]);
+        eo.x = surface_energy(R, S.psA - 2, ax.x, ay.x, az.x, sn[0][0], sn[0][1], sn[0][2]);
       }
       if (form[1]) {
-        en.y = surface_energy(R, psB - 2, px.y, py.y, pz.y, sn[1][0], sn[1][1], sn[1][2]);
-        eo.y = surface_energy(R, psB - 2, ax.y, ay.y, az.y, sn[1][0], sn[1][1], sn[1][2]);
+        en.y = surface_energy(R, S.psB - 2, px.y, py.y, pz.y, sn[1][0], sn[1][1], sn[1][2]);
+        eo.y = surface_energy(R, S.psB - 2, ax.y, ay.y, az.y, sn[1][0], sn[1][1], sn[1][2]);
       }
-      s_new = pk(en);
-      s_old = pk(eo);
+      E.s_new = pk(en);
+      E.s_old = pk(eo);
     }
-    dE = add2(dE, sub2(s_new, s_old));
+    E.dE = add2(E.dE, sub2(E.s_new, E.s_old));
   }
   if (FIELD) {
-    f_new = field_energy2(R, p);
-    f_old = field_energy2(R, n);
-    dE = add2(dE, sub2(f_new, f_old));
+    E.f_new = field_energy2(R, p);
+    E.f_old = field_energy2(R, n);
+    E.dE = add2(E.dE, sub2(E.f_new, E.f_old));
   }
-  // src/evolve.cpp:160: accept when u < exp(-(E_new - E_old)/T)
-  const float2 arg = unpk(mul2(dE, pk1(-invT))), u2 = accept_uniforms(rw);
-  const bool accA = actA && u2.x < __expf(arg.x), accB = actB && u2.y < __expf(arg.y);
+  return E;
+}
+
+// What a measured pass adds for a pair with its final directors (ax, ay, az).
+template <int POT, bool MASK, bool FIELD, bool PER, class Q>
+__device__ __forceinline__ void measure_pair(const RepDev &R, int c, const PairSlots &S, const PairEnergy &E, bool accA,
+                                             bool accB, const float2 &ax, const float2 &ay, const float2 &az, Q &sums) {
+  // the final directors and their energies.  Each bond counts in the local
+  // energy of each active end, from the colour-1 side; the all-site energy
+  // also counts inactive sites' bonds to active ones.  (The field energy of
+  // inactive sites is k_idle_field's.)
+  constexpr bool ALL = PER;  // both sites count
+  const V2 nf = {pk(ax), pk(ay), pk(az)};
+  const f32x2 m = pk(S.actA ? 1.f : 0.f, S.actB ? 1.f : 0.f);
+  add_q<ALL>(sums, nf, m);
+  f32x2 site = 0ull;
+  if (MASK) site = pick2(accA, accB, E.s_new, E.s_old);
+  if (FIELD) site = add2(site, pick2(accA, accB, E.f_new, E.f_old));
+  if ((MASK || FIELD) && !ALL) site = mul2(site, m);
+  f32x2 all = site, valid = site;
+  if (c == 1) {
+    f32x2 eb = pick2(accA, accB, E.e_new, E.e_old);
+    if (POT == POT_LL) eb = mul2(pk1(bond_scale<POT>(R)), eb);
+    eb = add_bond_const<POT, !PER>(R, S.w, eb);
+    if (ALL) {
+      all = fma2(pk1(2.f), eb, all);
+    } else {
+      const f32x2 k2 = pk(S.actA ? 2.f : (S.hereA ? 1.f : 0.f), S.actB ? 2.f : (S.hereB ? 1.f : 0.f));
+      all = fma2(k2, eb, all);
+      if (MASK) {
+        valid = fma2(mul2(pk1(2.f), m), eb, valid);
+        f32x2 xb = pick2(accA, accB, E.x_new, E.x_old);
+        if (POT == POT_LL) xb = mul2(pk1(bond_scale<POT>(R)), xb);
+        all = add2(all, add_bond_const<POT, true>(R, E.x, xb));
+      }
+    }
+  }
+  if (MASK || FIELD || c == 1) sums.add(0, all);
+  if (MASK) sums.add(1, valid);
+  else if (Q::kMasked && (FIELD || c == 1)) sums.add(1, all);  // a masked batch's bulk sites
+}
+
+__device__ __forceinline__ void accept_pair(bool accA, bool accB, const V2 &p, float2 &ax, float2 &ay, float2 &az) {
   const float2 px = unpk(p.x), py = unpk(p.y), pz = unpk(p.z);
   if (accA) {
     ax.x = px.x;
     ay.x = py.x;
     az.x = pz.x;
-    acc++;
   }
   if (accB) {
     ax.y = px.y;
     ay.y = py.y;
     az.y = pz.y;
-    acc++;
   }
-  if (MEAS) {
-    // the final directors and their energies.  Each bond counts in the local
-    // energy of each active end, from the colour-1 side; the all-site energy
-    // also counts inactive sites' bonds to active ones.  (The field energy of
-    // inactive sites is k_idle_field's.)
-    constexpr bool ALL = PER;  // both sites count
-    const V2 nf = {pk(ax), pk(ay), pk(az)};
-    const f32x2 m = pk(actA ? 1.f : 0.f, actB ? 1.f : 0.f);
-    add_q<ALL>(sums, nf, m);
-    f32x2 site = 0ull;
-    if (MASK) site = pick2(accA, accB, s_new, s_old);
-    if (FIELD) site = add2(site, pick2(accA, accB, f_new, f_old));
-    if ((MASK || FIELD) && !ALL) site = mul2(site, m);
-    f32x2 all = site, valid = site;
-    if (c == 1) {
-      f32x2 eb = pick2(accA, accB, e_new, e_old);
-      if (POT == POT_LL) eb = mul2(pk1(bond_scale<POT>(R)), eb);
-      eb = add_bond_const<POT, W>(R, w, eb);
-      if (ALL) {
-        all = fma2(pk1(2.f), eb, all);
-      } else {
-        const f32x2 k2 = pk(actA ? 2.f : (hereA ? 1.f : 0.f), actB ? 2.f : (hereB ? 1.f : 0.f));
-        all = fma2(k2, eb, all);
-        if (MASK) {
-          valid = fma2(mul2(pk1(2.f), m), eb, valid);
-          f32x2 xb = pick2(accA, accB, x_new, x_old);
-          if (POT == POT_LL) xb = mul2(pk1(bond_scale<POT>(R)), xb);
-          all = add2(all, add_bond_const<POT, true>(R, x, xb));
-        }
-      }
-    }
-    if (MASK || FIELD || c == 1) sums.add(0, all);
-    if (MASK) sums.add(1, valid);
-    else if (Q::kMasked && (FIELD || c == 1)) sums.add(1, all);  // a masked batch's bulk sites
-  }
+}
+
+// The update of one same-colour pair from its loaded neighbourhood (shared by
+// the z-march, its staged and prefetching forms and the resident sweeps): own
+// directors (ax, ay, az) in and out; the neighbourhood as in pair_slots; rw the
+// pair's Philox draw (pair_draw below).  Both sites run in packed arithmetic
+// (mcx_packed.cuh); a missing, phantom or inactive site's half is computed and
+// dropped.
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
+__device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev &R, int c, int s, bool hasB,
+                                                 float ee0, float ee1, float eyp, float eym, const OPair &o0,
+                                                 const OPair &yp, const OPair &ym, const OPair &op, const OPair &om,
+                                                 const float exv[3], uint16_t pself, uint8_t pex, bool zp, bool zm,
+                                                 const uint4 rw, long long ns_at, float ang, float invT, float2 &ax,
+                                                 float2 &ay, float2 &az, unsigned &acc, Q &sums,
+                                                 int tail = 0) {
+  constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
+  const PairSlots S = pair_slots<MASK, PER>(s, hasB, ee0, ee1, eyp, eym, o0, yp, ym, op, om, exv, pself, pex, zp, zm,
+                                            tail);
+  const V2 n = {pk(ax), pk(ay), pk(az)};
+  const V2 p = propose2(n, rw, ang);
+  const PairEnergy E = pair_energy<POT, MASK, FIELD, MEAS, PER>(a, R, c, ns_at, S, n, p, ax, ay, az);
+  // src/evolve.cpp:160: accept when u < exp(-(E_new - E_old)/T)
+  const float2 arg = unpk(mul2(E.dE, pk1(-invT))), u2 = accept_uniforms(rw);
+  const bool accA = S.actA && u2.x < __expf(arg.x), accB = S.actB && u2.y < __expf(arg.y);
+  accept_pair(accA, accB, p, ax, ay, az);
+  acc += (accA ? 1u : 0u) + (accB ? 1u : 0u);
+  if (MEAS) measure_pair<POT, MASK, FIELD, PER>(R, c, S, E, accA, accB, ax, ay, az, sums);
 }
 
 // The pair's Philox draw (counter: pair index, sweep, colour; key: seed,

@@ -13,6 +13,8 @@
 //   W2t [64][72] bf16   W2 transposed and halved (gelu_bf16x2 returns twice the GELU), 8 pad
 //   W3t [ 8][72] bf16   W3 transposed and halved (n = 0..7, outputs 4..7 zero)
 //   b1 [64], b2 [64], b3 [8] float
+//   c1 [32][4], c2 [32][4] float  per n-tile and lane of a quad the FP32 C
+//                      fragment {b, b', b, b'} that a layer's sums start from
 // The row pads keep the B-fragment loads of a warp on 32 distinct banks.
 #pragma once
 #include <cuda_bf16.h>
@@ -30,7 +32,10 @@ constexpr int kMlpW3 = kMlpW2 + kMlpH * kW2s * 2;
 constexpr int kMlpB1 = kMlpW3 + kMlpOut * kW3s * 2;
 constexpr int kMlpB2 = kMlpB1 + kMlpH * 4;
 constexpr int kMlpB3 = kMlpB2 + kMlpH * 4;
-constexpr int kMlpBytes = kMlpB3 + kMlpOut * 4;  // 16032
+constexpr int kMlpC1 = kMlpB3 + kMlpOut * 4;
+constexpr int kMlpC2 = kMlpC1 + 32 * 16;
+constexpr int kMlpBytes = kMlpC2 + 32 * 16;  // 17056
+static_assert(kMlpC1 % 16 == 0 && kMlpBytes % 16 == 0, "C fragments are read as 16-byte words");
 constexpr float kLogKMin = -4.0f, kLogKMax = 6.0f;
 
 __device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], uint32_t b0, uint32_t b1) {
@@ -39,6 +44,15 @@ __device__ __forceinline__ void mma_bf16(float d[4], const uint32_t a[4], uint32
       "{%0,%1,%2,%3};"
       : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
       : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// d = a b + c, c a fragment of its own (the bias)
+__device__ __forceinline__ void mma_bf16_c(float d[4], const uint32_t a[4], uint32_t b0, uint32_t b1, const float4 &c) {
+  asm volatile(
+      "mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+      "{%10,%11,%12,%13};"
+      : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+      : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(c.x), "f"(c.y), "f"(c.z), "f"(c.w));
 }
 
 __device__ __forceinline__ float tanh_approx(float x) {
@@ -98,89 +112,131 @@ __device__ __forceinline__ void ldsm_b2(const uint8_t *wt, int stride_elems, int
                : "r"(addr));
 }
 
+// A fragment of a 16 x 16 tile of X (rows r0.., columns k0..): four 8x8
+// matrices, rows 0-7 and 8-15 at k0, then both at k0 + 8.
+__device__ __forceinline__ void ldsm_a4(const __nv_bfloat16 *X, int r0, int k0, uint32_t a[4]) {
+  const int lane = threadIdx.x & 31;
+  const uint32_t addr =
+      (uint32_t)__cvta_generic_to_shared(X + (size_t)(r0 + (lane & 15)) * kXs + k0 + ((lane >> 4) << 3));
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+               : "=r"(a[0]), "=r"(a[1]), "=r"(a[2]), "=r"(a[3])
+               : "r"(addr));
+}
+
 // The network for 64 rows of X (bf16, row stride kXs) -> Y (64 x 4 floats),
 // by one warp.  Rows are sites; all 32 lanes must call.
+//
+// kMT 16-row tiles go through the layers together: a weight or bias fragment
+// is read once for all of them, and their GELU chains (six dependent packed
+// operations each) overlap.  Every accumulator starts from the bias fragment
+// as the first MMA's C operand, so no register is filled for it.
+constexpr int kMT = 2;
 __device__ __forceinline__ void mlp_warp(const uint8_t *W, const __nv_bfloat16 *X, float *Y) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
   const uint8_t *W1 = W + kMlpW1, *W2 = W + kMlpW2, *W3 = W + kMlpW3;
-  const float *b1 = reinterpret_cast<const float *>(W + kMlpB1);
-  const float *b2 = reinterpret_cast<const float *>(W + kMlpB2);
+  const float4 *c1 = reinterpret_cast<const float4 *>(W + kMlpC1) + tg;
+  const float4 *c2 = reinterpret_cast<const float4 *>(W + kMlpC2) + tg;
   const float *b3 = reinterpret_cast<const float *>(W + kMlpB3);
 #pragma unroll 1
-  for (int mt = 0; mt < 4; mt++) {
-    const __nv_bfloat16 *Xr = X + (size_t)(16 * mt) * kXs;
-    // layer 1: 2 k-tiles x 8 n-tiles
-    uint32_t a1[2][4];
+  for (int mt = 0; mt < 4; mt += kMT) {
+    uint32_t a2[kMT][4][4];  // layer-2 A fragments (k-tile q = layer-1 n-tiles 2q, 2q+1)
+    {
+      uint32_t a1[kMT][2][4];
 #pragma unroll
-    for (int kt = 0; kt < 2; kt++) {
-      a1[kt][0] = *reinterpret_cast<const uint32_t *>(Xr + g * kXs + kt * 16 + 2 * tg);
-      a1[kt][1] = *reinterpret_cast<const uint32_t *>(Xr + (g + 8) * kXs + kt * 16 + 2 * tg);
-      a1[kt][2] = *reinterpret_cast<const uint32_t *>(Xr + g * kXs + kt * 16 + 8 + 2 * tg);
-      a1[kt][3] = *reinterpret_cast<const uint32_t *>(Xr + (g + 8) * kXs + kt * 16 + 8 + 2 * tg);
-    }
-    uint32_t a2[4][4];  // layer-2 A fragments (k-tile q = layer-1 n-tiles 2q, 2q+1)
+      for (int t = 0; t < kMT; t++)
 #pragma unroll
-    for (int q = 0; q < 4; q++) {
-      float h[2][4];
+        for (int kt = 0; kt < 2; kt++) ldsm_a4(X, 16 * (mt + t), kt * 16, a1[t][kt]);
+      // layer 1: 2 k-tiles x 8 n-tiles
 #pragma unroll
-      for (int half = 0; half < 2; half++) {
-        const int nt = 2 * q + half;
-        const float bb0 = b1[nt * 8 + 2 * tg], bb1 = b1[nt * 8 + 2 * tg + 1];
-        h[half][0] = bb0;
-        h[half][1] = bb1;
-        h[half][2] = bb0;
-        h[half][3] = bb1;
+      for (int q = 0; q < 4; q++) {
+        const float4 ca = c1[(2 * q) * 4], cb = c1[(2 * q + 1) * 4];
+        uint32_t bf[2][4];
+        ldsm_b2(W1, kW1s, 16 * q, 0, bf[0]);
+        ldsm_b2(W1, kW1s, 16 * q, 16, bf[1]);
+#pragma unroll
+        for (int t = 0; t < kMT; t++) {
+          float h[2][4];
+          mma_bf16_c(h[0], a1[t][0], bf[0][0], bf[0][1], ca);
+          mma_bf16_c(h[1], a1[t][0], bf[0][2], bf[0][3], cb);
+          mma_bf16(h[0], a1[t][1], bf[1][0], bf[1][1]);
+          mma_bf16(h[1], a1[t][1], bf[1][2], bf[1][3]);
+          a2[t][q][0] = gelu_bf16x2(h[0][0], h[0][1]);
+          a2[t][q][1] = gelu_bf16x2(h[0][2], h[0][3]);
+          a2[t][q][2] = gelu_bf16x2(h[1][0], h[1][1]);
+          a2[t][q][3] = gelu_bf16x2(h[1][2], h[1][3]);
+        }
       }
-#pragma unroll
-      for (int kt = 0; kt < 2; kt++) {
-        uint32_t bf[4];
-        ldsm_b2(W1, kW1s, 16 * q, kt * 16, bf);
-        mma_bf16(h[0], a1[kt], bf[0], bf[1]);
-        mma_bf16(h[1], a1[kt], bf[2], bf[3]);
-      }
-      a2[q][0] = gelu_bf16x2(h[0][0], h[0][1]);
-      a2[q][1] = gelu_bf16x2(h[0][2], h[0][3]);
-      a2[q][2] = gelu_bf16x2(h[1][0], h[1][1]);
-      a2[q][3] = gelu_bf16x2(h[1][2], h[1][3]);
     }
     // layer 2 in pairs of n-tiles, each pair feeding one layer-3 k-tile
-    float y[4] = {0.f, 0.f, 0.f, 0.f};
+    float y[kMT][4];
+#pragma unroll
+    for (int t = 0; t < kMT; t++)
+#pragma unroll
+      for (int r = 0; r < 4; r++) y[t][r] = 0.f;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      float h[2][4];
-#pragma unroll
-      for (int half = 0; half < 2; half++) {
-        const int nt = 2 * q + half;
-        const float bb0 = b2[nt * 8 + 2 * tg], bb1 = b2[nt * 8 + 2 * tg + 1];
-        h[half][0] = bb0;
-        h[half][1] = bb1;
-        h[half][2] = bb0;
-        h[half][3] = bb1;
-      }
+      const float4 ca = c2[(2 * q) * 4], cb = c2[(2 * q + 1) * 4];
+      float h[kMT][2][4];
 #pragma unroll
       for (int kt = 0; kt < 4; kt++) {
         uint32_t bf[4];
         ldsm_b2(W2, kW2s, 16 * q, kt * 16, bf);
-        mma_bf16(h[0], a2[kt], bf[0], bf[1]);
-        mma_bf16(h[1], a2[kt], bf[2], bf[3]);
+#pragma unroll
+        for (int t = 0; t < kMT; t++) {
+          if (kt == 0) {
+            mma_bf16_c(h[t][0], a2[t][kt], bf[0], bf[1], ca);
+            mma_bf16_c(h[t][1], a2[t][kt], bf[2], bf[3], cb);
+          } else {
+            mma_bf16(h[t][0], a2[t][kt], bf[0], bf[1]);
+            mma_bf16(h[t][1], a2[t][kt], bf[2], bf[3]);
+          }
+        }
       }
-      uint32_t a3[4];
-      a3[0] = gelu_bf16x2(h[0][0], h[0][1]);
-      a3[1] = gelu_bf16x2(h[0][2], h[0][3]);
-      a3[2] = gelu_bf16x2(h[1][0], h[1][1]);
-      a3[3] = gelu_bf16x2(h[1][2], h[1][3]);
       const uint8_t *wr = W3 + (g * kW3s + q * 16 + 2 * tg) * 2;
-      mma_bf16(y, a3, lds32(wr), lds32(wr + 16));
+      const uint32_t w0 = lds32(wr), w1 = lds32(wr + 16);
+#pragma unroll
+      for (int t = 0; t < kMT; t++) {
+        uint32_t a3[4];
+        a3[0] = gelu_bf16x2(h[t][0][0], h[t][0][1]);
+        a3[1] = gelu_bf16x2(h[t][0][2], h[t][0][3]);
+        a3[2] = gelu_bf16x2(h[t][1][0], h[t][1][1]);
+        a3[3] = gelu_bf16x2(h[t][1][2], h[t][1][3]);
+        mma_bf16(y[t], a3, w0, w1);
+      }
     }
     if (tg < 2) {
       const int c0 = 2 * tg;
-      float *Y0 = Y + (16 * mt + g) * 4, *Y1 = Y + (16 * mt + g + 8) * 4;
-      Y0[c0] = y[0] + b3[c0];
-      Y0[c0 + 1] = y[1] + b3[c0 + 1];
-      Y1[c0] = y[2] + b3[c0];
-      Y1[c0 + 1] = y[3] + b3[c0 + 1];
+      const float d0 = b3[c0], d1 = b3[c0 + 1];
+#pragma unroll
+      for (int t = 0; t < kMT; t++) {
+        float *Y0 = Y + (16 * (mt + t) + g) * 4 + c0;
+        *reinterpret_cast<float2 *>(Y0) = make_float2(y[t][0] + d0, y[t][1] + d1);
+        *reinterpret_cast<float2 *>(Y0 + 32) = make_float2(y[t][2] + d0, y[t][3] + d1);
+      }
     }
   }
+}
+
+// Rows of the two sites of a lane in its warp's 64-row tiles: A rows first,
+// then B rows, so that the lanes' row stores fall on distinct banks.
+__device__ __forceinline__ int site_row(int lane, int b) { return lane + 32 * b; }
+
+// Zeros the columns that feature rows never write (kXw words on).
+constexpr int kXw = 10;  // words of a feature row: 19 inputs and a zero
+__device__ __forceinline__ void clear_row_tails(__nv_bfloat16 *X, int lane) {
+#pragma unroll
+  for (int b = 0; b < 2; b++) {
+    uint32_t *d = reinterpret_cast<uint32_t *>(X + (size_t)site_row(lane, b) * kXs);
+    *reinterpret_cast<uint2 *>(d + kXw) = make_uint2(0u, 0u);
+    *reinterpret_cast<uint4 *>(d + 12) = make_uint4(0u, 0u, 0u, 0u);
+  }
+}
+
+__device__ __forceinline__ void store_row(__nv_bfloat16 *X, int row, const uint32_t *r) {
+  uint32_t *d = reinterpret_cast<uint32_t *>(X + (size_t)row * kXs);
+  *reinterpret_cast<uint4 *>(d) = make_uint4(r[0], r[1], r[2], r[3]);
+  *reinterpret_cast<uint4 *>(d + 4) = make_uint4(r[4], r[5], r[6], r[7]);
+  *reinterpret_cast<uint2 *>(d + 8) = make_uint2(r[8], r[9]);
 }
 
 // log cosh, stable: |x| + log(1 + exp(-2|x|)) (the -log 2 cancels in ratios).

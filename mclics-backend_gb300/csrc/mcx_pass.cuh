@@ -678,13 +678,11 @@ __device__ __forceinline__ void feature_words(const float nb[6][3], const float 
   for (int q = 10; q < 16; q++) r[q] = 0u;
 }
 
-__device__ __forceinline__ void write_features(__nv_bfloat16 *row, const float nb[6][3], const float w[6], float T,
+__device__ __forceinline__ void write_features(__nv_bfloat16 *X, int row, const float nb[6][3], const float w[6], float T,
                                                bool live) {
   uint32_t r[16];
   feature_words(nb, w, T, live, r);
-  uint32_t *d = reinterpret_cast<uint32_t *>(row);
-#pragma unroll
-  for (int q = 0; q < 16; q++) d[q] = r[q];
+  store_row(X, row, r);  // words 10..15 are zeros that clear_row_tails wrote
 }
 
 template <int POT, bool MASK, bool FIELD, int MODE>
@@ -740,18 +738,15 @@ __device__ __forceinline__ void compute_pair_learned(const PassArgs &a, int c, i
   const int psA = MASK ? pself2.x : 1, psB = MASK ? pself2.y : 1;
   const float T = g.valid ? S->T : 0.f;
   __syncwarp();
-  write_features(X + (size_t)(2 * lane) * kXs, nbA, wA, T, g.valid);
-  write_features(X + (size_t)(2 * lane + 1) * kXs, nbB, wB, T, g.valid && g.hasB);
+  write_features(X, site_row(lane, 0), nbA, wA, T, g.valid);
+  write_features(X, site_row(lane, 1), nbB, wB, T, g.valid && g.hasB);
   __syncwarp();
   mlp_warp(W, X, Y);
   __syncwarp();
   if (!g.valid) return;
-  float yA[4], yB[4];
-#pragma unroll
-  for (int q = 0; q < 4; q++) {
-    yA[q] = Y[(2 * lane) * 4 + q];
-    yB[q] = Y[(2 * lane + 1) * 4 + q];
-  }
+  const float4 y0 = reinterpret_cast<const float4 *>(Y)[site_row(lane, 0)];
+  const float4 y1 = reinterpret_cast<const float4 *>(Y)[site_row(lane, 1)];
+  const float yA[4] = {y0.x, y0.y, y0.z, y0.w}, yB[4] = {y1.x, y1.y, y1.z, y1.w};
   float2 ax = st.v[0][tid], ay = st.v[1][tid], az = st.v[2][tid];
   const unsigned long long sw = UPD ? S->sweep : 0ull;
   const float invT = UPD ? 1.0f / S->T : 0.f;
@@ -809,6 +804,7 @@ __global__ void __launch_bounds__(kPB, LEARN ? MCX_LEARN_MIN_BLOCKS : MCX_PASS_M
   if (LEARN) {
     for (int i = threadIdx.x; i < kMlpBytes / 16; i += kPB)
       reinterpret_cast<int4 *>(mlpW)[i] = reinterpret_cast<const int4 *>(a.mlp)[i];
+    clear_row_tails(mlpX, threadIdx.x & 31);
     __syncthreads();
   }
   const int G = gridDim.x, n = a.nmap;

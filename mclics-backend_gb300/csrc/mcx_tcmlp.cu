@@ -77,28 +77,25 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_warp(const uint8_t *mlp, con
   float *Y = reinterpret_cast<float *>(sm + kMlpBytes + (kTcThreads / 32) * 64 * kXs * 2) + (size_t)warp * 64 * 4;
   for (int i = threadIdx.x; i < kMlpBytes / 16; i += kTcThreads)
     reinterpret_cast<int4 *>(W)[i] = reinterpret_cast<const int4 *>(mlp)[i];
+  clear_row_tails(X, lane);
   __syncthreads();
   const int warps = gridDim.x * (kTcThreads / 32);
 #pragma unroll 1
   for (int base = (blockIdx.x * (kTcThreads / 32) + warp) * 64; base < n; base += warps * 64) {
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int row = base + 2 * lane + h;
+      const int row = base + site_row(lane, h);
       uint32_t w[16];
       pack_inputs(in + (size_t)row * 19, row < n, w);
-      uint32_t *r = reinterpret_cast<uint32_t *>(X + (size_t)(2 * lane + h) * kXs);
-#pragma unroll
-      for (int q = 0; q < 16; q++) r[q] = w[q];
+      store_row(X, site_row(lane, h), w);
     }
     __syncwarp();
     mlp_warp(W, X, Y);
     __syncwarp();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
-      const int row = base + 2 * lane + h;
-      if (row < n)
-#pragma unroll
-        for (int q = 0; q < 4; q++) out[(size_t)row * 4 + q] = Y[(2 * lane + h) * 4 + q];
+      const int row = base + site_row(lane, h);
+      if (row < n) reinterpret_cast<float4 *>(out)[row] = reinterpret_cast<const float4 *>(Y)[site_row(lane, h)];
     }
     __syncwarp();
   }
