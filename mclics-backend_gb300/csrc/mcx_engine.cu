@@ -103,12 +103,15 @@ struct mcx_engine {
   long long dir_total = 0;  // floats of d_dir
   // training of the network: FP32 master weights, Adam moments, gradient
   float *d_w = nullptr, *d_am = nullptr, *d_av = nullptr, *d_g = nullptr, *d_loss = nullptr;
+  uint8_t *d_image = nullptr;  // BF16 image of d_w for the gradient kernel
+  float *d_part = nullptr;     // its CTAs' partial gradients
+  long long part_bytes = 0;
   bool w_stale = true;  // d_w does not hold e->mlp yet (Adam restarts)
   int adam_step = 0;
   float *d_samples = nullptr;
   long long sample_cap = 0;
-  int *d_idx = nullptr, *d_repof = nullptr;
-  long long idx_cap = 0, repof_cap = 0, loss_bytes = 0;
+  int *d_repof = nullptr;
+  long long repof_cap = 0, loss_bytes = 0;
   int held_samples = 0;  // samples in d_samples (last collection or mcx_mlp_grad upload)
 };
 
@@ -231,8 +234,9 @@ static void free_engine(mcx_engine *e) {
   cudaFree(e->d_av);
   cudaFree(e->d_g);
   cudaFree(e->d_loss);
+  cudaFree(e->d_image);
+  cudaFree(e->d_part);
   cudaFree(e->d_samples);
-  cudaFree(e->d_idx);
   cudaFree(e->d_repof);
   if (e->stream) cudaStreamDestroy(e->stream);
   delete e;
@@ -1665,11 +1669,16 @@ static mcx_status train_prepare(mcx_engine *e) {
       cudaError_t r = cudaMalloc(b, wb);
       if (r != cudaSuccess) return fail(e, MCX_ERR_NOMEM, "training buffers: %s", cudaGetErrorString(r));
     }
+    cudaError_t r = cudaMalloc(&e->d_image, train_image_bytes());
+    if (r != cudaSuccess) return fail(e, MCX_ERR_NOMEM, "training buffers: %s", cudaGetErrorString(r));
+    CK(e, cudaMemsetAsync(e->d_image, 0, train_image_bytes(), e->stream));  // its padding stays zero
   }
   if (e->w_stale) {
     CK(e, cudaMemcpyAsync(e->d_w, e->mlp.data(), wb, cudaMemcpyHostToDevice, e->stream));
     CK(e, cudaMemsetAsync(e->d_am, 0, wb, e->stream));
     CK(e, cudaMemsetAsync(e->d_av, 0, wb, e->stream));
+    CK(e, launch_adam(nullptr, 0, e->d_w, e->d_am, e->d_av, e->d_image, nullptr, nullptr, 0, 0.f, false, e->stream));
+    e->launches++;
     CK(e, cudaStreamSynchronize(e->stream));
     e->adam_step = 0;
     e->w_stale = false;
@@ -1734,10 +1743,11 @@ extern "C" mcx_status mcx_mlp_grad(mcx_engine *e, const float *samples, int n, f
   CK(e, ensure_bytes((void **)&e->d_loss, &e->loss_bytes, sizeof(float)));
   CK(e, cudaMemcpyAsync(e->d_samples, samples, sb, cudaMemcpyHostToDevice, e->stream));
   e->held_samples = n;
-  CK(e, cudaMemsetAsync(e->d_g, 0, sizeof(float) * MCX_MLP_PARAMS, e->stream));
-  CK(e, cudaMemsetAsync(e->d_loss, 0, sizeof(float), e->stream));
-  CK(e, launch_mlp_grad(e->d_w, e->d_samples, nullptr, n, e->d_g, e->d_loss, grad_grid(n), e->stream));
-  e->launches++;
+  const int grid = grad_grid(n);
+  CK(e, ensure_bytes((void **)&e->d_part, &e->part_bytes, (long long)grid * train_part_floats() * sizeof(float)));
+  CK(e, launch_mlp_grad(e->d_image, e->d_samples, n, 0, 0u, 0u, e->d_part, grid, false, e->stream));
+  CK(e, launch_adam(e->d_part, grid, e->d_w, e->d_am, e->d_av, e->d_image, e->d_g, e->d_loss, 0, 0.f, false, e->stream));
+  e->launches += 2;
   CK(e, cudaMemcpyAsync(grad, e->d_g, sizeof(float) * MCX_MLP_PARAMS, cudaMemcpyDeviceToHost, e->stream));
   float l = 0.f;
   CK(e, cudaMemcpyAsync(&l, e->d_loss, sizeof(float), cudaMemcpyDeviceToHost, e->stream));
@@ -1800,17 +1810,18 @@ extern "C" mcx_status mcx_train_mlp(mcx_engine *e, const mcx_train_config *cfg, 
   if (cfg->samples > 0)
     if (mcx_status st = collect(e, cfg->samples, cfg->seed, cfg->augment)) return st;
   const int nsamp = e->held_samples;
-  CK(e, ensure_bytes((void **)&e->d_idx, &e->idx_cap, (long long)cfg->batch * sizeof(int)));
   CK(e, ensure_bytes((void **)&e->d_loss, &e->loss_bytes, (long long)std::max(1, cfg->steps) * sizeof(float)));
-  CK(e, cudaMemsetAsync(e->d_loss, 0, sizeof(float) * std::max(1, cfg->steps), e->stream));
   const int grid = grad_grid(cfg->batch);
+  CK(e, ensure_bytes((void **)&e->d_part, &e->part_bytes, (long long)grid * train_part_floats() * sizeof(float)));
   for (int s = 0; s < cfg->steps; s++) {
     e->adam_step++;
-    CK(e, launch_batch_index(e->d_idx, cfg->batch, nsamp, cfg->seed, (uint32_t)e->adam_step, e->stream));
-    CK(e, cudaMemsetAsync(e->d_g, 0, sizeof(float) * MCX_MLP_PARAMS, e->stream));
-    CK(e, launch_mlp_grad(e->d_w, e->d_samples, e->d_idx, cfg->batch, e->d_g, e->d_loss + s, grid, e->stream));
-    CK(e, launch_adam(e->d_w, e->d_am, e->d_av, e->d_g, e->adam_step, cfg->lr, e->stream));
-    e->launches += 3;
+    // each launch sets up (and, for the gradient, loads its samples) while the
+    // one before drains
+    CK(e, launch_mlp_grad(e->d_image, e->d_samples, cfg->batch, nsamp, cfg->seed, (uint32_t)e->adam_step, e->d_part,
+                          grid, e->pdl, e->stream));
+    CK(e, launch_adam(e->d_part, grid, e->d_w, e->d_am, e->d_av, e->d_image, nullptr, e->d_loss + s, e->adam_step,
+                      cfg->lr, e->pdl, e->stream));
+    e->launches += 2;
   }
   std::vector<float> w(MCX_MLP_PARAMS);
   CK(e, cudaMemcpyAsync(w.data(), e->d_w, sizeof(float) * MCX_MLP_PARAMS, cudaMemcpyDeviceToHost, e->stream));

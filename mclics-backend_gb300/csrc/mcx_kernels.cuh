@@ -199,9 +199,15 @@ int train_smem_bytes();
 int sample_floats();
 cudaError_t launch_collect(const RepDev *reps, const RepState *st, const float *dir, const uint8_t *pt, float *out,
                            const int *rep_of, int n, uint32_t seed, int augment, cudaStream_t s);
-cudaError_t launch_mlp_grad(const float *w, const float *samples, const int *index, int n, float *grad, float *loss,
-                            int grid, cudaStream_t s);
-cudaError_t launch_adam(float *w, float *m, float *v, const float *g, int step, float lr, cudaStream_t s);
-cudaError_t launch_batch_index(int *idx, int n, int nsamples, uint32_t seed, uint32_t step, cudaStream_t s);
+int train_image_bytes();
+int train_part_floats();
+// Partial loss and gradient of n samples (draw_from > 0: drawn from that many
+// by seed and step) at the weights of image, one row of train_part_floats()
+// floats per CTA; launch_adam sums the rows into grad / loss (either may be
+// null), with step > 0 updates the weights by Adam, and writes their image.
+cudaError_t launch_mlp_grad(const uint8_t *image, const float *samples, int n, int draw_from, uint32_t seed,
+                            uint32_t step, float *part, int grid, bool pdl, cudaStream_t s);
+cudaError_t launch_adam(const float *part, int rows, float *w, float *m, float *v, uint8_t *image, float *grad,
+                        float *loss, int step, float lr, bool pdl, cudaStream_t s);
 
 }  // namespace mcx

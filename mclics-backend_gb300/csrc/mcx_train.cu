@@ -15,8 +15,18 @@
 //               CTA contracts activations with output gradients over the 64
 //               samples -- again on the tensor cores, operands transposed by
 //               ldmatrix.trans -- into FP32 weight gradients held in
-//               registers; one FP32 atomic per weight and CTA at the end.
-//   k_adam      Adam on the FP32 master weights (padding entries stay zero).
+//               registers, which the CTA writes to its row of a partial-sum
+//               buffer.  The batch's sample indices are drawn in the kernel.
+//   k_adam      sums the partial gradients in a fixed order, runs Adam on the
+//               FP32 master weights (padding entries stay zero) and writes the
+//               BF16 image of the weights that k_mlp_grad's CTAs copy to shared
+//               memory; without the update it is the sum for mcx_mlp_grad.
+//
+// What bounds a training step is latency, not work (8192 samples are 128 chunks
+// of 64, one per CTA): weights converted by every CTA from strided FP32 reads,
+// 870,000 atomics on 6,792 addresses, and five launches took 31 us a step.  Two
+// launches, a copied image and partial sums that are read once take 11; the
+// results no longer depend on the order of atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <math.h>
@@ -27,6 +37,7 @@
 #include "../../include/mcx.h"
 #include "mcx_device.cuh"
 #include "mcx_kernels.cuh"
+#include "mcx_march.cuh"
 #include "mcx_mlp.cuh"
 
 namespace mcx {
@@ -153,14 +164,21 @@ __global__ void k_collect(CollectArgs a) {
 // Loss and gradient.
 // ---------------------------------------------------------------------------
 struct GradArgs {
-  const float *w;        // FP32 master weights (flat)
+  const uint8_t *image;  // BF16 weights and FP32 biases (kG* layout)
   const float *samples;  // [n][kSampleF]
-  const int *index;      // sample indices of this batch (null: 0..n-1)
   int n;                 // samples in the batch
   float inv_n;           // 1/n: the loss is a mean
-  float *grad;           // FP32 [kPTotal], accumulated
-  float *loss;           // accumulated mean loss
+  int draw_from;         // > 0: the batch is drawn with replacement from this many samples
+  uint32_t seed, step;   // the draw's key and counter
+  float *part;           // [grid][kPartF] partial gradients, the loss at kPTotal
 };
+constexpr int kPartF = (kPTotal + 1 + 31) / 32 * 32;  // floats per partial row
+
+// Batch sample i of a step (with replacement).
+__device__ __forceinline__ int batch_index(int i, int nsamples, uint32_t seed, uint32_t step) {
+  const uint4 r = philox4x32_10(make_uint4((uint32_t)i, step, 0xBA7Cu, 0xC011u), seed, 0x7EA1u);
+  return (int)(((unsigned long long)r.x * (unsigned long long)nsamples) >> 32);
+}
 
 __device__ __forceinline__ void ldsm_x4_t(uint32_t r[4], const void *p) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -190,7 +208,9 @@ constexpr int kGW3t = kGW2t + kMlpH * kW2s * 2;    // [8][72]  bf16 (forward)
 constexpr int kGW2r = kGW3t + kMlpOut * kW3s * 2;  // [64][72] bf16 row = input (backward)
 constexpr int kGW3r = kGW2r + kMlpH * kRowH * 2;   // [64][24] bf16 row = hidden, cols = out (backward)
 constexpr int kGB = kGW3r + kMlpH * kRowY * 2;     // b1[64] b2[64] b3[8] floats
-constexpr int kGX = kGB + (2 * kMlpH + kMlpOut) * 4;  // chunk tiles
+constexpr int kGImage = kGB + (2 * kMlpH + kMlpOut) * 4;  // bytes of the weight image
+static_assert(kGImage % 16 == 0, "the image is copied in 16-byte words");
+constexpr int kGX = kGImage;                       // chunk tiles
 constexpr int kGA1 = kGX + kTS * kXs * 2;
 constexpr int kGA2 = kGA1 + kTS * kRowH * 2;
 constexpr int kGdH1 = kGA2 + kTS * kRowH * 2;
@@ -215,55 +235,64 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
   __nv_bfloat16 *dH2 = reinterpret_cast<__nv_bfloat16 *>(sm + kGdH2);
   __nv_bfloat16 *dY = reinterpret_cast<__nv_bfloat16 *>(sm + kGdY);
   float *Ys = reinterpret_cast<float *>(sm + kGY);
-  // weights: FP32 master -> BF16 in the forward (transposed) and backward layouts
-  for (int e = tid; e < kMlpH * kW1s; e += kTW * 32) {
-    const int n = e / kW1s, k = e % kW1s;
-    W1t[e] = __float2bfloat16_rn(k < kMlpIn ? a.w[kPW1 + k * kMlpH + n] : 0.f);
-  }
-  for (int e = tid; e < kMlpH * kW2s; e += kTW * 32) {
-    const int n = e / kW2s, k = e % kW2s;
-    W2t[e] = __float2bfloat16_rn(k < kMlpH ? a.w[kPW2 + k * kMlpH + n] : 0.f);
-    W2r[e] = __float2bfloat16_rn(k < kMlpH ? a.w[kPW2 + n * kMlpH + k] : 0.f);  // row n = input, col k = output
-  }
-  for (int e = tid; e < kMlpOut * kW3s; e += kTW * 32) {
-    const int n = e / kW3s, k = e % kW3s;
-    W3t[e] = __float2bfloat16_rn(k < kMlpH ? a.w[kPW3 + k * kMlpOut + n] : 0.f);
-  }
-  for (int e = tid; e < kMlpH * kRowY; e += kTW * 32) {
-    const int i = e / kRowY, o = e % kRowY;
-    W3r[e] = __float2bfloat16_rn(o < kMlpOut ? a.w[kPW3 + i * kMlpOut + o] : 0.f);
-  }
-  for (int e = tid; e < 2 * kMlpH + kMlpOut; e += kTW * 32)
-    bias[e] = e < kMlpH ? a.w[kPB1 + e] : (e < 2 * kMlpH ? a.w[kPB2 + e - kMlpH] : a.w[kPB3 + e - 2 * kMlpH]);
-  __syncthreads();
   // weight-gradient accumulators (FP32, fragment layout)
   float gW2[8][4], gWx[8][4];  // gWx: gW1 slice (warps 0,1) or gW3 slices (warps 2,3: [2][4] used)
 #pragma unroll
   for (int q = 0; q < 8; q++)
 #pragma unroll
     for (int r = 0; r < 4; r++) gW2[q][r] = gWx[q][r] = 0.f;
-  float gb = 0.f;  // bias gradient owned by this thread: b1 (tid < 64), b2 (64 <= tid < 128)
-  float gb3 = 0.f; // b3 entries (tid < 8)
+  // bias gradients are column sums over the samples: b1 is the gradient of an
+  // input that is always 1 (X column 31, a padding row of W1), b2 and b3 are
+  // products with a tile of ones in accumulators that warps 2 and 3 leave free
+  // (gWx[2..5] b2, gWx[6] b3)
+  bool loaded = false;
+  const uint32_t ones[4] = {0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u};
   float lsum = 0.f;
   const int nchunk = (a.n + kTS - 1) / kTS;
   for (int ch = blockIdx.x; ch < nchunk; ch += gridDim.x) {
     const int row0 = warp * 16;  // this warp's rows in the chunk tiles
     // ---- inputs: lane l fills half a row ----
+    float tx = 0.f, ty = 0.f, tz = 0.f;  // the target of sample l (lanes 0..15)
     {
       const int r = lane >> 1, half = lane & 1;
       const int sidx = ch * kTS + row0 + r;
-      float v[16];
+      float4 v[4];
+#pragma unroll
+      for (int q = 0; q < 4; q++) v[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+      float4 t = v[0];
       if (sidx < a.n) {
-        const float *sp = a.samples + (size_t)(a.index ? a.index[sidx] : sidx) * kSampleF;
-        for (int q = 0; q < 16; q++) {
-          const int col = half * 16 + q;
-          v[q] = col < 19 ? sp[col] : 0.f;
+        const int at = a.draw_from > 0 ? batch_index(sidx, a.draw_from, a.seed, a.step) : sidx;
+        const float4 *sp = reinterpret_cast<const float4 *>(a.samples + (size_t)at * kSampleF) + half * 4;
+        v[0] = sp[0];
+        if (half) {
+          t = make_float4(v[0].w, 0.f, 0.f, 0.f);  // floats 19, 20, 21: the target
+          const float2 u = *reinterpret_cast<const float2 *>(sp + 1);
+          t.y = u.x;
+          t.z = u.y;
+          v[0].w = 0.f;
+          v[3].w = 1.f;  // column 31
+        } else {
+#pragma unroll
+          for (int q = 1; q < 4; q++) v[q] = sp[q];
         }
-      } else {
-        for (int q = 0; q < 16; q++) v[q] = 0.f;
       }
-      uint32_t *xr = reinterpret_cast<uint32_t *>(X + (size_t)(row0 + r) * kXs + half * 16);
-      for (int q = 0; q < 8; q++) xr[q] = pack_bf16(v[2 * q], v[2 * q + 1]);
+      uint4 *xr = reinterpret_cast<uint4 *>(X + (size_t)(row0 + r) * kXs + half * 16);
+#pragma unroll
+      for (int q = 0; q < 2; q++)
+        xr[q] = make_uint4(pack_bf16(v[2 * q].x, v[2 * q].y), pack_bf16(v[2 * q].z, v[2 * q].w),
+                           pack_bf16(v[2 * q + 1].x, v[2 * q + 1].y), pack_bf16(v[2 * q + 1].z, v[2 * q + 1].w));
+      const int from = (2 * lane + 1) & 31;
+      tx = __shfl_sync(0xffffffffu, t.x, from);
+      ty = __shfl_sync(0xffffffffu, t.y, from);
+      tz = __shfl_sync(0xffffffffu, t.z, from);
+    }
+    if (!loaded) {
+      // the samples do not depend on the step before; the weights do
+      grid_dependency_wait();
+      for (int e = tid; e < kGImage / 16; e += kTW * 32)
+        reinterpret_cast<uint4 *>(sm)[e] = __ldcg(reinterpret_cast<const uint4 *>(a.image) + e);
+      loaded = true;
+      __syncthreads();
     }
     __syncwarp();
     const __nv_bfloat16 *Xr = X + (size_t)row0 * kXs;
@@ -343,8 +372,7 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
       const int sidx = ch * kTS + row0 + lane;
       float d[4] = {0.f, 0.f, 0.f, 0.f};
       if (sidx < a.n) {
-        const float *sp = a.samples + (size_t)(a.index ? a.index[sidx] : sidx) * kSampleF;
-        const float nx = sp[19], ny = sp[20], nz = sp[21];
+        const float nx = tx, ny = ty, nz = tz;
         const float *yy = Ys + (row0 + lane) * 4;
         const float nm = sqrtf(yy[0] * yy[0] + yy[1] * yy[1] + yy[2] * yy[2]);
         const float inm = nm > 1e-12f ? 1.f / nm : 0.f;
@@ -439,6 +467,7 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
           uint32_t bf[2];
           ldsm_x2_t(bf, dH2 + (size_t)(s0 + (lane & 15)) * kRowH + nt * 8);
           mma_bf16(gW2[nt], af, bf[0], bf[1]);
+          if (warp >= 2 && (nt >> 2) == warp - 2) mma_bf16(gWx[2 + (nt & 3)], ones, bf[0], bf[1]);
         }
       }
       if (warp < 2) {  // gW1 rows [16 warp, +16) (input features)
@@ -453,6 +482,7 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
       } else {  // gW3 rows [32 (warp-2), +32): two 16-row tiles, one 8-wide output tile
         uint32_t bf[2];
         ldsm_x2_t(bf, dY + (size_t)(s0 + (lane & 15)) * kRowY);
+        mma_bf16(gWx[6], ones, bf[0], bf[1]);
 #pragma unroll
         for (int mt = 0; mt < 2; mt++) {
           uint32_t af[4];
@@ -461,78 +491,123 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
         }
       }
     }
-    // bias gradients: column sums of dH1 (tid < 64), dH2 (64..127), dY (tid < 8)
-    if (tid < 64) {
-      for (int s2 = 0; s2 < kTS; s2++) gb += __bfloat162float(dH1[(size_t)s2 * kRowH + tid]);
-    } else {
-      for (int s2 = 0; s2 < kTS; s2++) gb += __bfloat162float(dH2[(size_t)s2 * kRowH + tid - 64]);
-    }
-    if (tid < kMlpOut)
-      for (int s2 = 0; s2 < kTS; s2++) gb3 += __bfloat162float(dY[(size_t)s2 * kRowY + tid]);
     __syncthreads();
   }
-  // ---- one atomic per weight and CTA ----
+  // ---- the CTA's partial sums, in the flat parameter layout ----
+  grid_launch_dependents();
+  float *part = a.part + (size_t)blockIdx.x * kPartF;
+  auto put = [&](int at, float x, float y) { *reinterpret_cast<float2 *>(part + at) = make_float2(x, y); };
 #pragma unroll
   for (int nt = 0; nt < 8; nt++) {
-    const int o0 = nt * 8 + 2 * tg;
-    const int i0 = warp * 16 + g;
-    atomicAdd(a.grad + kPW2 + i0 * kMlpH + o0, gW2[nt][0]);
-    atomicAdd(a.grad + kPW2 + i0 * kMlpH + o0 + 1, gW2[nt][1]);
-    atomicAdd(a.grad + kPW2 + (i0 + 8) * kMlpH + o0, gW2[nt][2]);
-    atomicAdd(a.grad + kPW2 + (i0 + 8) * kMlpH + o0 + 1, gW2[nt][3]);
+    const int o0 = nt * 8 + 2 * tg, i0 = warp * 16 + g;
+    put(kPW2 + i0 * kMlpH + o0, gW2[nt][0], gW2[nt][1]);
+    put(kPW2 + (i0 + 8) * kMlpH + o0, gW2[nt][2], gW2[nt][3]);
     if (warp < 2) {
-      atomicAdd(a.grad + kPW1 + i0 * kMlpH + o0, gWx[nt][0]);
-      atomicAdd(a.grad + kPW1 + i0 * kMlpH + o0 + 1, gWx[nt][1]);
-      atomicAdd(a.grad + kPW1 + (i0 + 8) * kMlpH + o0, gWx[nt][2]);
-      atomicAdd(a.grad + kPW1 + (i0 + 8) * kMlpH + o0 + 1, gWx[nt][3]);
+      const bool one = i0 + 8 == kMlpIn - 1;  // the column of ones
+      put(kPW1 + i0 * kMlpH + o0, gWx[nt][0], gWx[nt][1]);
+      put(kPW1 + (i0 + 8) * kMlpH + o0, one ? 0.f : gWx[nt][2], one ? 0.f : gWx[nt][3]);
+      if (one) put(kPB1 + o0, gWx[nt][2], gWx[nt][3]);
     }
   }
   if (warp >= 2) {
 #pragma unroll
     for (int mt = 0; mt < 2; mt++) {
-      const int i0 = (warp - 2) * 32 + mt * 16 + g;
-      const int o0 = 2 * tg;
-      atomicAdd(a.grad + kPW3 + i0 * kMlpOut + o0, gWx[mt][0]);
-      atomicAdd(a.grad + kPW3 + i0 * kMlpOut + o0 + 1, gWx[mt][1]);
-      atomicAdd(a.grad + kPW3 + (i0 + 8) * kMlpOut + o0, gWx[mt][2]);
-      atomicAdd(a.grad + kPW3 + (i0 + 8) * kMlpOut + o0 + 1, gWx[mt][3]);
+      const int i0 = (warp - 2) * 32 + mt * 16 + g, o0 = 2 * tg;
+      put(kPW3 + i0 * kMlpOut + o0, gWx[mt][0], gWx[mt][1]);
+      put(kPW3 + (i0 + 8) * kMlpOut + o0, gWx[mt][2], gWx[mt][3]);
+    }
+    if (g == 0) {
+#pragma unroll
+      for (int q = 0; q < 4; q++) put(kPB2 + ((warp - 2) * 4 + q) * 8 + 2 * tg, gWx[2 + q][0], gWx[2 + q][1]);
+      if (warp == 2) put(kPB3 + 2 * tg, gWx[6][0], gWx[6][1]);
     }
   }
-  atomicAdd(a.grad + (tid < 64 ? kPB1 + tid : kPB2 + tid - 64), gb);
-  if (tid < kMlpOut) atomicAdd(a.grad + kPB3 + tid, gb3);
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-  if (lane == 0) atomicAdd(a.loss, lsum);
+  __shared__ float s_loss[kTW];
+  if (lane == 0) s_loss[warp] = lsum;
+  __syncthreads();
+  if (tid == 0) part[kPTotal] = (s_loss[0] + s_loss[1]) + (s_loss[2] + s_loss[3]);
 }
 
-// Adam (Kingma & Ba 2015) on the FP32 master weights; the layout's padding
+struct AdamArgs {
+  const float *part;  // [rows][kPartF] partial gradients and losses
+  int rows;
+  float *w, *m, *v;   // FP32 master weights and moments
+  uint8_t *image;     // the BF16 image (kG* layout) of the updated weights
+  float *grad;        // the summed gradient (null: not wanted)
+  float *loss;        // the summed loss
+  int step;           // 0: no update (the image, and the sums if rows > 0)
+  float lr, b1, b2, eps;
+};
+
+// The BF16 image entries of weight i (forward, transposed; and backward).
+__device__ __forceinline__ void put_image(uint8_t *im, int i, float w) {
+  const __nv_bfloat16 b = __float2bfloat16_rn(w);
+  __nv_bfloat16 *W1t = reinterpret_cast<__nv_bfloat16 *>(im + kGW1t), *W2t = reinterpret_cast<__nv_bfloat16 *>(im + kGW2t),
+                *W3t = reinterpret_cast<__nv_bfloat16 *>(im + kGW3t), *W2r = reinterpret_cast<__nv_bfloat16 *>(im + kGW2r),
+                *W3r = reinterpret_cast<__nv_bfloat16 *>(im + kGW3r);
+  float *bias = reinterpret_cast<float *>(im + kGB);
+  if (i < kPB1) {
+    const int k = i / kMlpH, n = i % kMlpH;
+    W1t[n * kW1s + k] = k < 19 ? b : __float2bfloat16_rn(0.f);  // inputs 19..30 are zeros, 31 the ones of b1's gradient
+  } else if (i < kPW2) {
+    bias[i - kPB1] = w;
+  } else if (i < kPB2) {
+    const int k = (i - kPW2) / kMlpH, n = (i - kPW2) % kMlpH;
+    W2t[n * kW2s + k] = b;
+    W2r[k * kRowH + n] = b;
+  } else if (i < kPW3) {
+    bias[kMlpH + i - kPB2] = w;
+  } else if (i < kPB3) {
+    const int k = (i - kPW3) / kMlpOut, o = (i - kPW3) % kMlpOut;
+    W3t[o * kW3s + k] = b;
+    W3r[k * kRowY + o] = b;
+  } else {
+    bias[2 * kMlpH + i - kPB3] = w;
+  }
+}
+
+// A CTA sums 32 parameters: warp w the partial rows w, w + 8, ..., then warp 0
+// the eight sums in order.  Adam (Kingma & Ba 2015); the layout's padding
 // (input rows 19..31 of W1, output columns 4..7 of W3 and b3) stays zero.
-__global__ void k_adam(float *w, float *m, float *v, const float *g, int step, float lr, float b1, float b2,
-                       float eps) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+constexpr int kAdamWarps = 8;
+__global__ void __launch_bounds__(kAdamWarps * 32) k_adam(AdamArgs a) {
+  __shared__ float s_sum[kAdamWarps][32];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
+  grid_dependency_wait();
+  float sum = 0.f;
+#pragma unroll 16
+  for (int r = warp; r < a.rows; r += kAdamWarps) sum += __ldcg(a.part + (size_t)r * kPartF + i);
+  s_sum[warp][lane] = sum;
+  __syncthreads();
+  grid_launch_dependents();
+  if (warp != 0) return;
+  float gi = 0.f;
+#pragma unroll
+  for (int w = 0; w < kAdamWarps; w += 2) gi += s_sum[w][lane] + s_sum[w + 1][lane];
+  if (i == kPTotal && a.loss) *a.loss = gi;
   if (i >= kPTotal) return;
+  if (a.grad) a.grad[i] = gi;
   bool pad = false;
   if (i < kPB1) pad = (i - kPW1) / kMlpH >= 19;
   else if (i >= kPW3 && i < kPB3) pad = (i - kPW3) % kMlpOut >= 4;
   else if (i >= kPB3) pad = i - kPB3 >= 4;
-  if (pad) {
-    w[i] = 0.f;
-    return;
+  float wi = a.w[i];
+  if (a.step > 0) {
+    if (pad) {
+      wi = 0.f;
+    } else {
+      const float mi = a.b1 * a.m[i] + (1.f - a.b1) * gi;
+      const float vi = a.b2 * a.v[i] + (1.f - a.b2) * gi * gi;
+      a.m[i] = mi;
+      a.v[i] = vi;
+      const float mh = mi / (1.f - powf(a.b1, (float)a.step));
+      const float vh = vi / (1.f - powf(a.b2, (float)a.step));
+      wi -= a.lr * mh / (sqrtf(vh) + a.eps);
+    }
+    a.w[i] = wi;
   }
-  const float gi = g[i];
-  const float mi = b1 * m[i] + (1.f - b1) * gi;
-  const float vi = b2 * v[i] + (1.f - b2) * gi * gi;
-  m[i] = mi;
-  v[i] = vi;
-  const float mh = mi / (1.f - powf(b1, (float)step));
-  const float vh = vi / (1.f - powf(b2, (float)step));
-  w[i] -= lr * mh / (sqrtf(vh) + eps);
-}
-
-__global__ void k_batch_index(int *idx, int n, int nsamples, uint32_t seed, uint32_t step) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
-  const uint4 r = philox4x32_10(make_uint4((uint32_t)i, step, 0xBA7Cu, 0xC011u), seed, 0x7EA1u);
-  idx[i] = (int)(((unsigned long long)r.x * (unsigned long long)nsamples) >> 32);
+  put_image(a.image, i, wi);
 }
 
 }  // namespace mcx
@@ -552,27 +627,40 @@ cudaError_t launch_collect(const RepDev *reps, const RepState *st, const float *
   return cudaGetLastError();
 }
 
-cudaError_t launch_mlp_grad(const float *w, const float *samples, const int *index, int n, float *grad, float *loss,
-                            int grid, cudaStream_t s) {
+int train_image_bytes() { return kGImage; }
+int train_part_floats() { return kPartF; }
+
+static cudaError_t launch_train(const void *fn, dim3 grid, int threads, int smem, void *arg, bool pdl, cudaStream_t s) {
+  void *params[] = {arg};
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl ? 1 : 0;
+  return cudaLaunchKernelExC(&cfg, fn, params);
+}
+
+cudaError_t launch_mlp_grad(const uint8_t *image, const float *samples, int n, int draw_from, uint32_t seed,
+                            uint32_t step, float *part, int grid, bool pdl, cudaStream_t s) {
   static bool attr = false;
   if (!attr) {
     cudaError_t r = cudaFuncSetAttribute(k_mlp_grad, cudaFuncAttributeMaxDynamicSharedMemorySize, kGSmem);
     if (r != cudaSuccess) return r;
     attr = true;
   }
-  GradArgs a{w, samples, index, n, 1.f / (float)n, grad, loss};
-  k_mlp_grad<<<grid, kTW * 32, kGSmem, s>>>(a);
-  return cudaGetLastError();
+  GradArgs a{image, samples, n, 1.f / (float)n, draw_from, seed, step, part};
+  return launch_train((const void *)k_mlp_grad, dim3(grid), kTW * 32, kGSmem, &a, pdl, s);
 }
 
-cudaError_t launch_adam(float *w, float *m, float *v, const float *g, int step, float lr, cudaStream_t s) {
-  k_adam<<<(kPTotal + 255) / 256, 256, 0, s>>>(w, m, v, g, step, lr, 0.9f, 0.999f, 1e-8f);
-  return cudaGetLastError();
-}
-
-cudaError_t launch_batch_index(int *idx, int n, int nsamples, uint32_t seed, uint32_t step, cudaStream_t s) {
-  k_batch_index<<<(n + 255) / 256, 256, 0, s>>>(idx, n, nsamples, seed, step);
-  return cudaGetLastError();
+cudaError_t launch_adam(const float *part, int rows, float *w, float *m, float *v, uint8_t *image, float *grad,
+                        float *loss, int step, float lr, bool pdl, cudaStream_t s) {
+  AdamArgs a{part, rows, w, m, v, image, grad, loss, step, lr, 0.9f, 0.999f, 1e-8f};
+  return launch_train((const void *)k_adam, dim3((kPTotal + 1 + 31) / 32), kAdamWarps * 32, 0, &a, pdl, s);
 }
 
 }  // namespace mcx
