@@ -65,6 +65,7 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_amar
     const bool zper = R.zb == BOUND_PERIODIC;
     const int kb = u.z, ke = u.z + (u.w & kUnitPlanes);
     const uint32_t seed = R.seed, stream = R.stream;
+    const RepDev K = local_constants(R);
     grid_dependency_wait(m);  // directors and state may be written by the previous pass until here
     const unsigned long long sw = S->sweep;
     const float ang = S->ang_var, invT = 1.0f / S->T;
@@ -107,11 +108,11 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_amar
       const float exv[3] = {f1[0], f1[NT], f1[2 * NT]};
       const bool zp = k + 1 < nz || zper;
       const uint4 rw_next = pair_draw(m.pid + m.dpid, c, sw, seed, stream);  // unused after the last plane
-      update_pair_draw<POT, false, FIELD, MODE, PER>(a, R, c, m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, o0, yp, ym, op,
+      update_pair_draw<POT, false, FIELD, MODE, PER>(a, K, c, m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, o0, yp, ym, op,
                                                      om, exv, 0x0101, 1, zp, zm, rw, m.off, ang, invT, ax, ay, az, acc,
                                                      sums);
       if (MODE == MODE_SWEEP_MEASURE && a.meas_both && c == 1) {  // the colour-0 pair of this row (PassArgs::meas_both)
-        measure_opposite<FIELD, PER>(R, o0.v[0], o0.v[1], o0.v[2], m.hasB, sums);
+        measure_opposite<FIELD, PER>(K, o0.v[0], o0.v[1], o0.v[2], m.hasB, sums);
       }
       rw = rw_next;
       *reinterpret_cast<float2 *>(m.A0 + m.off) = ax;

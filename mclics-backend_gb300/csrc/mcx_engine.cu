@@ -79,9 +79,10 @@ struct mcx_engine {
   bool pmarch = false;  // the z-march as one cooperative launch per run of sweeps (grid barriers)
   bool qmarch = false;  // the z-march with four sites per thread (unmasked, nx a multiple of 8)
   bool resident = false;  // runs of sweeps with every replica resident in a cluster's shared memory
-  int res_c = 0, res_nt = 0, res_smem = 0;  // its clusters' CTAs, threads and shared memory (0: cannot run)
-  std::vector<int> res_cut;                 // [nrep][res_c + 2]: rows of its CTAs (launch_resident)
-  int *d_cut = nullptr;
+  struct ResPlan {
+    int c = 0, nt = 0, smem = 0;  // CTAs per cluster (0: cannot run), threads, shared memory
+    int *d_cut = nullptr;         // [nrep][c + 2]: rows of the CTAs (launch_resident)
+  } res[2];                       // of unmeasured and of measured runs
   std::vector<std::vector<int>> rowcnt;     // active sites per row of a masked replica (empty: all)
   // per replica of a masked batch, row j + ny * k: 0 no active site, 1 only
   // bulk sites (point type 1), 2 anything else (empty: unknown)
@@ -228,7 +229,7 @@ static void free_engine(mcx_engine *e) {
   cudaFree(e->d_mlp);
   cudaFree(e->d_units);
   cudaFree(e->d_lunits);
-  cudaFree(e->d_cut);
+  for (auto &r : e->res) cudaFree(r.d_cut);
   cudaFree(e->d_w);
   cudaFree(e->d_am);
   cudaFree(e->d_av);
@@ -278,53 +279,51 @@ static void effective_bounds(mcx_replica_desc &d) {
 // waves, which keeps the last wave from running mostly idle.
 // The class of a unit of a masked replica from its rows and planes and the
 // rows and planes next to them: kUnitDead when none holds an active site,
-// kUnitBulk when all hold bulk sites only, 0 otherwise.
+// kUnitBulk when all hold bulk sites only (with kUnitFull when they all exist,
+// the rows' x neighbours too, and pairs are complete), 0 otherwise.
 static int unit_class(const mcx_engine *e, const int4 &u, int nt) {
   const std::vector<uint8_t> &act = e->rowact[u.x];
   if (act.empty()) return 0;
   const RepDev &R = e->rep[u.x];
-  if (u.w & kUnitTiled) {  // the tile's rows, over its x range (segact), and the rows and planes next to them
-    const std::vector<uint8_t> &seg = e->segact[u.x];
-    const int nseg = (R.hp + kTileW - 1) / kTileW;
-    const int j0 = u.y >> kTileQBits, sc = (u.y & ((1 << kTileQBits) - 1)) / kTileW;
-    const int j1 = std::min(j0 + nt / kTileW, R.ny) - 1, nk = u.w & kUnitPlanes;
-    unsigned seen = 0;
-    for (int k = u.z - 1; k <= u.z + nk; k++) {
-      int kk = k;
-      if (kk < 0 || kk >= R.nz) {
-        if (R.zb != BOUND_PERIODIC) continue;
-        kk = (kk + R.nz) % R.nz;
-      }
-      for (int j = j0 - 1; j <= j1 + 1; j++) {
-        int jj = j;
-        if (jj < 0 || jj >= R.ny) {
-          if (R.yb != BOUND_PERIODIC) continue;
-          jj = (jj + R.ny) % R.ny;
-        }
-        seen |= 1u << seg[((size_t)jj + (size_t)R.ny * kk) * nseg + sc];
-      }
-    }
-    return seen == 1u ? kUnitDead : (seen == 2u ? kUnitBulk : 0);
+  const bool tiled = (u.w & kUnitTiled) != 0;
+  const int nk = u.w & kUnitPlanes;
+  int j0, j1, sc = 0, nseg = 0;
+  bool full = R.nx % 4 == 0;
+  if (tiled) {  // the tile's rows, over its x range with the x neighbours (segact)
+    nseg = (R.hp + kTileW - 1) / kTileW;
+    sc = (u.y & ((1 << kTileQBits) - 1)) / kTileW;
+    j0 = u.y >> kTileQBits;
+    j1 = std::min(j0 + nt / kTileW, R.ny) - 1;
+    if (R.xb != BOUND_PERIODIC && (sc == 0 || (sc + 1) * 4 * kTileW >= R.nx)) full = false;
+  } else {
+    j0 = u.y / R.hp;
+    j1 = (std::min(u.y + nt, R.hp * R.ny) - 1) / R.hp;
+    if (R.xb != BOUND_PERIODIC) full = false;
   }
-  const int pend = std::min(u.y + nt, R.hp * R.ny);
-  const int j0 = u.y / R.hp, j1 = (pend - 1) / R.hp, nk = u.w & kUnitPlanes;
   unsigned seen = 0;  // bit c: a row of class c
   for (int k = u.z - 1; k <= u.z + nk; k++) {
     int kk = k;
     if (kk < 0 || kk >= R.nz) {
-      if (R.zb != BOUND_PERIODIC) continue;
+      if (R.zb != BOUND_PERIODIC) {
+        full = false;
+        continue;
+      }
       kk = (kk + R.nz) % R.nz;
     }
     for (int j = j0 - 1; j <= j1 + 1; j++) {
       int jj = j;
       if (jj < 0 || jj >= R.ny) {
-        if (R.yb != BOUND_PERIODIC) continue;
+        if (R.yb != BOUND_PERIODIC) {
+          full = false;
+          continue;
+        }
         jj = (jj + R.ny) % R.ny;
       }
-      seen |= 1u << act[(size_t)jj + (size_t)R.ny * kk];
+      const size_t row = (size_t)jj + (size_t)R.ny * kk;
+      seen |= 1u << (tiled ? e->segact[u.x][row * nseg + sc] : act[row]);
     }
   }
-  return seen == 1u ? kUnitDead : (seen == 2u ? kUnitBulk : 0);
+  return seen == 1u ? kUnitDead : (seen == 2u ? (full ? kUnitBulk | kUnitFull : kUnitBulk) : 0);
 }
 
 // Site pairs of a plane per z-march work unit: one per thread, two per thread
@@ -465,6 +464,15 @@ static void plan_march(mcx_engine *e) {
     }
   }
   mark_dead_units(e);
+  // units without an active site in or next to them have nothing to do: they
+  // are not launched (the persistent form keeps them; its CTAs all take part in
+  // its barriers)
+  if (e->var.mask && !e->pmarch) {
+    for (const int4 &u : e->units)
+      if (u.w & kUnitDead) e->rep[u.x].mcta--;
+    e->units.erase(std::remove_if(e->units.begin(), e->units.end(), [](const int4 &u) { return (u.w & kUnitDead) != 0; }),
+                   e->units.end());
+  }
 }
 
 extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engine **out) {
@@ -1090,22 +1098,23 @@ static double march_estimate(const mcx_engine *e) {
   return 2.3 + (e->var.mask ? 1.5 : 1.0) * 0.5 * sites / rate;
 }
 
-// Chooses the resident form's cluster size and CTA size: the shape with the
-// least estimated time per pass.  Returns the estimate, 0 when no shape runs
-// this batch (a replica's rows do not fit a cluster's shared memory).
+// Chooses the resident form's cluster and CTA size for unmeasured and measured
+// runs: the shape with the least estimated time per pass.  Returns the estimate
+// for unmeasured ones, 0 when no shape runs this batch (a replica's rows do not
+// fit a cluster's shared memory).
 static double plan_resident(mcx_engine *e) {
-  e->res_c = 0;
   int minz = 1 << 30, dev = 0, nsm = 0;
   for (const RepDev &R : e->rep) minz = std::min(minz, R.nz);
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  double best = 1e30;
-  std::vector<int> cut;
+  double best[2] = {1e30, 1e30};
+  std::vector<int> cut, keep[2];
+  for (auto &r : e->res) r.c = 0;
   for (int C : {1, 2, 4, 8, 16}) {
     if (C > minz) break;  // a CTA's rows span at least one plane
     long long smem = 0;
     int sites = 0;
-    // the replicas of one shape are cut alike; look at the memory first
+    // even shares first: most shapes that do not fit need no cutting to show it
     for (const RepDev &R : e->rep)
       smem = std::max(smem, resident_smem_bytes(R, e->var.mask, (R.ny * R.nz + C - 1) / C));
     if (smem > kResidentSmem) continue;
@@ -1117,33 +1126,39 @@ static double plan_resident(mcx_engine *e) {
     }
     if (smem > kResidentSmem) continue;
     const int pairs = (sites + 3) / 4;  // of one colour
-    int last = 0;
-    for (int cap = 128; cap <= resident_max_threads(); cap *= 2) {
-      const int it = (pairs + cap - 1) / cap, nt = std::max(64, ((pairs + it - 1) / it + 31) / 32 * 32);
-      if (nt == last) continue;
-      last = nt;
-      const int live = resident_clusters(e->var, C, nt, (int)smem);
-      if (live <= 0) continue;
-      const double est = resident_estimate(e, pairs, C, nt, live, nsm);
-      if (est < best) {
-        best = est;
-        e->res_c = C;
-        e->res_nt = nt;
-        e->res_smem = (int)smem;
-        e->res_cut = cut;
+    for (int m = 0; m < 2; m++) {
+      const int mode = m ? MODE_SWEEP_MEASURE : MODE_SWEEP;
+      int last = 0;
+      for (int cap : {128, 256, resident_max_threads(e->var.mask, mode)}) {
+        const int it = (pairs + cap - 1) / cap, nt = std::max(64, ((pairs + it - 1) / it + 31) / 32 * 32);
+        if (nt == last) continue;
+        last = nt;
+        const int live = resident_clusters(e->var, mode, C, nt, (int)smem);
+        if (live <= 0) continue;
+        const double est = resident_estimate(e, pairs, C, nt, live, nsm);
+        if (est < best[m]) {
+          best[m] = est;
+          e->res[m].c = C;
+          e->res[m].nt = nt;
+          e->res[m].smem = (int)smem;
+          keep[m] = cut;
+        }
       }
     }
   }
-  if (e->res_c == 0) return 0.0;
-  cudaFree(e->d_cut);
-  e->d_cut = nullptr;
-  if (cudaMalloc(&e->d_cut, sizeof(int) * e->res_cut.size()) != cudaSuccess ||
-      cudaMemcpy(e->d_cut, e->res_cut.data(), sizeof(int) * e->res_cut.size(), cudaMemcpyHostToDevice) != cudaSuccess) {
-    cudaGetLastError();
-    e->res_c = 0;
-    return 0.0;
+  for (int m = 0; m < 2; m++) {
+    mcx_engine::ResPlan &r = e->res[m];
+    cudaFree(r.d_cut);
+    r.d_cut = nullptr;
+    if (e->res[0].c == 0 || e->res[1].c == 0) return 0.0;
+    if (cudaMalloc(&r.d_cut, sizeof(int) * keep[m].size()) != cudaSuccess ||
+        cudaMemcpy(r.d_cut, keep[m].data(), sizeof(int) * keep[m].size(), cudaMemcpyHostToDevice) != cudaSuccess) {
+      cudaGetLastError();
+      e->res[0].c = e->res[1].c = 0;
+      return 0.0;
+    }
   }
-  return best;
+  return best[0];
 }
 
 // Whether the sweeps' kernels leave the inactive sites' field energy to
@@ -1169,8 +1184,9 @@ static mcx_status run_sweeps(mcx_engine *e, int n, int m) {
     PassArgs pa = pass_args(e);
     for (int done = 0; done < n;) {
       const int k = std::min(n - done, kResidentSweeps);
-      CK(e, launch_resident(e->var, m ? MODE_SWEEP_MEASURE : MODE_SWEEP, pa, e->d_cut, e->nrep, k, e->res_c, e->res_nt,
-                            e->res_smem, e->stream));
+      const mcx_engine::ResPlan &r = e->res[m ? 1 : 0];
+      CK(e, launch_resident(e->var, m ? MODE_SWEEP_MEASURE : MODE_SWEEP, pa, r.d_cut, e->nrep, k, r.c, r.nt, r.smem,
+                            e->stream));
       e->launches += 1;
       done += k;
     }
@@ -1533,7 +1549,8 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
       const int reps = 32;
       for (int w = 0; w < 2; w++) {
         CKA(cudaEventRecord(t0, e->stream));
-        CKA(launch_resident(e->var, MODE_SWEEP, pa, e->d_cut, e->nrep, reps, e->res_c, e->res_nt, e->res_smem, e->stream));
+        const mcx_engine::ResPlan &r = e->res[0];
+        CKA(launch_resident(e->var, MODE_SWEEP, pa, r.d_cut, e->nrep, reps, r.c, r.nt, r.smem, e->stream));
         CKA(cudaEventRecord(t1, e->stream));
         CKA(cudaEventSynchronize(t1));
         e->launches++;

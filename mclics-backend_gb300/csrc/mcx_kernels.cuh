@@ -40,6 +40,9 @@ constexpr int kUnitDead = 1 << 30;
 // the unmasked update, which gives the same result there without the mask's
 // loads and weights.
 constexpr int kUnitBulk = 1 << 29;
+// kUnitFull marks a bulk unit all of whose bonds exist and whose pairs are
+// complete: the update with constant weights.
+constexpr int kUnitFull = 1 << 27;
 // kUnitTiled marks a unit of the z-march that is a tile of kTileW pairs of a
 // row times NT / kTileW rows (its second field (j0 << 12) | q0: first row,
 // first pair of the row) rather than NT consecutive pairs of the plane.
@@ -47,7 +50,7 @@ constexpr int kUnitBulk = 1 << 29;
 // tiles, so that the units inside the droplet hold only bulk sites and run
 // the unmasked update.
 constexpr int kUnitTiled = 1 << 28;
-constexpr int kUnitPlanes = kUnitTiled - 1;
+constexpr int kUnitPlanes = kUnitFull - 1;
 constexpr int kTileLg = 2, kTileW = 1 << kTileLg;  // pairs per tile row (one 32-byte sector)
 constexpr int kTileQBits = 12;                      // q0 field: hp < 4096
 
@@ -139,9 +142,9 @@ cudaError_t launch_pmarch(const Variant &v, int mode, const PassArgs &a, int nt,
 // cut: per replica the first row (j + ny k) of each of its C CTAs, the row
 // count and the largest share; every share spans at least one plane.
 long long resident_smem_bytes(const RepDev &R, bool mask, int n);
-int resident_max_threads();
+int resident_max_threads(bool mask, int mode);
 constexpr int kResidentSmem = 220 * 1024;  // dynamic shared memory of a CTA, below the 227 KB limit
-int resident_clusters(const Variant &v, int C, int nt, int smem);
+int resident_clusters(const Variant &v, int mode, int C, int nt, int smem);
 cudaError_t launch_resident(const Variant &v, int mode, const PassArgs &a, const int *cut, int nrep, int nsweeps,
                             int C, int nt, int smem, cudaStream_t st);
 // The learned-proposal z-march (mcx_lmarch.cu): units of lmarch_block_threads()

@@ -93,6 +93,29 @@ __device__ __forceinline__ void load_opair_at(const March &m, int off, int offp,
   }
 }
 
+// The constants an unmasked update reads, in registers.  A pass whose loop
+// holds barriers or asynchronous copies reads global constants again after
+// each of them (their memory clobbers), a load of some hundred cycles per
+// plane.
+__device__ __forceinline__ RepDev local_constants(const RepDev &R) {
+  RepDev c;
+  c.A = R.A;
+  c.ga = R.ga;
+  c.gb = R.gb;
+  c.gc = R.gc;
+  c.mu = R.mu;
+  c.sigma = R.sigma;
+  c.gconst = R.gconst;
+  c.B1 = R.B1;
+  c.C = R.C;
+  c.elecA = R.elecA;
+  c.elecE = R.elecE;
+  c.ex = R.ex;
+  c.ey = R.ey;
+  c.ez = R.ez;
+  return c;
+}
+
 // The thread's march state for pair p of the plane (p < hp * ny) of colour
 // c, starting at plane kb: its geometry, y rows, x extras and the offsets of
 // plane kb.  Constants only (no director or state reads).  ODD false: the
@@ -155,8 +178,13 @@ __device__ __forceinline__ void march_init(const PassArgs &a, const RepDev &R, i
 #ifndef MCX_MARCH_MASK_REGS
 #define MCX_MARCH_MASK_REGS 128
 #endif
-template <int POT, bool MASK, int NT>
+template <int POT, bool MASK, int NT, int MODE = MODE_SWEEP>
 constexpr int march_min_blocks() {
+  // measured masked passes at 168 registers: at 128 they spill 460 to 540 bytes,
+  // more than the L1 cache holds for 16 warps (8 droplets of 96^3: 65.7 us a
+  // pass against 71.4; unmeasured ones spill 120 bytes and are slower at 144 or
+  // 168, 52.6 and 55.0 against 51.8)
+  if (MASK && MODE == MODE_SWEEP_MEASURE) return 65536 / (NT * 168) > 0 ? 65536 / (NT * 168) : 1;
   return POT == POT_LL && !MASK ? (NT == 64 ? 9 : (NT == 128 ? MCX_MARCH_LL128_BLOCKS : MCX_MARCH_LL256_BLOCKS))
                                 : (MCX_MARCH_MASK_REGS > 0 ? 65536 / (NT * MCX_MARCH_MASK_REGS) : 1);
 }

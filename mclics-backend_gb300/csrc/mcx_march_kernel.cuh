@@ -85,7 +85,7 @@ __device__ __forceinline__ void march_chunk(const PassArgs &a, const RepDev &R, 
 }
 
 template <int POT, bool MASK, bool FIELD, int MODE, int NT, bool PER, bool ODD>
-__global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>()) k_march(PassArgs a) {
+__global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT, MODE>()) k_march(PassArgs a) {
   static_assert(MODE == MODE_SWEEP || MODE == MODE_SWEEP_MEASURE, "sweep modes only");
   const int4 u = a.units[blockIdx.x];
   const int r = u.x, c = a.colour;
@@ -116,6 +116,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT>()) k_march
     if (MODE == MODE_SWEEP_MEASURE && !(MASK && FIELD) && threadIdx.x < kQ) slot = ring_slot(a, S);
     if (MASK && (u.w & kUnitDead)) {
       // no active site in or next to the unit: nothing to update or to measure
+    } else if (MASK && !ODD && (u.w & kUnitFull)) {  // only bulk sites around, every bond present: constant weights
+      march_chunk<POT, false, FIELD, MODE, true>(a, R, c, m, kb, ke, S, acc, sums);
     } else if (MASK && (u.w & kUnitBulk))  // only bulk sites around: the unmasked update
       march_chunk<POT, false, FIELD, MODE, false>(a, R, c, m, kb, ke, S, acc, sums);
     else

@@ -39,7 +39,11 @@
 
 namespace mcx {
 
-constexpr int kResThreads = 512;  // most threads per CTA
+// Most threads per CTA: measured masked builds take up to 168 registers per
+// thread (at 128 they spill 260 bytes; 16 droplets of 25^3: 6.9 us a pass
+// against 7.9; unmeasured ones fit 128, and at 168 fewer CTAs share an SM, 5.2
+// against 4.3)
+constexpr int kResThreads = 512, kResMaskThreads = 384;
 
 // A pair of the CTA's rows: offsets (floats) into a (colour, component) plane
 // of shared memory, and which of its bonds exist.
@@ -186,7 +190,7 @@ __device__ __forceinline__ bool res_wait(uint64_t *bar, uint32_t parity) {
 }
 
 template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
-__global__ void __launch_bounds__(kResThreads, 1) k_resident(PassArgs a, const int *cut, int nsweeps, int C) {
+__global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskThreads : kResThreads, 1) k_resident(PassArgs a, const int *cut, int nsweeps, int C) {
   constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
   extern __shared__ __align__(16) uint8_t res_smem[];
   __shared__ unsigned s_cnt[3];            // accepted moves of sweeps i, i+1, i+2 (mod 3), every CTA's
@@ -526,7 +530,9 @@ long long resident_smem_bytes(const RepDev &R, bool mask, int n) {
   return 24ll * L.fl + (long long)sizeof(ResPair) * L.pairs + (mask ? 2ll * L.pt + 4ll * L.pairs : 0);
 }
 
-int resident_max_threads() { return kResThreads; }
+int resident_max_threads(bool mask, int mode) {
+  return mask && mode == MODE_SWEEP_MEASURE ? kResMaskThreads : kResThreads;
+}
 
 static void res_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int nrep, int C, int nt, int smem,
                        cudaStream_t st) {
@@ -542,28 +548,21 @@ static void res_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int nre
 }
 
 // Clusters of C CTAs of nt threads with smem bytes the GPU holds at once (0:
-// the shape cannot run); sets the kernels' attributes.
-int resident_clusters(const Variant &v, int C, int nt, int smem) {
-  int best = 1 << 30;
-  for (int mode : {MODE_SWEEP, MODE_SWEEP_MEASURE}) {
-    const void *fn = res_kernel(v, mode);
-    // the largest values any engine uses: the attributes belong to the kernel
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem) != cudaSuccess ||
-        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    cudaLaunchConfig_t cfg = {};
-    cudaLaunchAttribute at;
-    res_config(cfg, at, 1, C, nt, smem, nullptr);
-    int n = 0;
-    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
-      cudaGetLastError();
-      return 0;
-    }
-    best = n < best ? n : best;
+// the shape cannot run); sets the kernel's attributes.
+int resident_clusters(const Variant &v, int mode, int C, int nt, int smem) {
+  const void *fn = res_kernel(v, mode);
+  // the largest values any engine uses: the attributes belong to the kernel
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute at;
+  res_config(cfg, at, 1, C, nt, smem, nullptr);
+  int n = 0;
+  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem) != cudaSuccess ||
+      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
   }
-  return best;
+  return n;
 }
 
 cudaError_t launch_resident(const Variant &v, int mode, const PassArgs &a, const int *cut, int nrep, int nsweeps,
