@@ -89,6 +89,9 @@ struct PassArgs {
   // the Q-tensor and field terms of the colour-0 sites, read from the opposite
   // pairs it loads anyway (one reduction per sweep instead of two)
   int meas_both;
+  // measured masked passes of the z-marches add inactive sites' field energy
+  // site by site (else k_idle_field has added it for the run)
+  int idle_in_pass;
 };
 
 struct FlushArgs {

@@ -143,7 +143,7 @@ __device__ __forceinline__ void update_pair_learned(const PassArgs &a, const Rep
   const bool accA = S.actA && A.u < __expf(lr.x), accB = S.actB && B.u < __expf(lr.y);
   accept_pair(accA, accB, p, ax, ay, az);
   acc += (accA ? 1u : 0u) + (accB ? 1u : 0u);
-  if (MEAS) measure_pair<POT, MASK, FIELD, PER>(R, c, S, E, accA, accB, ax, ay, az, sums);
+  if (MEAS) measure_pair<POT, MASK, FIELD, PER>(R, c, S, E, accA, accB, ax, ay, az, sums, a.idle_in_pass != 0);
 }
 
 // the tensor-core form holds 63 KB of shared memory: three CTAs per SM, so
@@ -199,7 +199,9 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
     tmem = *tslot;
   }
   grid_dependency_wait(m);
-  if (!(MASK && (u.w & kUnitDead))) {  // a dead unit: no active site in or next to it
+  if (MASK && (u.w & kUnitDead)) {  // no active site in or next to it
+    if (valid && a.idle_in_pass) dead_unit<FIELD, MODE>(R, m, kb, ke, sums);
+  } else {
     const unsigned long long sw = S->sweep;
     const float T = S->T, invT = 1.0f / S->T;
 #pragma unroll 1
@@ -212,7 +214,7 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
       // network, and only the colour-1 sites' bonds to active ones are measured
       // (the tensor-core form evaluates the network per CTA and does not skip)
       const bool idle = !TC && MASK && __all_sync(0xffffffffu, !valid || pself == 0);
-      if (!(idle && (MODE == MODE_SWEEP || c == 0))) {
+      if (!(idle && (MODE == MODE_SWEEP || (c == 0 && !(FIELD && a.idle_in_pass))))) {
         float4 yA = make_float4(0.f, 0.f, 0.f, 0.f), yB = yA;
         if (!idle) {
           Hood h;

@@ -37,10 +37,11 @@ __device__ __forceinline__ void measure_opposite(const RepDev &R, const float2 &
                                                  bool hasB, Q &sums) {
   const V2 n = {pk(x), pk(y), pk(z)};
   const f32x2 m = pk(1.f, hasB ? 1.f : 0.f);
-  add_q<PER>(sums, n, m);
+  sums.tensor(n, PER ? n : mul2(n, m));
   if (FIELD) {
-    const f32x2 ef = field_energy2(R, n);
-    sums.add(0, PER ? ef : mul2(ef, m));
+    f32x2 ef = field_energy2(R, n);
+    if (!PER) ef = mul2(ef, m);
+    sums.template energy<false, true>(0, 0ull, ef, ef, 0ull, 0ull, 0ull);
   }
 }
 
@@ -78,6 +79,24 @@ __device__ __forceinline__ void grid_dependency_wait(March &m) {
                : "+l"(m.A0), "+l"(m.A1), "+l"(m.A2), "+l"(m.O0), "+l"(m.O1), "+l"(m.O2)
                :
                : "memory");
+}
+
+// A unit without an active site in or next to it (kUnitDead) of an engine whose
+// passes add inactive sites' field energy themselves (PassArgs::idle_in_pass).
+template <bool FIELD, int MODE, class Q>
+__device__ __forceinline__ void dead_unit(const RepDev &R, March &m, int kb, int ke, Q &sums) {
+  if (!(FIELD && MODE == MODE_SWEEP_MEASURE)) return;
+  int s = m.s;
+#pragma unroll 1
+  for (int k = kb; k < ke; k++) {
+    const V2 n = {pk(*reinterpret_cast<const float2 *>(m.A0 + m.off)), pk(*reinterpret_cast<const float2 *>(m.A1 + m.off)),
+                  pk(*reinterpret_cast<const float2 *>(m.A2 + m.off))};
+    const bool hereA = !(s && m.tail == 1), hereB = m.hasB && !(s && m.tail == 2);
+    const f32x2 f = mul2(field_energy2(R, n), pk(hereA ? 1.f : 0.f, hereB ? 1.f : 0.f));
+    sums.template energy<false, true>(0, 0ull, f, 0ull, 0ull, 0ull, 0ull);
+    m.off += m.dz;
+    s ^= 1;
+  }
 }
 
 template <bool MASK>
@@ -355,42 +374,41 @@ __device__ __forceinline__ PairEnergy pair_energy(const PassArgs &a, const RepDe
 }
 
 // What a measured pass adds for a pair with its final directors (ax, ay, az).
+// Each bond counts in the local energy of each active end, from the colour-1
+// side; the all-site energy also counts inactive sites' bonds to active ones,
+// and their field energy with idle (k_idle_field adds it otherwise).
 template <int POT, bool MASK, bool FIELD, bool PER, class Q>
 __device__ __forceinline__ void measure_pair(const RepDev &R, int c, const PairSlots &S, const PairEnergy &E, bool accA,
-                                             bool accB, const float2 &ax, const float2 &ay, const float2 &az, Q &sums) {
-  // the final directors and their energies.  Each bond counts in the local
-  // energy of each active end, from the colour-1 side; the all-site energy
-  // also counts inactive sites' bonds to active ones.  (The field energy of
-  // inactive sites is k_idle_field's.)
+                                             bool accB, const float2 &ax, const float2 &ay, const float2 &az, Q &sums,
+                                             bool idle) {
   constexpr bool ALL = PER;  // both sites count
   const V2 nf = {pk(ax), pk(ay), pk(az)};
   const f32x2 m = pk(S.actA ? 1.f : 0.f, S.actB ? 1.f : 0.f);
-  add_q<ALL>(sums, nf, m);
-  f32x2 site = 0ull;
-  if (MASK) site = pick2(accA, accB, E.s_new, E.s_old);
-  if (FIELD) site = add2(site, pick2(accA, accB, E.f_new, E.f_old));
-  if ((MASK || FIELD) && !ALL) site = mul2(site, m);
-  f32x2 all = site, valid = site;
+  sums.tensor(nf, ALL ? nf : mul2(nf, m));
+  f32x2 s = 0ull, f0 = 0ull, f1 = 0ull, b0 = 0ull, b1 = 0ull, x = 0ull;
+  if (MASK) s = mul2(pick2(accA, accB, E.s_new, E.s_old), m);
+  if (FIELD) {
+    const f32x2 f = pick2(accA, accB, E.f_new, E.f_old);
+    f0 = f1 = ALL ? f : mul2(f, m);
+    if (MASK && idle) f0 = mul2(f, pk(S.hereA ? 1.f : 0.f, S.hereB ? 1.f : 0.f));
+  }
   if (c == 1) {
     f32x2 eb = pick2(accA, accB, E.e_new, E.e_old);
     if (POT == POT_LL) eb = mul2(pk1(bond_scale<POT>(R)), eb);
     eb = add_bond_const<POT, !PER>(R, S.w, eb);
     if (ALL) {
-      all = fma2(pk1(2.f), eb, all);
+      b0 = b1 = add2(eb, eb);
     } else {
-      const f32x2 k2 = pk(S.actA ? 2.f : (S.hereA ? 1.f : 0.f), S.actB ? 2.f : (S.hereB ? 1.f : 0.f));
-      all = fma2(k2, eb, all);
+      b0 = mul2(pk(S.actA ? 2.f : (S.hereA ? 1.f : 0.f), S.actB ? 2.f : (S.hereB ? 1.f : 0.f)), eb);
+      if (Q::kMasked) b1 = mul2(pk(S.actA ? 2.f : 0.f, S.actB ? 2.f : 0.f), eb);
       if (MASK) {
-        valid = fma2(mul2(pk1(2.f), m), eb, valid);
-        f32x2 xb = pick2(accA, accB, E.x_new, E.x_old);
-        if (POT == POT_LL) xb = mul2(pk1(bond_scale<POT>(R)), xb);
-        all = add2(all, add_bond_const<POT, true>(R, E.x, xb));
+        x = pick2(accA, accB, E.x_new, E.x_old);
+        if (POT == POT_LL) x = mul2(pk1(bond_scale<POT>(R)), x);
+        x = add_bond_const<POT, true>(R, E.x, x);
       }
     }
   }
-  if (MASK || FIELD || c == 1) sums.add(0, all);
-  if (MASK) sums.add(1, valid);
-  else if (Q::kMasked && (FIELD || c == 1)) sums.add(1, all);  // a masked batch's bulk sites
+  sums.template energy<MASK, FIELD>(c, s, f0, f1, b0, b1, x);
 }
 
 __device__ __forceinline__ void accept_pair(bool accA, bool accB, const V2 &p, float2 &ax, float2 &ay, float2 &az) {
@@ -432,7 +450,7 @@ __device__ __forceinline__ void update_pair_draw(const PassArgs &a, const RepDev
   const bool accA = S.actA && u2.x < __expf(arg.x), accB = S.actB && u2.y < __expf(arg.y);
   accept_pair(accA, accB, p, ax, ay, az);
   acc += (accA ? 1u : 0u) + (accB ? 1u : 0u);
-  if (MEAS) measure_pair<POT, MASK, FIELD, PER>(R, c, S, E, accA, accB, ax, ay, az, sums);
+  if (MEAS) measure_pair<POT, MASK, FIELD, PER>(R, c, S, E, accA, accB, ax, ay, az, sums, a.idle_in_pass != 0);
 }
 
 // The pair's Philox draw (counter: pair index, sweep, colour; key: seed,

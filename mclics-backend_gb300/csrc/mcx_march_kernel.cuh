@@ -33,7 +33,9 @@ __device__ __forceinline__ void march_plane(const PassArgs &a, const RepDev &R, 
     // two inactive sites: nothing moves, and a measured sweep adds only the
     // colour-1 sites' bonds to active ones (a warp of such pairs skips the draw
     // and the arithmetic)
-    if (pself == 0 && (MODE == MODE_SWEEP || c == 0 || (o0.pt | yp.pt | ym.pt | op.pt | om.pt | pex) == 0)) return;
+    if (pself == 0 && !(FIELD && MODE == MODE_SWEEP_MEASURE && a.idle_in_pass) &&
+        (MODE == MODE_SWEEP || c == 0 || (o0.pt | yp.pt | ym.pt | op.pt | om.pt | pex) == 0))
+      return;
   }
   update_pair<POT, MASK, FIELD, MODE, PER>(a, R, c, m.s, m.hasB, m.ee0, m.ee1, m.eyp, m.eym, o0, yp, ym, op, om, exv,
                                            pself, pex, zp, zm, m.pid, m.off, seed, stream, sw, ang, invT, ax, ay, az,
@@ -115,7 +117,8 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT, MODE>()) k
     // not in the masked field build, where the live register cost it 1.1%
     if (MODE == MODE_SWEEP_MEASURE && !(MASK && FIELD) && threadIdx.x < kQ) slot = ring_slot(a, S);
     if (MASK && (u.w & kUnitDead)) {
-      // no active site in or next to the unit: nothing to update or to measure
+      // no active site in or next to the unit: nothing to update
+      if (a.idle_in_pass) dead_unit<FIELD, MODE>(R, m, kb, ke, sums);
     } else if (MASK && !ODD && (u.w & kUnitFull)) {  // only bulk sites around, every bond present: constant weights
       march_chunk<POT, false, FIELD, MODE, true>(a, R, c, m, kb, ke, S, acc, sums);
     } else if (MASK && (u.w & kUnitBulk))  // only bulk sites around: the unmasked update

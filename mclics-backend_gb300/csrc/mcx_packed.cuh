@@ -275,39 +275,59 @@ __device__ __forceinline__ float2 accept_uniforms(const uint4 &w) {
   return unpk(add2(pk(one_plus(a), one_plus(b)), pk1(-1.f)));
 }
 
-// Sums of a measured pass (kQ quantities) over a thread's pairs, both sites of
-// a pair in the halves of a value.  MASKED: the energy of active sites is a sum
-// of its own.
+// Sums of a measured pass (kQ quantities) over a thread's pairs, in the scalar
+// update's order: site A's terms, then site B's, one FP32 addition each (a
+// packed accumulator per quantity would save some additions and give other last
+// bits, which the statistics of lattices of some hundred sites show in their
+// ninth digit).  MASKED: the energy of active sites is a sum of its own.
 template <bool MASKED>
 struct PairSums {
   static constexpr bool kMasked = MASKED;
-  f32x2 v[kQ];
+  float v[kQ];
   __device__ __forceinline__ void clear() {
 #pragma unroll
-    for (int q = 0; q < kQ; q++) v[q] = 0ull;
+    for (int q = 0; q < kQ; q++) v[q] = 0.f;
   }
-  __device__ __forceinline__ void add(int q, f32x2 t) { v[q] = add2(v[q], t); }
-  __device__ __forceinline__ void add_product(int q, f32x2 a, f32x2 b) { v[q] = fma2(a, b, v[q]); }
+  __device__ __forceinline__ void site_q(float x, float y, float z, float xm, float ym, float zm) {
+    v[2] = fmaf(xm, x, v[2]);
+    v[3] = fmaf(xm, y, v[3]);
+    v[4] = fmaf(xm, z, v[4]);
+    v[5] = fmaf(ym, y, v[5]);
+    v[6] = fmaf(zm, y, v[6]);
+  }
+  // Q-tensor products of a pair; nm: its directors, zero for a site that does not count
+  __device__ __forceinline__ void tensor(const V2 &n, const V2 &nm) {
+    const float2 x = unpk(n.x), y = unpk(n.y), z = unpk(n.z), xm = unpk(nm.x), ym = unpk(nm.y), zm = unpk(nm.z);
+    site_q(x.x, y.x, z.x, xm.x, ym.x, zm.x);
+    site_q(x.y, y.y, z.y, xm.y, ym.y, zm.y);
+  }
+  // energies: anchoring s, field (all sites f0, active ones f1), bonds (b0, b1)
+  // and bonds to inactive sites x
+  template <bool MASK, bool FIELD>
+  __device__ __forceinline__ void energy(int c, f32x2 s, f32x2 f0, f32x2 f1, f32x2 b0, f32x2 b1, f32x2 x) {
+#pragma unroll
+    for (int h = 0; h < 2; h++) {
+      auto of = [&](f32x2 t) { return h ? unpk(t).y : unpk(t).x; };
+      if (MASK) v[0] += of(s);
+      if (FIELD) v[0] += of(f0);
+      if (c == 1) {
+        v[0] += of(b0);
+        if (MASK) v[0] += of(x);
+      }
+      if (MASKED) {
+        if (MASK) v[1] += of(s);
+        if (FIELD) v[1] += of(f1);
+        if (c == 1) v[1] += of(b1);
+      }
+    }
+  }
   __device__ __forceinline__ void fold(float out[kQ]) const {
 #pragma unroll
-    for (int q = 0; q < kQ; q++) {
-      const float2 u = unpk(v[q]);
-      out[q] = u.x + u.y;
-    }
+    for (int q = 0; q < kQ; q++) out[q] = v[q];
   }
 };
 
-// The Q-tensor products of a pair of sites, m 1 for sites that count and 0 for
-// others.
-template <bool ALL, class Q>
-__device__ __forceinline__ void add_q(Q &sums, const V2 &n, f32x2 m) {
-  const f32x2 x = ALL ? n.x : mul2(n.x, m), y = ALL ? n.y : mul2(n.y, m), z = ALL ? n.z : mul2(n.z, m);
-  sums.add_product(2, x, n.x);
-  sums.add_product(3, x, n.y);
-  sums.add_product(4, x, n.z);
-  sums.add_product(5, y, n.y);
-  sums.add_product(6, y, n.z);
-}
+__device__ __forceinline__ V2 mul2(const V2 &n, f32x2 m) { return {mul2(n.x, m), mul2(n.y, m), mul2(n.z, m)}; }
 
 // Electric term of both sites (field_energy).
 __device__ __forceinline__ f32x2 field_energy2(const RepDev &R, const V2 &n) {

@@ -104,7 +104,28 @@ struct SplitSums {
       hi[q] = s;
     }
   }
-  __device__ __forceinline__ void add_product(int q, f32x2 a, f32x2 b) { add(q, mul2(a, b)); }
+  __device__ __forceinline__ void tensor(const V2 &n, const V2 &nm) {
+    add(2, mul2(nm.x, n.x));
+    add(3, mul2(nm.x, n.y));
+    add(4, mul2(nm.x, n.z));
+    add(5, mul2(nm.y, n.y));
+    add(6, mul2(nm.z, n.y));
+  }
+  template <bool MASK, bool FIELD>
+  __device__ __forceinline__ void energy(int c, f32x2 s, f32x2 f0, f32x2 f1, f32x2 b0, f32x2 b1, f32x2 x) {
+    if (!MASK && !FIELD && c != 1) return;
+    f32x2 all = b0, valid = b1;
+    if (FIELD) {
+      all = add2(all, f0);
+      valid = add2(valid, f1);
+    }
+    if (MASK) {
+      all = add2(all, add2(s, x));
+      valid = add2(valid, s);
+    }
+    add(0, all);
+    if (MASKED) add(1, valid);
+  }
 };
 
 // (h, l) + (x, y), the rounding error of the high parts kept
