@@ -263,7 +263,8 @@ int mcx_get_pass(const mcx_engine *eng);
 /* The z-march pass's shape: CTA size (64, 128 or 256 threads, one site pair
  * each) and chunk depth (planes per CTA; planes <= 0 cuts near-equal chunks
  * so that the work units fill max(1, -planes) waves of the CTAs the GPU holds
- * at once).  Default 128 x 8. */
+ * at once).  The default is chosen from the batch's potential, masks and size
+ * (balanced chunks of 64, 128 or 256 threads). */
 mcx_status mcx_set_march_shape(mcx_engine *eng, int block, int planes);
 /* Autotuner: times the z-march pass (register form and, for unmasked batches,
  * the prefetching and four-site forms) for block sizes {64, 128, 256} and chunk

@@ -73,6 +73,7 @@ struct mcx_engine {
   // z-march pass (the default sweep pass of the plain proposal)
   bool march = true;
   int march_nt = 128, march_k = 8;
+  bool shape_auto = true;  // the shape is default_shape's, not asked for
   bool pdl = true;  // programmatic dependent launch of the z-march passes
   bool tmarch = false;  // the z-march with rows staged by bulk copies (unmasked lattices)
   bool amarch = false;  // the z-march with a per-thread cp.async prefetch (unmasked LL / GHRL)
@@ -477,6 +478,39 @@ static void plan_march(mcx_engine *e) {
   }
 }
 
+// The z-march's shape when none is asked for: chunks balanced over one wave of
+// the CTAs the GPU holds (two for unmasked GHRL).  Against 128 x 8 fixed, whose
+// eight planes in a row leave a small lattice's pass at 8 us and up whatever its
+// size, microseconds per pass: LL 48^3 7.5 -> 3.0, 3 x 96^3 13.7 -> 11.2, 4 x
+// 90x92x100 23.5 -> 17.8 (256 threads; 128: 3.1, 12.3, 18.0); GHRL 48^3 7.5 ->
+// 3.4, 8 x 68x62x68 22.2 -> 19.4 (128 threads x 2 waves; 256 x 1: 3.6, 20.6).
+// Masked batches: 128 threads, balanced, up to 300,000 active sites (61^3 droplet
+// 14.3 -> 5.1, 2 slabs of 48^3 7.1 -> 4.5; 128 x 4: 8.3, 5.4).  Above, four
+// planes, so that more units are all bulk or have no active site: 128 threads
+// where most sites are active (6 slabs of 80x76x60 16.8 -> 15.5, 12 of 56x42x42
+// 11.6 -> 11.2; 64 threads 17.1, 11.9), 64 in droplets (8 of 96^3 59.2 -> 51.9, 6
+// of 80^3 29.9 -> 24.9, 3 of 100^3 34.4 -> 28.8; 128 threads 58.4, 26.8, 31.6).
+static void default_shape(mcx_engine *e) {
+  if (tiny_batch(e)) {
+    e->march_nt = 128;
+    e->march_k = 8;
+    return;
+  }
+  long long active = 0, sites = 0;
+  for (const RepDev &R : e->rep) {
+    active += R.valid;
+    sites += (long long)R.nx * R.ny * R.nz;
+  }
+  if (e->var.mask) {
+    const bool small = active <= 300000;
+    e->march_nt = small || 5 * active > 3 * sites ? 128 : 64;
+    e->march_k = small ? 0 : 4;
+  } else {
+    e->march_nt = e->var.pot == POT_GHRL ? 128 : 256;
+    e->march_k = e->var.pot == POT_GHRL ? -2 : 0;
+  }
+}
+
 extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engine **out) {
   if (!out || !descs || n <= 0) return fail(nullptr, MCX_ERR_INVALID, "mcx_create: need n > 0 descriptors and an output pointer");
   *out = nullptr;
@@ -581,8 +615,8 @@ extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engin
   for (int r = 0; r < n; r++) e->rep[r].ns_off = e->var.mask ? e->rep[r].dir_off : -1;
   {
     const char *nt = getenv("MCX_MARCH_NT"), *kk = getenv("MCX_MARCH_K"), *mo = getenv("MCX_MARCH");
-    if (nt && march_block_ok(atoi(nt))) e->march_nt = atoi(nt);
-    if (kk && atoi(kk) > 0) e->march_k = atoi(kk);
+    if (nt && march_block_ok(atoi(nt))) e->march_nt = atoi(nt), e->shape_auto = false;
+    if (kk && atoi(kk) > 0) e->march_k = atoi(kk), e->shape_auto = false;
     if (mo && atoi(mo) == 0) e->march = false;
     const char *pd = getenv("MCX_PDL");
     if (pd && atoi(pd) == 0) e->pdl = false;
@@ -714,7 +748,8 @@ extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engin
     }
   }
   e->defer_plan = false;
-  if (e->var.mask) {
+  if (e->shape_auto) default_shape(e);
+  if (e->var.mask || e->shape_auto) {
     st = apply_march_shape(e, e->march_nt, e->march_k);
     if (st) {
       g_last_error = e->err;
@@ -1290,6 +1325,7 @@ extern "C" mcx_status mcx_set_pass(mcx_engine *e, int kind) {
     return fail(e, MCX_ERR_UNSUPPORTED, "the TMA-staged z-march needs an unmasked batch whose rows fit in shared memory");
   if (kind == MCX_PASS_MARCH_ASYNC && !amarch_prepare(e->var, e->march_nt))
     return fail(e, MCX_ERR_UNSUPPORTED, "the prefetching z-march needs an unmasked LL or GHRL batch");
+  if (kind == MCX_PASS_MARCH_PERSISTENT && e->shape_auto && !pmarch_block_ok(e->march_nt)) e->march_nt = 128;
   if (kind == MCX_PASS_MARCH_PERSISTENT && !pmarch_block_ok(e->march_nt))
     return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march runs blocks of 128 or 256 threads");
   if (kind == MCX_PASS_MARCH_QUAD && !qmarch_ok(e))
@@ -1471,6 +1507,7 @@ extern "C" mcx_status mcx_set_march_shape(mcx_engine *e, int block, int planes) 
     return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march runs blocks of 128 or 256 threads");
   CK(e, cudaStreamSynchronize(e->stream));
   e->resident = false;  // a shape is asked for: the z-march runs it
+  e->shape_auto = false;
   return apply_march_shape(e, block, planes);
 }
 
