@@ -244,7 +244,9 @@ int mcx_get_staged(const mcx_engine *eng);
  *                    in the shared memory of a cluster of 1 to 16 CTAs
  *                    (replicas up to about 40^3; MCX_ERR_UNSUPPORTED
  *                    otherwise).  The default of engines whose replicas are
- *                    small enough that it is estimated faster;
+ *                    small enough that it is estimated faster (and
+ *                    have 1,200 active sites or more, 2,200 where
+ *                    inactive sites have field energy);
  *                    mcx_set_march_shape returns to MCX_PASS_MARCH, which also
  *                    runs the single passes of mcx_pass_timing.
  * No counterpart in the reference. */
@@ -264,7 +266,8 @@ int mcx_get_pass(const mcx_engine *eng);
  * each) and chunk depth (planes per CTA; planes <= 0 cuts near-equal chunks
  * so that the work units fill max(1, -planes) waves of the CTAs the GPU holds
  * at once).  The default is chosen from the batch's potential, masks and size
- * (balanced chunks of 64, 128 or 256 threads). */
+ * (balanced chunks of 128 or 256 threads; four planes in large masked batches;
+ * 128 x 8 where a replica has some hundred active sites). */
 mcx_status mcx_set_march_shape(mcx_engine *eng, int block, int planes);
 /* Autotuner: times the z-march pass (register form and, for unmasked batches,
  * the prefetching and four-site forms) for block sizes {64, 128, 256} and chunk

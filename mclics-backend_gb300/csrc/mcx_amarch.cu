@@ -1,8 +1,7 @@
 // mcx_amarch.cu -- the z-march of the plain proposal with a per-thread
 // cp.async prefetch of the next plane's neighbourhood (k_amarch), and its
 // launchers.  Same work units, Philox counters and pair update as k_march
-// (mcx_march.cu), so the two agree bit for bit except at decisions within an
-// ulp of their threshold (see mcx_march.cu); this form hides each plane's
+// (mcx_march.cu), so the two agree bit for bit; this form hides each plane's
 // load latency behind the arithmetic of the plane before it.
 #include <cuda_runtime.h>
 
