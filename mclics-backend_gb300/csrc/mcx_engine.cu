@@ -331,6 +331,7 @@ static int unit_class(const mcx_engine *e, const int4 &u, int nt) {
       const size_t row = (size_t)jj + (size_t)R.ny * kk;
       seen |= 1u << (tiled ? e->segact[u.x][row * nseg + sc] : act[row]);
     }
+    if (seen & (seen - 1)) return 0;  // rows of two classes
   }
   return seen == 1u ? kUnitDead : (seen == 2u ? (full ? kUnitBulk | kUnitFull : kUnitBulk) : 0);
 }
@@ -1396,29 +1397,60 @@ static int learn_depth(const mcx_engine *e, int nt, int slots) {
   if (tiny_batch(e)) return 8;
   int maxnz = 1;
   for (const RepDev &R : e->rep) maxnz = std::max(maxnz, R.nz);
+  // masked: per replica and block of pairs the live planes before each plane: those
+  // with an active site in the block's rows, the rows next to them or the planes
+  // next to it (a unit is dead when each of its planes is, unit_class)
+  std::vector<std::vector<std::vector<int>>> live(e->var.mask ? e->nrep : 0);
+  for (int r = 0; r < (int)live.size(); r++) {
+    const RepDev &R = e->rep[r];
+    const std::vector<uint8_t> &act = e->rowact[r];
+    std::vector<char> has(R.nz + 2);  // planes -1 .. nz
+    for (int p0 = 0; p0 < R.hp * R.ny; p0 += nt) {
+      const int j0 = p0 / R.hp - 1, j1 = (std::min(p0 + nt, R.hp * R.ny) - 1) / R.hp + 1;
+      for (int k = 0; k < R.nz; k++) {
+        bool on = act.empty();
+        for (int j = j0; j <= j1 && !on; j++)
+          if ((j >= 0 && j < R.ny) || R.yb == BOUND_PERIODIC)
+            on = act[(size_t)((j + R.ny) % R.ny) + (size_t)R.ny * k] != 0;
+        has[k + 1] = on;
+      }
+      has[0] = R.zb == BOUND_PERIODIC ? has[R.nz] : 0;
+      has[R.nz + 1] = R.zb == BOUND_PERIODIC ? has[1] : 0;
+      std::vector<int> n(R.nz + 1, 0);
+      for (int k = 0; k < R.nz; k++) n[k + 1] = n[k] + (has[k] || has[k + 1] || has[k + 2]);
+      live[r].push_back(std::move(n));
+    }
+  }
+  // the units of depth d in launch order
+  auto each = [&](int d, auto &&f) {
+    for (int r = 0; r < e->nrep; r++) {
+      const RepDev &R = e->rep[r];
+      const int blocks = (R.hp * R.ny + nt - 1) / nt, chunks = (R.nz + d - 1) / d;
+      for (int q = 0; q < chunks; q++) {
+        const int k0 = (int)((long long)q * R.nz / chunks), k1 = (int)((long long)(q + 1) * R.nz / chunks);
+        for (int b = 0; b < blocks; b++)
+          if (!e->var.mask || live[r][b][k1] > live[r][b][k0]) f((k1 - k0) + 0.3);
+      }
+    }
+  };
   double best = 1e300;
   int best_d = 1;
   std::vector<double> busy;
   for (int n = 1; n <= std::min(maxnz, 32); n++) {
     const int d = (maxnz + n - 1) / n;
     if (n > 1 && d == (maxnz + n - 2) / (n - 1)) continue;
+    // no schedule beats the work shared out evenly: most depths need no more
+    double work = 0.0, end = 0.0;
+    each(d, [&](double t) { work += t; });
+    if (work / slots >= best) continue;
     // slots as a heap of the times they fall free (the earliest first)
     busy.assign(slots, 0.0);
-    double end = 0.0;
-    for (int r = 0; r < e->nrep; r++) {
-      const RepDev &R = e->rep[r];
-      const int npp = R.hp * R.ny, chunks = (R.nz + d - 1) / d;
-      for (int q = 0; q < chunks; q++) {
-        const int k0 = (int)((long long)q * R.nz / chunks), k1 = (int)((long long)(q + 1) * R.nz / chunks);
-        for (int p0 = 0; p0 < npp; p0 += nt) {
-          if (e->var.mask && unit_class(e, make_int4(r, p0, k0, k1 - k0), nt) == kUnitDead) continue;
-          std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
-          busy.back() += (k1 - k0) + 0.3;
-          end = std::max(end, busy.back());
-          std::push_heap(busy.begin(), busy.end(), std::greater<double>());
-        }
-      }
-    }
+    each(d, [&](double t) {
+      std::pop_heap(busy.begin(), busy.end(), std::greater<double>());
+      busy.back() += t;
+      end = std::max(end, busy.back());
+      std::push_heap(busy.begin(), busy.end(), std::greater<double>());
+    });
     if (end < best) {
       best = end;
       best_d = d;
