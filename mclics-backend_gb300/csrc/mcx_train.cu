@@ -241,12 +241,9 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
   for (int q = 0; q < 8; q++)
 #pragma unroll
     for (int r = 0; r < 4; r++) gW2[q][r] = gWx[q][r] = 0.f;
-  // bias gradients are column sums over the samples: b1 is the gradient of an
-  // input that is always 1 (X column 31, a padding row of W1), b2 and b3 are
-  // products with a tile of ones in accumulators that warps 2 and 3 leave free
-  // (gWx[2..5] b2, gWx[6] b3)
+  float gb = 0.f;   // bias gradient owned by this thread: b1 (tid < 64), b2 (64 <= tid < 128)
+  float gb3 = 0.f;  // b3 entries (tid < 8)
   bool loaded = false;
-  const uint32_t ones[4] = {0x3F803F80u, 0x3F803F80u, 0x3F803F80u, 0x3F803F80u};
   float lsum = 0.f;
   const int nchunk = (a.n + kTS - 1) / kTS;
   for (int ch = blockIdx.x; ch < nchunk; ch += gridDim.x) {
@@ -270,7 +267,6 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
           t.y = u.x;
           t.z = u.y;
           v[0].w = 0.f;
-          v[3].w = 1.f;  // column 31
         } else {
 #pragma unroll
           for (int q = 1; q < 4; q++) v[q] = sp[q];
@@ -467,7 +463,6 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
           uint32_t bf[2];
           ldsm_x2_t(bf, dH2 + (size_t)(s0 + (lane & 15)) * kRowH + nt * 8);
           mma_bf16(gW2[nt], af, bf[0], bf[1]);
-          if (warp >= 2 && (nt >> 2) == warp - 2) mma_bf16(gWx[2 + (nt & 3)], ones, bf[0], bf[1]);
         }
       }
       if (warp < 2) {  // gW1 rows [16 warp, +16) (input features)
@@ -482,7 +477,6 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
       } else {  // gW3 rows [32 (warp-2), +32): two 16-row tiles, one 8-wide output tile
         uint32_t bf[2];
         ldsm_x2_t(bf, dY + (size_t)(s0 + (lane & 15)) * kRowY);
-        mma_bf16(gWx[6], ones, bf[0], bf[1]);
 #pragma unroll
         for (int mt = 0; mt < 2; mt++) {
           uint32_t af[4];
@@ -490,6 +484,16 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
           mma_bf16(gWx[mt], af, bf[0], bf[1]);
         }
       }
+    }
+    // bias gradients: column sums of dH1 (tid < 64), dH2 (64..127), dY (tid < 8),
+    // FP32 additions sample by sample (a tensor-core product with ones gives
+    // other last bits and saves nothing: 2.20 ms per 200 steps either way)
+    const __nv_bfloat16 *dH = tid < 64 ? dH1 + tid : dH2 + tid - 64;
+#pragma unroll 16
+    for (int s2 = 0; s2 < kTS; s2++) gb += __bfloat162float(dH[(size_t)s2 * kRowH]);
+    if (tid < kMlpOut) {
+#pragma unroll 16
+      for (int s2 = 0; s2 < kTS; s2++) gb3 += __bfloat162float(dY[(size_t)s2 * kRowY + tid]);
     }
     __syncthreads();
   }
@@ -503,10 +507,8 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
     put(kPW2 + i0 * kMlpH + o0, gW2[nt][0], gW2[nt][1]);
     put(kPW2 + (i0 + 8) * kMlpH + o0, gW2[nt][2], gW2[nt][3]);
     if (warp < 2) {
-      const bool one = i0 + 8 == kMlpIn - 1;  // the column of ones
       put(kPW1 + i0 * kMlpH + o0, gWx[nt][0], gWx[nt][1]);
-      put(kPW1 + (i0 + 8) * kMlpH + o0, one ? 0.f : gWx[nt][2], one ? 0.f : gWx[nt][3]);
-      if (one) put(kPB1 + o0, gWx[nt][2], gWx[nt][3]);
+      put(kPW1 + (i0 + 8) * kMlpH + o0, gWx[nt][2], gWx[nt][3]);
     }
   }
   if (warp >= 2) {
@@ -516,12 +518,9 @@ __global__ void __launch_bounds__(kTW * 32) k_mlp_grad(GradArgs a) {
       put(kPW3 + i0 * kMlpOut + o0, gWx[mt][0], gWx[mt][1]);
       put(kPW3 + (i0 + 8) * kMlpOut + o0, gWx[mt][2], gWx[mt][3]);
     }
-    if (g == 0) {
-#pragma unroll
-      for (int q = 0; q < 4; q++) put(kPB2 + ((warp - 2) * 4 + q) * 8 + 2 * tg, gWx[2 + q][0], gWx[2 + q][1]);
-      if (warp == 2) put(kPB3 + 2 * tg, gWx[6][0], gWx[6][1]);
-    }
   }
+  part[tid < 64 ? kPB1 + tid : kPB2 + tid - 64] = gb;
+  if (tid < kMlpOut) part[kPB3 + tid] = gb3;
   for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
   __shared__ float s_loss[kTW];
   if (lane == 0) s_loss[warp] = lsum;
@@ -549,7 +548,7 @@ __device__ __forceinline__ void put_image(uint8_t *im, int i, float w) {
   float *bias = reinterpret_cast<float *>(im + kGB);
   if (i < kPB1) {
     const int k = i / kMlpH, n = i % kMlpH;
-    W1t[n * kW1s + k] = k < 19 ? b : __float2bfloat16_rn(0.f);  // inputs 19..30 are zeros, 31 the ones of b1's gradient
+    W1t[n * kW1s + k] = b;
   } else if (i < kPW2) {
     bias[i - kPB1] = w;
   } else if (i < kPB2) {
