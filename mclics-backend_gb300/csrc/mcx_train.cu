@@ -24,8 +24,8 @@
 //
 // What bounds a training step is latency, not work (8192 samples are 128 chunks
 // of 64, one per CTA): weights converted by every CTA from strided FP32 reads,
-// 870,000 atomics on 6,792 addresses, and five launches took 31 us a step.  Two
-// launches, a copied image and partial sums that are read once take 11; the
+// 870,000 atomics on 6,792 addresses, and five launches took 30 us a step.  Two
+// launches, a copied image and partial sums that are read once take 12; the
 // results no longer depend on the order of atomics.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -566,24 +566,30 @@ __device__ __forceinline__ void put_image(uint8_t *im, int i, float w) {
   }
 }
 
-// A CTA sums 32 parameters: warp w the partial rows w, w + 8, ..., then warp 0
-// the eight sums in order.  Adam (Kingma & Ba 2015); the layout's padding
+// A CTA sums 32 parameters: its warps load the partial rows, warp 0 adds them one
+// by one in row order, which is one of the orders that atomic additions of the
+// CTAs' gradients could take (eight sums of every eighth row, added at the end,
+// are none of them, and save 1 us of a step's 12).  Adam (Kingma & Ba 2015); the layout's padding
 // (input rows 19..31 of W1, output columns 4..7 of W3 and b3) stays zero.
-constexpr int kAdamWarps = 8;
+constexpr int kAdamWarps = 8, kAdamRows = 128;  // kAdamRows: rows held at a time
 __global__ void __launch_bounds__(kAdamWarps * 32) k_adam(AdamArgs a) {
-  __shared__ float s_sum[kAdamWarps][32];
+  __shared__ float s_part[kAdamRows][32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, i = blockIdx.x * 32 + lane;
   grid_dependency_wait();
-  float sum = 0.f;
+  float gi = 0.f;
+  for (int r0 = 0; r0 < a.rows; r0 += kAdamRows) {
+    const int n = min(kAdamRows, a.rows - r0);
+    if (r0 > 0) __syncthreads();  // warp 0 has added the rows before
 #pragma unroll 16
-  for (int r = warp; r < a.rows; r += kAdamWarps) sum += __ldcg(a.part + (size_t)r * kPartF + i);
-  s_sum[warp][lane] = sum;
-  __syncthreads();
+    for (int r = warp; r < n; r += kAdamWarps) s_part[r][lane] = __ldcg(a.part + (size_t)(r0 + r) * kPartF + i);
+    __syncthreads();
+    if (warp == 0) {
+#pragma unroll 16
+      for (int r = 0; r < n; r++) gi += s_part[r][lane];
+    }
+  }
   grid_launch_dependents();
   if (warp != 0) return;
-  float gi = 0.f;
-#pragma unroll
-  for (int w = 0; w < kAdamWarps; w += 2) gi += s_sum[w][lane] + s_sum[w + 1][lane];
   if (i == kPTotal && a.loss) *a.loss = gi;
   if (i >= kPTotal) return;
   if (a.grad) a.grad[i] = gi;

@@ -52,6 +52,17 @@ def test_bias_gradients_round_after_every_sample(seed):
         assert np.array_equal(g[b], want)
 
 
+@pytest.mark.parametrize("n", [128, 512, 8192, 16384])
+def test_gradient_adds_its_chunks_in_order(n):
+    """One chunk per CTA (at most 256 of them), added in FP32 one after another."""
+    s = _samples(n, 7)
+    with _engine() as eng:
+        want = np.zeros(mcx.MLP_PARAMS, np.float32)
+        for c in range(0, n, 64):
+            want = want + eng.mlp_grad(s[c:c + 64])[1] * np.float32(64 / n)
+        assert np.array_equal(eng.mlp_grad(s)[1], want)
+
+
 def record(path):
     """Weights after training with batches of at most two chunks, whose sum does
     not depend on which chunk is added first (recorded with atomic additions)."""
