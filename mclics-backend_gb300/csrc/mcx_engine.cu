@@ -16,6 +16,7 @@
 #include <vector>
 
 #include "../../include/mcx.h"
+#include "mcx_alloc.h"
 #include "mcx_device.cuh"
 #include "mcx_host.h"
 #include "mcx_kernels.cuh"
@@ -1793,19 +1794,20 @@ static mcx_status train_prepare(mcx_engine *e) {
   if (e->mlp.empty()) return fail(e, MCX_ERR_INVALID, "set the network weights (mcx_set_mlp) first");
   const size_t wb = sizeof(float) * MCX_MLP_PARAMS;
   if (!e->d_w) {
-    float **bufs[4] = {&e->d_w, &e->d_am, &e->d_av, &e->d_g};
-    for (float **b : bufs) {
-      cudaError_t r = cudaMalloc(b, wb);
-      if (r != cudaSuccess) return fail(e, MCX_ERR_NOMEM, "training buffers: %s", cudaGetErrorString(r));
+    // together, so that a call after a failed one does not find some of them missing
+    const int r = alloc_together({{(void **)&e->d_w, wb}, {(void **)&e->d_am, wb}, {(void **)&e->d_av, wb},
+                                  {(void **)&e->d_g, wb}, {(void **)&e->d_image, (size_t)train_image_bytes()}},
+                                 [](void **p, size_t n) { return cudaMalloc(p, n); }, cudaFree);
+    if (r != 0) {
+      cudaGetLastError();
+      return fail(e, MCX_ERR_NOMEM, "training buffers: %s", cudaGetErrorString((cudaError_t)r));
     }
-    cudaError_t r = cudaMalloc(&e->d_image, train_image_bytes());
-    if (r != cudaSuccess) return fail(e, MCX_ERR_NOMEM, "training buffers: %s", cudaGetErrorString(r));
-    CK(e, cudaMemsetAsync(e->d_image, 0, train_image_bytes(), e->stream));  // its padding stays zero
   }
   if (e->w_stale) {
     CK(e, cudaMemcpyAsync(e->d_w, e->mlp.data(), wb, cudaMemcpyHostToDevice, e->stream));
     CK(e, cudaMemsetAsync(e->d_am, 0, wb, e->stream));
     CK(e, cudaMemsetAsync(e->d_av, 0, wb, e->stream));
+    CK(e, cudaMemsetAsync(e->d_image, 0, train_image_bytes(), e->stream));  // its padding stays zero
     CK(e, launch_adam(nullptr, 0, e->d_w, e->d_am, e->d_av, e->d_image, nullptr, nullptr, 0, 0.f, false, e->stream));
     e->launches++;
     CK(e, cudaStreamSynchronize(e->stream));
