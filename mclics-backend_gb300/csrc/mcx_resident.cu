@@ -15,17 +15,21 @@
 // Halo rows and acceptances travel as asynchronous stores (st.async, red.async)
 // that count their bytes on the receiving CTA's mbarrier, so a CTA waits for
 // its neighbours' rows only and no store is fenced: with a cluster barrier per
-// pass, 30% of a 16^3 pass was the barrier's release fence.  Who may overwrite
-// what:
+// pass, 30% of a 16^3 pass was the barrier's release fence.  mcx_phase.h says
+// which barrier counts what.  Who may overwrite what, and what orders it:
 //   - a CTA's halo rows of colour c are read by its own rows next to them, in
 //     its pass of the other colour, and rewritten by the neighbour's next pass
 //     of colour c.  For c = 1 that pass starts after the neighbour has received
-//     every one of those rows of the pass that reads the halo; for c = 0, after
-//     it has received the acceptances that follow that pass.
-//   - a counter slot is cleared two sweeps before it is added to again, and a
-//     CTA is at most one sweep ahead of another (it needs all acceptances); the
-//     bytes of even and odd sweeps count on barriers of their own, so an early
-//     one cannot complete the phase before it.
+//     the new directors of every pair that read the halo (in a pass of colour 0
+//     only pairs with an active site do, and those are sent); a pair's director
+//     depends on what it read.  For c = 0 it starts after the neighbour has
+//     received every warp's acceptances of that pass, which depend on what the
+//     warp's pairs read: on active pairs' by their decisions, on those of two
+//     inactive sites, which a measured pass of colour 1 reads for their bonds,
+//     by a bit of the energy sum (a fence there cost 1.5 us a sweep).
+//   - nobody clears the acceptance counters: they grow, and a thread subtracts
+//     what it read two sweeps before.  They are added to again after every
+//     warp's acceptances of the next sweep, so after its read.
 // Every wait has a limit, after which the error flag is set and the run ends
 // without waiting any more.
 //
@@ -34,6 +38,7 @@
 #include <cuda_runtime.h>
 
 #include "mcx_march.cuh"
+#include "mcx_phase.h"
 #include "mcx_step.h"
 #include "mcx_tma.cuh"
 
@@ -214,8 +219,8 @@ template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
 __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskThreads : kResThreads, 1) k_resident(PassArgs a, const int *cut, int nsweeps, int C) {
   constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
   extern __shared__ __align__(16) uint8_t res_smem[];
-  __shared__ unsigned s_cnt[3];            // accepted moves of sweeps i, i+1, i+2 (mod 3), every CTA's
-  __shared__ __align__(8) uint64_t bars[4];  // halo rows of colour 0, of colour 1; acceptances of even, odd sweeps
+  __shared__ unsigned s_cnt[2];            // accepted moves of the even and of the odd sweeps, every CTA's
+  __shared__ __align__(8) uint64_t bars[kResBars];  // halo_bar, count_bar (mcx_phase.h)
   __shared__ unsigned s_tx[2];             // pairs that arrive per pass of each colour
   __shared__ __align__(16) RepDev sR;      // the replica's constants: read in every pass
   const int rank = (int)cluster_rank(), r = blockIdx.x / C;
@@ -223,10 +228,10 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
   const int NT = blockDim.x, tid = threadIdx.x, lane = tid & 31;
   for (int i = tid; i < (int)(sizeof(RepDev) / 4); i += NT)
     reinterpret_cast<uint32_t *>(&sR)[i] = reinterpret_cast<const uint32_t *>(a.reps + r)[i];
-  if (tid < 3) s_cnt[tid] = 0;
+  if (tid < 2) s_cnt[tid] = 0;
   if (tid < 2) s_tx[tid] = 0;
   if (tid == 0) {
-    for (int q = 0; q < 4; q++) mbar_init(&bars[q], 1);
+    for (int q = 0; q < kResBars; q++) mbar_init(&bars[q], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncthreads();
@@ -253,7 +258,7 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
   const uint32_t rnext = map_rank(base, next) - 4u * (uint32_t)(n * hs);
   const uint32_t bprev = map_rank(smem_u32(bars), prev), bnext = map_rank(smem_u32(bars), next);
   const uint32_t rcnt = map_rank(smem_u32(s_cnt), lane < C ? lane : 0);
-  const uint32_t rcntb = map_rank(smem_u32(&bars[2]), lane < C ? lane : 0);
+  const uint32_t rcntb = map_rank(smem_u32(bars), lane < C ? lane : 0);
   // both colours of rows r0 - ny .. r0 + n + ny - 1 (zeros where z ends)
   for (int q = 0; q < 6; q++) {
     const float *g = a.dir + R.dir_off + (long long)q * R.plane;
@@ -382,6 +387,7 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
   const float invT = 1.0f / S->T;
   float ang = S->ang_var;
   unsigned long long total = 0;
+  unsigned seen0 = 0, seen1 = 0;  // the counters two sweeps before
   cluster_arrive();
   cluster_wait();
   const uint32_t tx[2] = {24u * s_tx[0], 24u * s_tx[1]}, tx_cnt = 4u * (uint32_t)(NT / 32) * (uint32_t)C;
@@ -401,22 +407,22 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
 #pragma unroll 1
   for (int i = 0; i < nsweeps; i++) {
     const unsigned long long sw = sw0 + (unsigned long long)i;
-    const int slot3 = i % 3;
-    const uint32_t ph = (uint32_t)i & 1u;
-    if (tid == 0) mbar_arrive_expect_tx(&bars[2 + ph], tx_cnt);
+    const uint32_t odd = (uint32_t)i & 1u;
+    if (tid == 0) mbar_arrive_expect_tx(&bars[count_bar(i)], tx_cnt);
     unsigned acc = 0;
     SplitSums<MASK> sums;
     if (MEAS) sums.clear();
 #pragma unroll 1
     for (int c = 0; c < 2; c++) {
-      if (tid == 0) mbar_arrive_expect_tx(&bars[c], tx[c]);
+      if (tid == 0) mbar_arrive_expect_tx(&bars[halo_bar(c, i)], tx[c]);
       float *Dc = D + (size_t)(3 * c) * L.fl;
       const float *Do = D + (size_t)(3 - 3 * c) * L.fl;
       const uint8_t *Pc = PT + (size_t)c * L.pt, *Po = PT + (size_t)(1 - c) * L.pt;
       const uint32_t rc = 4u * (uint32_t)(3 * c * L.fl);
       // the other colour's halo rows (colour 1's of the sweep before were
       // waited for at that sweep's end)
-      if (c == 1 && ok) ok = res_wait(&bars[0], ph);
+      if (c == 1 && ok) ok = res_wait(&bars[halo_bar(0, i)], halo_parity(0, i));
+      const uint32_t hb = 8u * (uint32_t)halo_bar(c, i);
 #pragma unroll 1
       for (int q0 = tid; q0 < count[c]; q0 += NT) {
         const int p = q0 == tid ? first[c] : pair_at(c, q0);
@@ -467,13 +473,13 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
         *reinterpret_cast<float2 *>(Dc + 2 * L.fl + off) = az;
         if (MASK && pself == 0) continue;  // measured only
         if (f & RF_PREV) {
-          const uint32_t t = rprev + rc + 4u * (uint32_t)off, b = bprev + 8u * (uint32_t)c;
+          const uint32_t t = rprev + rc + 4u * (uint32_t)off, b = bprev + hb;
           st_remote(t, ax, b);
           st_remote(t + 4u * (uint32_t)L.fl, ay, b);
           st_remote(t + 8u * (uint32_t)L.fl, az, b);
         }
         if (f & RF_NEXT) {
-          const uint32_t t = rnext + rc + 4u * (uint32_t)off, b = bnext + 8u * (uint32_t)c;
+          const uint32_t t = rnext + rc + 4u * (uint32_t)off, b = bnext + hb;
           st_remote(t, ax, b);
           st_remote(t + 4u * (uint32_t)L.fl, ay, b);
           st_remote(t + 8u * (uint32_t)L.fl, az, b);
@@ -485,9 +491,12 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
       }
     }
     // the sweep's acceptances to every CTA's counter
+    if (MASK && MEAS) {  // never true (no FP32 operation gives this NaN): a dependence on every pair's bonds
+      const float2 e = unpk(sums.hi[0]);
+      acc += (__float_as_uint(e.x) & __float_as_uint(e.y)) == 0xFFFFFFFFu;
+    }
     const unsigned wa = __reduce_add_sync(0xffffffffu, acc);
-    if (lane < C) red_remote(rcnt + 4u * (uint32_t)slot3, wa, rcntb + 8u * ph);
-    if (tid == 0) s_cnt[(i + 2) % 3] = 0;  // read at the end of the sweep before, ahead of this sweep's barrier
+    if (lane < C) red_remote(rcnt + 4u * odd, wa, rcntb + 8u * (uint32_t)count_bar(i));
     if (MEAS) {
       const double v = warp_split_sums(sums);
       double *ring = a.ring + (((size_t)r * (a.ring_cap + 1) +
@@ -499,8 +508,11 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
     }
     rw0 = pair_draw(pid0 + (uint32_t)first[0], 0, sw + 1, seed, stream);
     __syncthreads();  // this CTA's rows of colour 1
-    if (ok) ok = res_wait(&bars[1], ph) && res_wait(&bars[2 + ph], (uint32_t)(i >> 1) & 1u);
-    const unsigned sweep_acc = *(volatile unsigned *)&s_cnt[slot3];
+    if (ok)
+      ok = res_wait(&bars[halo_bar(1, i)], halo_parity(1, i)) && res_wait(&bars[count_bar(i)], count_parity(i));
+    const unsigned sum = *(volatile unsigned *)&s_cnt[odd], sweep_acc = sum - (odd ? seen1 : seen0);
+    if (odd) seen1 = sum;
+    else seen0 = sum;
     total += sweep_acc;
     if (!frozen) ang = next_step(ang, sweep_acc, (unsigned)R.valid);
   }
