@@ -380,11 +380,12 @@ mcx_status mcx_pass_timing(mcx_engine *eng, int n_sweeps, float *pass_ms, float 
  * duration in the production launch sequence, launch gaps included.  The
  * sweeps are real (state, RNG counter and step size advance). */
 mcx_status mcx_sweep_timing(mcx_engine *eng, int n_sweeps, float *ms);
-/* Test of the persistent z-march's bounded grid-barrier wait: one launch
- * whose barriers cannot complete.  Every CTA gives up after its poll limit
- * (about a second), sets the error flag and leaves; returns MCX_ERR_CUDA with
- * the barrier message (MCX_ERR_INVALID when that pass kind is not selected).
- * The engine's directors are left mid-sweep. */
+/* Test of the bounded waits of the persistent z-march and of the resident
+ * form: one launch whose barriers cannot complete.  Every CTA gives up after
+ * its limit (about a second; two milliseconds in the resident form's test),
+ * sets the error flag and leaves; returns MCX_ERR_CUDA with the form's message
+ * (MCX_ERR_INVALID when neither is selected).  The persistent form leaves the
+ * engine's directors mid-sweep, the resident form as they were. */
 mcx_status mcx_debug_barrier_timeout(mcx_engine *eng);
 
 /* Host-only helpers (no GPU needed). */

@@ -1321,7 +1321,7 @@ static mcx_status check_err_flag(mcx_engine *e, int r = 0, double *stats = nullp
     if (f & 2u)
       return fail(e, MCX_ERR_CUDA, "persistent z-march: a grid barrier was not reached in time; results are invalid");
     if (f & 8u)
-      return fail(e, MCX_ERR_CUDA, "resident sweeps: a neighbouring CTA's rows did not arrive in time; results are invalid");
+      return fail(e, MCX_ERR_CUDA, "resident sweeps: a neighbouring CTA's rows did not arrive in time; the replica kept its state, its sums are invalid");
     if (f & 4u)
       return fail(e, MCX_ERR_CUDA, "tensor-core network: an MMA did not complete in time; results are invalid");
     return fail(e, MCX_ERR_CUDA, "staged pass: a shared-memory tile copy did not complete in time; results are invalid");
@@ -2267,9 +2267,14 @@ extern "C" mcx_status mcx_combine_stats(mcx_engine *e, int n, const int *replica
 
 extern "C" mcx_status mcx_debug_barrier_timeout(mcx_engine *e) {
   if (!e) return fail(nullptr, MCX_ERR_INVALID, "null engine");
-  if (!persistent(e)) return fail(e, MCX_ERR_INVALID, "the persistent z-march is not selected");
+  if (!persistent(e) && !use_resident(e))
+    return fail(e, MCX_ERR_INVALID, "neither the persistent z-march nor the resident form is selected");
   PassArgs pa = pass_args(e);
-  CK(e, launch_pmarch(e->var, MODE_SWEEP, pa, e->march_nt, 1, e->d_err + 1, e->stream, 1u));
+  if (use_resident(e)) {
+    const mcx_engine::ResPlan &r = e->res[0];
+    CK(e, launch_resident(e->var, MODE_SWEEP, pa, r.d_cut, e->nrep, 3, r.c, r.nt, r.smem, e->stream, 2000000ull, 4u));
+  } else
+    CK(e, launch_pmarch(e->var, MODE_SWEEP, pa, e->march_nt, 1, e->d_err + 1, e->stream, 1u));
   e->launches += 1;
   CK(e, cudaStreamSynchronize(e->stream));
   return check_err_flag(e);

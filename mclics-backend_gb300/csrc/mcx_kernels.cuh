@@ -148,8 +148,12 @@ long long resident_smem_bytes(const RepDev &R, bool mask, int n);
 int resident_max_threads(bool mask, int mode);
 constexpr int kResidentSmem = 220 * 1024;  // dynamic shared memory of a CTA, below the 227 KB limit
 int resident_clusters(const Variant &v, int mode, int C, int nt, int smem);
+// limit: nanoseconds a wait may take; extra: bytes that each sweep waits for in
+// vain (a test of the limit).
+constexpr unsigned long long kResidentLimit = 1000000000ull;
 cudaError_t launch_resident(const Variant &v, int mode, const PassArgs &a, const int *cut, int nrep, int nsweeps,
-                            int C, int nt, int smem, cudaStream_t st);
+                            int C, int nt, int smem, cudaStream_t st, unsigned long long limit = kResidentLimit,
+                            unsigned extra = 0);
 // The learned-proposal z-march (mcx_lmarch.cu): units of lmarch_block_threads()
 // pairs; lmarch_prepare sets its shared memory and checks residency.  tc: the
 // network on the tcgen05 tensor cores (else the warp-level mma.sync code).

@@ -30,8 +30,12 @@
 //   - nobody clears the acceptance counters: they grow, and a thread subtracts
 //     what it read two sweeps before.  They are added to again after every
 //     warp's acceptances of the next sweep, so after its read.
-// Every wait has a limit, after which the error flag is set and the run ends
-// without waiting any more.
+// Every wait has a limit in time.  A CTA one of whose waits ran out leaves the
+// run at the end of that sweep; the others, which then miss its acceptances, in
+// the next.  They tell each other at the cluster barrier after the run, after
+// which nobody sends: then all wait for a millisecond, so that no row or count on
+// its way (a microsecond at most) meets a CTA that has ended, set the error flag
+// and leave the replica as it was before the run.
 //
 // Same Philox counters and pair update as k_march (mcx_march.cuh), so the chain
 // is the same bit for bit.
@@ -197,30 +201,51 @@ __device__ __forceinline__ void red_remote(uint32_t addr, unsigned v, uint32_t b
                "r"(v), "r"(bar)
                : "memory");
 }
-// Waits for a phase of a barrier that other CTAs complete; false when the
-// limit is reached (about a second).
-__device__ __forceinline__ bool res_wait(uint64_t *bar, uint32_t parity) {
+__device__ __forceinline__ void set_remote(uint32_t addr, unsigned v) {
+  asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long now_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+__device__ __forceinline__ bool res_try(uint32_t b, uint32_t parity) {
+  uint32_t done;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(done)
+      : "r"(b), "r"(parity)
+      : "memory");
+  return done != 0;
+}
+// Waits for a phase of a barrier that other CTAs complete; false when `limit`
+// nanoseconds (or some seconds of polls, should the timer not run) are over.
+__device__ __forceinline__ bool res_wait(uint64_t *bar, uint32_t parity, unsigned long long limit) {
   const uint32_t b = smem_u32(bar);
-  for (unsigned i = 0; i < (1u << 20); i++) {
-    uint32_t done;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\t"
-        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
-        "selp.u32 %0, 1, 0, p;\n\t}"
-        : "=r"(done)
-        : "r"(b), "r"(parity)
-        : "memory");
-    if (done) return true;
+  if (res_try(b, parity)) return true;
+  const unsigned long long t0 = now_ns();
+  for (unsigned i = 0; i < (1u << 25); i++) {
+    if (res_try(b, parity)) return true;
+    if (now_ns() - t0 > limit) return false;
   }
   return false;
 }
+// After a run that was given up: rows and counts on their way land.
+__device__ __forceinline__ void let_land() {
+  const unsigned long long t0 = now_ns();
+  for (unsigned i = 0; i < (1u << 20) && now_ns() - t0 < 1000000ull; i++) __nanosleep(1000);
+}
 
 template <int POT, bool MASK, bool FIELD, int MODE, bool PER>
-__global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskThreads : kResThreads, 1) k_resident(PassArgs a, const int *cut, int nsweeps, int C) {
+__global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskThreads : kResThreads, 1)
+    k_resident(PassArgs a, const int *cut, int nsweeps, int C, unsigned long long limit, unsigned extra) {
   constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE;
   extern __shared__ __align__(16) uint8_t res_smem[];
   __shared__ unsigned s_cnt[2];            // accepted moves of the even and of the odd sweeps, every CTA's
   __shared__ __align__(8) uint64_t bars[kResBars];  // halo_bar, count_bar (mcx_phase.h)
+  __shared__ unsigned s_bad;               // a CTA of the cluster gave up
   __shared__ unsigned s_tx[2];             // pairs that arrive per pass of each colour
   __shared__ __align__(16) RepDev sR;      // the replica's constants: read in every pass
   const int rank = (int)cluster_rank(), r = blockIdx.x / C;
@@ -229,6 +254,7 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
   for (int i = tid; i < (int)(sizeof(RepDev) / 4); i += NT)
     reinterpret_cast<uint32_t *>(&sR)[i] = reinterpret_cast<const uint32_t *>(a.reps + r)[i];
   if (tid < 2) s_cnt[tid] = 0;
+  if (tid == 0) s_bad = 0;
   if (tid < 2) s_tx[tid] = 0;
   if (tid == 0) {
     for (int q = 0; q < kResBars; q++) mbar_init(&bars[q], 1);
@@ -390,8 +416,8 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
   unsigned seen0 = 0, seen1 = 0;  // the counters two sweeps before
   cluster_arrive();
   cluster_wait();
-  const uint32_t tx[2] = {24u * s_tx[0], 24u * s_tx[1]}, tx_cnt = 4u * (uint32_t)(NT / 32) * (uint32_t)C;
-  bool ok = true;  // false: a wait ran out
+  const uint32_t tx[2] = {24u * s_tx[0], 24u * s_tx[1]}, tx_cnt = 4u * (uint32_t)(NT / 32) * (uint32_t)C + extra;
+  bool ok = true, gave_up = false;  // whether a wait of this thread, of any thread of the CTA ran out
   // the thread's first pair of each colour: its draw is made before the waits.
   // Masked: indices below nb32 are bulk pairs, so that a warp runs one kind
   const int nb32[2] = {(nb[0] + 31) & ~31, (nb[1] + 31) & ~31};
@@ -421,7 +447,7 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
       const uint32_t rc = 4u * (uint32_t)(3 * c * L.fl);
       // the other colour's halo rows (colour 1's of the sweep before were
       // waited for at that sweep's end)
-      if (c == 1 && ok) ok = res_wait(&bars[halo_bar(0, i)], halo_parity(0, i));
+      if (c == 1 && ok) ok = res_wait(&bars[halo_bar(0, i)], halo_parity(0, i), limit);
       const uint32_t hb = 8u * (uint32_t)halo_bar(c, i);
 #pragma unroll 1
       for (int q0 = tid; q0 < count[c]; q0 += NT) {
@@ -507,18 +533,31 @@ __global__ void __launch_bounds__(MASK && MODE == MODE_SWEEP_MEASURE ? kResMaskT
       if (!MASK && lane == 1) atomicAdd(ring + 1, v);  // lane 1 holds lane 0's: with every site active, E of active sites is E
     }
     rw0 = pair_draw(pid0 + (uint32_t)first[0], 0, sw + 1, seed, stream);
-    __syncthreads();  // this CTA's rows of colour 1
-    if (ok)
-      ok = res_wait(&bars[halo_bar(1, i)], halo_parity(1, i)) && res_wait(&bars[count_bar(i)], count_parity(i));
+    // this CTA's rows of colour 1, and whether a wait ran out since this barrier of the sweep before
+    if (__syncthreads_or(!ok)) {
+      gave_up = true;
+      break;
+    }
+    ok = res_wait(&bars[halo_bar(1, i)], halo_parity(1, i), limit) &&
+         res_wait(&bars[count_bar(i)], count_parity(i), limit);
     const unsigned sum = *(volatile unsigned *)&s_cnt[odd], sweep_acc = sum - (odd ? seen1 : seen0);
     if (odd) seen1 = sum;
     else seen0 = sum;
     total += sweep_acc;
     if (!frozen) ang = next_step(ang, sweep_acc, (unsigned)R.valid);
   }
-  if (!ok) atomicOr(a.err, 8u);
-  cluster_arrive();  // every store to this CTA has landed: it may end
+  gave_up = __syncthreads_or(gave_up || !ok);
+  if (gave_up && tid < C) set_remote(map_rank(smem_u32(&s_bad), tid), 1u);
+  cluster_arrive();  // nobody sends any more, and unless one gave up every store to this CTA has landed: it may end
   cluster_wait();
+  if (*(volatile unsigned *)&s_bad) {
+    let_land();
+    cluster_arrive();
+    cluster_wait();
+    if (tid == 0) atomicOr(a.err, 8u);
+    if (MEAS && rank == 0 && tid == 0) S->meas = meas0 + (unsigned long long)nsweeps;  // the ring's slots are counted on the host too
+    return;
+  }
   // directors back (own rows), and the replica's state
   for (int q = 0; q < 6; q++) {
     float *g = a.dir + R.dir_off + (long long)q * R.plane + (long long)r0 * hs;
@@ -599,11 +638,11 @@ int resident_clusters(const Variant &v, int mode, int C, int nt, int smem) {
 }
 
 cudaError_t launch_resident(const Variant &v, int mode, const PassArgs &a, const int *cut, int nrep, int nsweeps,
-                            int C, int nt, int smem, cudaStream_t st) {
+                            int C, int nt, int smem, cudaStream_t st, unsigned long long limit, unsigned extra) {
   PassArgs args = a;
   int ns = nsweeps, cc = C;
   const int *ct = cut;
-  void *params[] = {&args, &ct, &ns, &cc};
+  void *params[] = {&args, &ct, &ns, &cc, &limit, &extra};
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at;
   res_config(cfg, at, nrep, C, nt, smem, st);
