@@ -80,6 +80,8 @@ struct mcx_engine {
   bool march = true;
   int march_nt = 128, march_k = 8;
   bool shape_auto = true;  // the shape is default_shape's, not asked for
+  bool form_auto = true;   // so is the form (choose_form)
+  bool stale = false;      // masks were set since the form, the resident cuts and the learned units were planned
   bool pdl = true;  // programmatic dependent launch of the z-march passes
   bool tmarch = false;  // the z-march with rows staged by bulk copies (unmasked lattices)
   bool amarch = false;  // the z-march with a per-thread cp.async prefetch (unmasked LL / GHRL)
@@ -130,8 +132,8 @@ static PassArgs pass_args(mcx_engine *e);
 static bool use_tmarch(mcx_engine *e, bool on);
 static bool qmarch_ok(const mcx_engine *e);
 static mcx_status apply_march_shape(mcx_engine *e, int nt, int k);
-static double plan_resident(mcx_engine *e);
-static double march_estimate(const mcx_engine *e);
+static void choose_form(mcx_engine *e);
+static mcx_status plan_lmarch(mcx_engine *e);
 
 static mcx_status fail(mcx_engine *e, mcx_status st, const char *fmt, ...) {
   char buf[512];
@@ -343,14 +345,9 @@ static int unit_pairs(const mcx_engine *e) { return e->qmarch ? 2 * e->march_nt 
 
 static bool unit_dead(const mcx_engine *e, const int4 &u) { return unit_class(e, u, unit_pairs(e)) == kUnitDead; }
 
-// Flags of the z-march units and of the learned z-march's units (which only
-// use kUnitDead).
+// Flags of the z-march units.
 static void mark_dead_units(mcx_engine *e) {
   for (int4 &u : e->units) u.w = (u.w & (kUnitPlanes | kUnitTiled)) | unit_class(e, u, unit_pairs(e));
-  for (int4 &u : e->lunits) {
-    const int cls = unit_class(e, u, lmarch_block_threads());
-    u.w = (u.w & kUnitPlanes) | (cls == kUnitDead ? kUnitDead : 0);
-  }
 }
 
 // Plane runs of a replica for the z-march's chunks: maximal runs of planes k
@@ -517,6 +514,12 @@ static void default_shape(mcx_engine *e) {
     e->march_nt = e->var.pot == POT_GHRL ? 128 : 256;
     e->march_k = e->var.pot == POT_GHRL ? -2 : 0;
   }
+}
+
+// The z-march's units for the engine's present masks.
+static mcx_status replan_march(mcx_engine *e) {
+  if (e->shape_auto && !e->pmarch) default_shape(e);
+  return apply_march_shape(e, e->march_nt, e->march_k);
 }
 
 extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engine **out) {
@@ -757,20 +760,16 @@ extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engin
     }
   }
   e->defer_plan = false;
-  if (e->shape_auto) default_shape(e);
   if (e->var.mask || e->shape_auto) {
-    st = apply_march_shape(e, e->march_nt, e->march_k);
+    st = replan_march(e);
     if (st) {
       g_last_error = e->err;
       free_engine(e);
       return st;
     }
   }
-  // small lattices: resident where that is estimated faster than the z-march
-  if (e->march && !e->staged) {
-    const double t = plan_resident(e);
-    e->resident = t > 0.0 && t < march_estimate(e) && !tiny_batch(e);
-  }
+  choose_form(e);
+  e->stale = false;
   CKC(cudaStreamSynchronize(e->stream));
 #undef CKC
   *out = e;
@@ -911,16 +910,15 @@ extern "C" mcx_status mcx_set_mask(mcx_engine *e, int r, const int *pt, const fl
         }
     }
   }
-  // the z-march's chunks follow the mask's plane runs: plan them again (in
-  // mcx_create and mcx_load once, after every replica's mask)
+  // the z-march's shape and chunks follow the mask: plan them again (in
+  // mcx_create and mcx_load once, after every replica's mask); what only runs of
+  // sweeps need, before the next one (settle)
   if (e->defer_plan) {
     mark_dead_units(e);
-  } else if (mcx_status st = apply_march_shape(e, e->march_nt, e->march_k)) {
+  } else if (mcx_status st = replan_march(e)) {
     return st;
   }
-  if (e->d_lunits && !e->lunits.empty())
-    CK(e, cudaMemcpyAsync(e->d_lunits, e->lunits.data(), sizeof(int4) * e->lunits.size(), cudaMemcpyHostToDevice,
-                          e->stream));
+  e->stale = true;
   drop_graphs(e);
   CK(e, cudaStreamSynchronize(e->stream));
   return MCX_OK;
@@ -1227,6 +1225,27 @@ static double plan_resident(mcx_engine *e) {
   return best[0];
 }
 
+// The form when none is asked for: resident where that is estimated faster than
+// the z-march.  A form that was asked for stays, with cuts for the present masks.
+static void choose_form(mcx_engine *e) {
+  if (!e->march || e->staged || !(e->form_auto || e->resident)) return;
+  const double t = plan_resident(e);
+  e->resident = t > 0.0 && (!e->form_auto || (t < march_estimate(e) && !tiny_batch(e)));
+}
+
+// Plans again what depends on masks that were set since.
+static mcx_status settle(mcx_engine *e) {
+  if (!e->stale) return MCX_OK;
+  CK(e, cudaStreamSynchronize(e->stream));
+  choose_form(e);
+  if (e->d_lunits) {
+    drop_graphs(e);
+    if (mcx_status st = plan_lmarch(e)) return st;
+  }
+  e->stale = false;
+  return MCX_OK;
+}
+
 // Whether k_idle_field adds the inactive sites' field energy for a run of
 // sweeps: the z-march (plain or learned) and resident sweeps of a masked batch.
 static bool idle_field(const mcx_engine *e) {
@@ -1235,6 +1254,7 @@ static bool idle_field(const mcx_engine *e) {
 }
 
 static mcx_status run_sweeps(mcx_engine *e, int n, int m) {
+  if (mcx_status st = settle(e)) return st;
   if (m && n > 0 && idle_field(e)) {
     int plane = 0;
     for (const RepDev &R : e->rep) plane = std::max(plane, R.plane);
@@ -1352,6 +1372,7 @@ extern "C" mcx_status mcx_set_pass(mcx_engine *e, int kind) {
     return fail(e, MCX_ERR_UNSUPPORTED, "the four-site z-march needs an unmasked batch with nx a multiple of 8");
   if (kind == MCX_PASS_RESIDENT && plan_resident(e) == 0.0)
     return fail(e, MCX_ERR_UNSUPPORTED, "the resident form needs every replica to fit the shared memory of one cluster");
+  e->form_auto = false;
   if (kind != MCX_PASS_MARCH_TMA) e->tmarch = false;
   e->resident = kind == MCX_PASS_RESIDENT;
   e->amarch = kind == MCX_PASS_MARCH_ASYNC;
@@ -1377,6 +1398,7 @@ extern "C" int mcx_get_pass(const mcx_engine *e) {
   if (!e) return -1;
   if (e->staged) return MCX_PASS_STAGED;
   if (!e->march) return MCX_PASS_DIRECT;
+  if (e->stale) settle(const_cast<mcx_engine *>(e));
   if (e->resident) return MCX_PASS_RESIDENT;
   if (e->pmarch) return MCX_PASS_MARCH_PERSISTENT;
   if (e->qmarch) return MCX_PASS_MARCH_QUAD;
@@ -1464,30 +1486,38 @@ static int learn_depth(const mcx_engine *e, int nt, int slots) {
 // of a plane's pairs times chunks of near-equal depth (learn_depth); uploads
 // them and the replicas' CTA counts.
 static mcx_status plan_lmarch(mcx_engine *e) {
-  e->lunits.clear();
   const int nt = lmarch_block_threads();
   int dev = 0, nsm = 0;
   CK(e, cudaGetDevice(&dev));
   CK(e, cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
   const int d = learn_depth(e, nt, std::max(1, nsm * lmarch_blocks_per_sm(e->var, e->ltc)));
+  std::vector<int4> units;
+  std::vector<int> ctas(e->nrep, 0);
   for (int r = 0; r < e->nrep; r++) {
-    RepDev &R = e->rep[r];
+    const RepDev &R = e->rep[r];
     const int npp = R.hp * R.ny, chunks = (R.nz + d - 1) / d;
     const bool tiny = tiny_batch(e);  // whole depths, the rest last
-    R.lcta = 0;
     for (int q = 0; q < chunks; q++) {
       const int k0 = tiny ? q * d : (int)((long long)q * R.nz / chunks);
       const int k1 = tiny ? std::min(R.nz, k0 + d) : (int)((long long)(q + 1) * R.nz / chunks);
       for (int p0 = 0; p0 < npp; p0 += nt) {
-        e->lunits.push_back(make_int4(r, p0, k0, k1 - k0));
-        R.lcta++;
+        units.push_back(make_int4(r, p0, k0, k1 - k0));
+        ctas[r]++;
       }
     }
   }
-  for (int4 &u : e->lunits) u.w |= unit_class(e, u, nt) == kUnitDead ? kUnitDead : 0;
-  cudaFree(e->d_lunits);
-  e->d_lunits = nullptr;
-  CK(e, cudaMalloc(&e->d_lunits, sizeof(int4) * e->lunits.size()));
+  for (int4 &u : units) u.w |= unit_class(e, u, nt) == kUnitDead ? kUnitDead : 0;
+  if (units.size() > e->lunits.size() || !e->d_lunits) {  // the old units stay where there is no room for new ones
+    int4 *d_new = nullptr;
+    if (cudaMalloc(&d_new, sizeof(int4) * units.size()) != cudaSuccess) {
+      cudaGetLastError();
+      return fail(e, MCX_ERR_NOMEM, "learned z-march units");
+    }
+    cudaFree(e->d_lunits);
+    e->d_lunits = d_new;
+  }
+  e->lunits.swap(units);
+  for (int r = 0; r < e->nrep; r++) e->rep[r].lcta = ctas[r];
   CK(e, cudaMemcpyAsync(e->d_lunits, e->lunits.data(), sizeof(int4) * e->lunits.size(), cudaMemcpyHostToDevice,
                         e->stream));
   CK(e, cudaMemcpyAsync(e->d_rep, e->rep.data(), sizeof(RepDev) * e->nrep, cudaMemcpyHostToDevice, e->stream));
@@ -1558,7 +1588,7 @@ extern "C" mcx_status mcx_set_march_shape(mcx_engine *e, int block, int planes) 
     return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march runs blocks of 128 or 256 threads");
   CK(e, cudaStreamSynchronize(e->stream));
   e->resident = false;  // a shape is asked for: the z-march runs it
-  e->shape_auto = false;
+  e->shape_auto = e->form_auto = false;
   return apply_march_shape(e, block, planes);
 }
 
@@ -1677,6 +1707,7 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
       }
     }
   }
+  e->shape_auto = e->form_auto = false;
   e->resident = best_form == 5;
   e->tmarch = best_form == 1;
   e->amarch = best_form == 2;
@@ -1751,9 +1782,10 @@ static mcx_status upload_mlp(mcx_engine *e, const float *w) {
     // the warp-level network is the default: measured faster inside the
     // learned z-march (LL 96^3 x 128: 3.43 against 3.87 ms per pass)
     e->ltc = lp && atoi(lp) == MCX_MLP_TCGEN05 && lmarch_prepare(e->var, true);
-    e->lmarch_ok = !(lm && atoi(lm) == 0) && lmarch_prepare(e->var, e->ltc);
-    if (e->lmarch_ok)
+    if (!(lm && atoi(lm) == 0) && lmarch_prepare(e->var, e->ltc)) {
       if (mcx_status st = plan_lmarch(e)) return st;
+      e->lmarch_ok = true;
+    }
   }
   CK(e, cudaMemcpy(e->d_mlp, packed.data(), packed.size(), cudaMemcpyHostToDevice));
   return MCX_OK;
@@ -1899,7 +1931,7 @@ extern "C" mcx_status mcx_set_mlp_path(mcx_engine *e, int path) {
   e->ltc = path == MCX_MLP_TCGEN05;
   if (!lmarch_prepare(e->var, e->ltc)) return fail(e, MCX_ERR_CUDA, "mcx_set_mlp_path: learned z-march set-up failed");
   drop_graphs(e);
-  return MCX_OK;
+  return plan_lmarch(e);  // the two forms hold different numbers of CTAs at once
 }
 
 extern "C" int mcx_get_mlp_path(const mcx_engine *e) { return e && e->ltc ? MCX_MLP_TCGEN05 : MCX_MLP_WARP_MMA; }
@@ -2132,7 +2164,7 @@ extern "C" mcx_status mcx_load(mcx_engine *e, const char *path) {
     }
   e->defer_plan = false;
   if (e->var.mask)
-    if (mcx_status s2 = apply_march_shape(e, e->march_nt, e->march_k)) return s2;
+    if (mcx_status s2 = replan_march(e)) return s2;
   for (int r = 0; r < n; r++) {
     if (mcx_status s2 = mcx_set_state(e, r, ni[r].data())) return s2;
     st[r].T = cs[r].T;
@@ -2267,6 +2299,7 @@ extern "C" mcx_status mcx_combine_stats(mcx_engine *e, int n, const int *replica
 
 extern "C" mcx_status mcx_debug_barrier_timeout(mcx_engine *e) {
   if (!e) return fail(nullptr, MCX_ERR_INVALID, "null engine");
+  if (mcx_status st = settle(e)) return st;
   if (!persistent(e) && !use_resident(e))
     return fail(e, MCX_ERR_INVALID, "neither the persistent z-march nor the resident form is selected");
   PassArgs pa = pass_args(e);
@@ -2356,6 +2389,7 @@ extern "C" void *mcx_stream(mcx_engine *e) { return e ? (void *)e->stream : null
 extern "C" mcx_status mcx_sweep_timing(mcx_engine *e, int n, float *ms) {
   if (!e) return fail(nullptr, MCX_ERR_INVALID, "null engine");
   if (n <= 0 || !ms) return fail(e, MCX_ERR_INVALID, "need n_sweeps > 0 and an output");
+  if (mcx_status st = settle(e)) return st;
   cudaEvent_t a, b;
   CK(e, cudaEventCreate(&a));
   CK(e, cudaEventCreate(&b));
@@ -2376,6 +2410,7 @@ extern "C" mcx_status mcx_sweep_timing(mcx_engine *e, int n, float *ms) {
 extern "C" mcx_status mcx_pass_timing(mcx_engine *e, int n, float *pass_ms, float *total_ms) {
   if (!e) return fail(nullptr, MCX_ERR_INVALID, "null engine");
   if (n <= 0) return fail(e, MCX_ERR_INVALID, "need n_sweeps > 0");
+  if (mcx_status st = settle(e)) return st;
   std::vector<cudaEvent_t> ev(4 * (size_t)n);
   for (auto &x : ev) CK(e, cudaEventCreate(&x));
   PassArgs pa = pass_args(e);
