@@ -1365,13 +1365,16 @@ extern "C" mcx_status mcx_set_pass(mcx_engine *e, int kind) {
     return fail(e, MCX_ERR_UNSUPPORTED, "the TMA-staged z-march needs an unmasked batch whose rows fit in shared memory");
   if (kind == MCX_PASS_MARCH_ASYNC && !amarch_prepare(e->var, e->march_nt))
     return fail(e, MCX_ERR_UNSUPPORTED, "the prefetching z-march needs an unmasked LL or GHRL batch");
-  if (kind == MCX_PASS_MARCH_PERSISTENT && e->shape_auto && !pmarch_block_ok(e->march_nt)) e->march_nt = 128;
-  if (kind == MCX_PASS_MARCH_PERSISTENT && !pmarch_block_ok(e->march_nt))
+  if (kind == MCX_PASS_MARCH_PERSISTENT && !pmarch_block_ok(e->march_nt) && !e->shape_auto)
     return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march runs blocks of 128 or 256 threads");
   if (kind == MCX_PASS_MARCH_QUAD && !qmarch_ok(e))
     return fail(e, MCX_ERR_UNSUPPORTED, "the four-site z-march needs an unmasked batch with nx a multiple of 8");
-  if (kind == MCX_PASS_RESIDENT && plan_resident(e) == 0.0)
+  if (kind == MCX_PASS_RESIDENT && plan_resident(e) == 0.0) {
+    e->resident = false;  // an engine that ran it has no cuts now
     return fail(e, MCX_ERR_UNSUPPORTED, "the resident form needs every replica to fit the shared memory of one cluster");
+  }
+  const bool was[] = {e->form_auto, e->resident, e->tmarch, e->amarch, e->qmarch, e->staged, e->march};
+  const int was_nt = e->march_nt;
   e->form_auto = false;
   if (kind != MCX_PASS_MARCH_TMA) e->tmarch = false;
   e->resident = kind == MCX_PASS_RESIDENT;
@@ -1382,10 +1385,15 @@ extern "C" mcx_status mcx_set_pass(mcx_engine *e, int kind) {
   e->march = kind == MCX_PASS_MARCH || kind == MCX_PASS_MARCH_TMA || kind == MCX_PASS_MARCH_ASYNC ||
              kind == MCX_PASS_MARCH_PERSISTENT || kind == MCX_PASS_MARCH_QUAD || kind == MCX_PASS_RESIDENT;
   if (e->march) {
-    if (mcx_status st = apply_march_shape(e, e->march_nt, e->march_k)) return st;  // chunks follow the form's residency
-    if (e->pmarch && !pmarch_fits(e)) {
+    // chunks follow the form's residency; a shape that nobody asked for is one of
+    // the persistent form's there, and the default again after it
+    if (e->pmarch && e->shape_auto && !pmarch_block_ok(e->march_nt)) e->march_nt = 128;
+    if (mcx_status st = replan_march(e)) return st;
+    if (e->pmarch && !pmarch_fits(e)) {  // refused: the form and shape of before
       e->pmarch = false;
-      apply_march_shape(e, e->march_nt, e->march_k);
+      e->form_auto = was[0], e->resident = was[1], e->tmarch = was[2], e->amarch = was[3], e->qmarch = was[4];
+      e->staged = was[5], e->march = was[6];
+      apply_march_shape(e, was_nt, e->march_k);
       return fail(e, MCX_ERR_UNSUPPORTED, "the persistent z-march needs every work unit resident at once; this batch has more column blocks than the GPU holds CTAs");
     }
     return MCX_OK;
