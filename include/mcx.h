@@ -207,10 +207,10 @@ long long mcx_kernel_launches(const mcx_engine *eng);
 
 /* Chooses the sweep kernel: on != 0 the staged pass (tiles of rows brought
  * into shared memory by TMA bulk copies, double-buffered, persistent CTAs),
- * 0 the direct pass (each thread loads its neighbours from global memory).
- * The direct pass is the default (it measures faster on the lattices
- * benchmarked so far); the staged pass needs every replica's tile to fit in
- * shared memory.  Both compute the same update (see mcx_set_pass). */
+ * 0 the form the engine would run by default (mcx_set_pass), or the z-march
+ * where another pass or a z-march shape was asked for.  The staged pass needs
+ * every replica's tile to fit in shared memory.  Both compute the same update
+ * (see mcx_set_pass). */
 mcx_status mcx_set_staged(mcx_engine *eng, int on);
 int mcx_get_staged(const mcx_engine *eng);
 
@@ -221,9 +221,9 @@ int mcx_get_staged(const mcx_engine *eng);
  * summation order): the autotuner's choice changes the speed, never the
  * trajectory.
  *
- *   MCX_PASS_MARCH   the default of larger lattices: a CTA marches a block of same-colour site
- *                    pairs of one z-plane through a chunk of planes, keeping
- *                    the z neighbours in registers;
+ *   MCX_PASS_MARCH   the default of larger lattices: a CTA marches a block of
+ *                    same-colour site pairs of one z-plane through a chunk of
+ *                    planes, keeping the z neighbours in registers;
  *   MCX_PASS_DIRECT  persistent CTAs, each pair's neighbourhood loaded by
  *                    cp.async into shared memory;
  *   MCX_PASS_STAGED  the staged TMA pass above (mcx_set_staged);

@@ -1414,7 +1414,13 @@ extern "C" int mcx_get_pass(const mcx_engine *e) {
 }
 
 extern "C" mcx_status mcx_set_staged(mcx_engine *e, int on) {
-  return mcx_set_pass(e, on ? MCX_PASS_STAGED : MCX_PASS_MARCH);
+  if (!e) return fail(nullptr, MCX_ERR_INVALID, "null engine");
+  const bool own = e->form_auto;  // a form that nobody asked for is the default again after the staged pass
+  if (!on && own && !e->staged) return MCX_OK;
+  if (mcx_status st = mcx_set_pass(e, on ? MCX_PASS_STAGED : MCX_PASS_MARCH)) return st;
+  e->form_auto = own;
+  if (!on) choose_form(e);
+  return MCX_OK;
 }
 
 extern "C" int mcx_get_staged(const mcx_engine *e) { return e && e->staged ? 1 : 0; }

@@ -44,3 +44,23 @@ def test_a_refused_form_leaves_the_one_before():
         with pytest.raises(mcx.McxError) as e:
             eng.pass_kind = "march_persistent"
         assert e.value.status == 4 and eng.pass_kind == before
+
+
+def test_staging_off_is_the_default_form():
+    with mcx.Engine([mcx.replica(nx=16, ny=16, nz=16)]) as eng:
+        assert eng.pass_kind == "resident"
+        eng.staged = False
+        assert eng.pass_kind == "resident"
+        eng.staged = True
+        assert eng.pass_kind == "staged"
+        eng.staged = False
+        assert eng.pass_kind == "resident"
+        eng.pass_kind = "direct"
+        eng.staged = False  # another pass was asked for
+        assert eng.pass_kind == "march"
+        eng.sweep(3)
+        eng.sync()
+    with mcx.Engine([mcx.replica(nx=16, ny=16, nz=16)]) as eng:
+        eng.set_march_shape(128, 8)
+        eng.staged = False
+        assert eng.pass_kind == "march"
