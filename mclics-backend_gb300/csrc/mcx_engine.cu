@@ -626,8 +626,9 @@ extern "C" mcx_status mcx_create(int n, const mcx_replica_desc *descs, mcx_engin
   for (int r = 0; r < n; r++) e->rep[r].ns_off = e->var.mask ? e->rep[r].dir_off : -1;
   {
     const char *nt = getenv("MCX_MARCH_NT"), *kk = getenv("MCX_MARCH_K"), *mo = getenv("MCX_MARCH");
-    if (nt && march_block_ok(atoi(nt))) e->march_nt = atoi(nt), e->shape_auto = false;
-    if (kk && atoi(kk) > 0) e->march_k = atoi(kk), e->shape_auto = false;
+    // a shape that is asked for: the z-march runs it (mcx_set_march_shape)
+    if (nt && march_block_ok(atoi(nt))) e->march_nt = atoi(nt), e->shape_auto = e->form_auto = false;
+    if (kk && atoi(kk) > 0) e->march_k = atoi(kk), e->shape_auto = e->form_auto = false;
     if (mo && atoi(mo) == 0) e->march = false;
     const char *pd = getenv("MCX_PDL");
     if (pd && atoi(pd) == 0) e->pdl = false;

@@ -64,3 +64,10 @@ def test_staging_off_is_the_default_form():
         eng.set_march_shape(128, 8)
         eng.staged = False
         assert eng.pass_kind == "march"
+
+
+@pytest.mark.parametrize("name,value", [("MCX_MARCH_NT", "64"), ("MCX_MARCH_K", "2")])
+def test_a_shape_from_the_environment_runs_the_march(name, value, monkeypatch):
+    monkeypatch.setenv(name, value)
+    with mcx.Engine([mcx.replica(nx=16, ny=16, nz=16)]) as eng:
+        assert eng.pass_kind == "march"
