@@ -1430,7 +1430,8 @@ extern "C" int mcx_get_staged(const mcx_engine *e) { return e && e->staged ? 1 :
 // order to the CTAs the GPU holds at once, finish first (a unit costs its
 // planes and about a third of a plane for its weights and set-up; a unit
 // without an active site nothing).  A fixed depth of 8 left the second of two
-// waves 58% idle on 4 x 96^3.
+// waves 58% idle on 4 x 96^3.  At most 32 planes: a thread's sums are FP32.
+constexpr int kLearnDeepest = 32;
 static int learn_depth(const mcx_engine *e, int nt, int slots) {
   if (tiny_batch(e)) return 8;
   int maxnz = 1;
@@ -1474,9 +1475,10 @@ static int learn_depth(const mcx_engine *e, int nt, int slots) {
   double best = 1e300;
   int best_d = 1;
   std::vector<double> busy;
-  for (int n = 1; n <= std::min(maxnz, 32); n++) {
+  const int n0 = (maxnz + kLearnDeepest - 1) / kLearnDeepest;
+  for (int n = n0; n <= std::min(maxnz, n0 + 31); n++) {
     const int d = (maxnz + n - 1) / n;
-    if (n > 1 && d == (maxnz + n - 2) / (n - 1)) continue;
+    if (n > n0 && d == (maxnz + n - 2) / (n - 1)) continue;
     // no schedule beats the work shared out evenly: most depths need no more
     double work = 0.0, end = 0.0;
     each(d, [&](double t) { work += t; });

@@ -268,9 +268,15 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
     }
   }
   grid_launch_dependents();
-  float qs[kQ];
+  // chunks deeper than 8 planes (32 at most, learn_depth): the warp's and the CTA's
+  // sums in two parts, which makes up for the thread's longer ones (energy of a
+  // sweep of 8 x LL 96^3, rms against FP64: 1.2e-9 of itself; 5.0e-9 with FP32
+  // sums, 2.9e-9 in chunks of 8 planes)
+  float qs[kQ], low[kQ];
   sums.fold(qs);
-  flush_replica<kLPB, MODE>(a, r, 1, (unsigned)R.lcta, acc, qs, MASK);
+#pragma unroll
+  for (int q = 0; q < kQ; q++) low[q] = 0.f;
+  flush_replica<kLPB, MODE>(a, r, 1, (unsigned)R.lcta, acc, qs, MASK, -1, -1, ke - kb > kLongPlanes ? low : nullptr);
   if (TC) {  // every TMEM read is done (tc_mlp ends on a fenced barrier; flush_replica syncs again)
     tc_fence_after();
     if (warp == 0) tc_dealloc(tmem, kLmarchTcCols);

@@ -51,9 +51,9 @@ __device__ __forceinline__ void march_plane(const PassArgs &a, const RepDev &R, 
 
 // The march of one unit's chunk of planes kb..ke-1 (everything after the
 // dependency wait).
-template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q>
+template <int POT, bool MASK, bool FIELD, int MODE, bool PER, class Q, class L>
 __device__ __forceinline__ void march_chunk(const PassArgs &a, const RepDev &R, int c, March &m, int kb, int ke,
-                                            const RepState *S, unsigned &acc, Q &sums) {
+                                            const RepState *S, unsigned &acc, Q &sums, L &all) {
   const int nz = R.nz;
   const bool zper = R.zb == BOUND_PERIODIC;
   const uint32_t seed = R.seed, stream = R.stream;
@@ -70,6 +70,7 @@ __device__ __forceinline__ void march_chunk(const PassArgs &a, const RepDev &R, 
   bool zm = zm0;
 #pragma unroll 1
   for (int k = kb; k < ke; k++) {
+    all.plane(k - kb, sums);
     const bool zp = k + 1 < nz || zper;
     const int up = k + 1 < nz ? 1 : 1 - nz;
     load_opair_at<MASK>(m, m.off + up * m.dz, m.offp + up * m.dzp, zp, op);
@@ -96,6 +97,9 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT, MODE>()) k
   unsigned acc = 0;
   PairSums<MASK> sums;
   sums.clear();
+  // masked batches' default chunks are not deep: four planes, or balanced ones of
+  // at most 300,000 sites
+  LongSums<MODE == MODE_SWEEP_MEASURE && !MASK> all(NT > 128 || (u.w & kUnitPlanes) > kLongPlanes);
   int slot = -1;  // the sweep's ring slot (measured passes)
   int p = u.y + (int)threadIdx.x;
   bool live = p < R.hp * R.ny;
@@ -120,17 +124,17 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT, MODE>()) k
       // no active site in or next to the unit: nothing to update
       if (a.idle_in_pass) dead_unit<FIELD, MODE>(R, m, kb, ke, sums);
     } else if (MASK && !ODD && (u.w & kUnitFull)) {  // only bulk sites around, every bond present: constant weights
-      march_chunk<POT, false, FIELD, MODE, true>(a, R, c, m, kb, ke, S, acc, sums);
+      march_chunk<POT, false, FIELD, MODE, true>(a, R, c, m, kb, ke, S, acc, sums, all);
     } else if (MASK && (u.w & kUnitBulk))  // only bulk sites around: the unmasked update
-      march_chunk<POT, false, FIELD, MODE, false>(a, R, c, m, kb, ke, S, acc, sums);
+      march_chunk<POT, false, FIELD, MODE, false>(a, R, c, m, kb, ke, S, acc, sums, all);
     else
-      march_chunk<POT, MASK, FIELD, MODE, PER>(a, R, c, m, kb, ke, S, acc, sums);
+      march_chunk<POT, MASK, FIELD, MODE, PER>(a, R, c, m, kb, ke, S, acc, sums, all);
   }
   grid_dependency_wait();    // threads without a pair reach here without having waited
   grid_launch_dependents();  // the next pass may start its set-up now
-  float qs[kQ];
-  sums.fold(qs);
-  flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, MASK, -1, slot);
+  float qs[kQ], low[kQ];
+  all.fold(sums, qs, low);
+  flush_replica<NT, MODE>(a, r, 1, (unsigned)R.mcta, acc, qs, MASK, -1, slot, all.on ? low : nullptr);
 }
 
 }  // namespace mcx

@@ -264,15 +264,52 @@ __device__ __forceinline__ float warp_sums(const float qs[kQ]) {
   return v[0] + __shfl_xor_sync(0xffffffffu, v[0], 1);
 }
 
+// (h, l) + (x, y), the rounding error of the high parts kept
+__device__ __forceinline__ void add_split(float &h, float &l, float x, float y) {
+  const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
+  l = __fadd_rn(__fadd_rn(l, y), __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b)));
+  h = s;
+}
+
+// warp_sums of values in two parts.
+__device__ __forceinline__ double warp_sums(const float qs[kQ], const float low[kQ]) {
+  const int lane = threadIdx.x & 31;
+  float h[8], l[8];
+#pragma unroll
+  for (int q = 0; q < 8; q++) {
+    h[q] = q < kQ ? qs[q] : 0.f;
+    l[q] = q < kQ ? low[q] : 0.f;
+  }
+#pragma unroll
+  for (int w = 4; w > 0; w >>= 1) {
+    const bool up = lane & (4 * w);
+#pragma unroll
+    for (int q = 0; q < w; q++) {
+      const float gh = __shfl_xor_sync(0xffffffffu, up ? h[q] : h[q + w], 4 * w);
+      const float gl = __shfl_xor_sync(0xffffffffu, up ? l[q] : l[q + w], 4 * w);
+      h[q] = up ? h[q + w] : h[q];
+      l[q] = up ? l[q + w] : l[q];
+      add_split(h[q], l[q], gh, gl);
+    }
+  }
+#pragma unroll
+  for (int d = 2; d > 0; d >>= 1)
+    add_split(h[0], l[0], __shfl_xor_sync(0xffffffffu, h[0], d), __shfl_xor_sync(0xffffffffu, l[0], d));
+  return (double)h[0] + (double)l[0];
+}
+
 // slot_pre: the ring slot if the caller read it early (ring_slot; -1: read
-// it here, at the end of the CTA, where its latency is exposed).
+// it here, at the end of the CTA, where its latency is exposed).  low: the low
+// parts of the sums (LongSums; null where qs is all of them).
 template <int NT, int MODE>
 __device__ __forceinline__ void flush_replica(const PassArgs &a, int r, int units, unsigned total, unsigned acc,
-                                              float qs[kQ], bool mask, int colour = -1, int slot_pre = -1) {
+                                              float qs[kQ], bool mask, int colour = -1, int slot_pre = -1,
+                                              const float *low = nullptr) {
   constexpr bool MEAS = MODE == MODE_SWEEP_MEASURE || MODE == MODE_MEASURE_ONLY;
   constexpr bool COUNT = MODE == MODE_SWEEP || MODE == MODE_SWEEP_MEASURE;
   __shared__ unsigned s_acc[NT / 32];
   __shared__ float s_q[NT / 32][kQ];
+  __shared__ double s_long[NT / 32][kQ];  // with low
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const RepDev &R = a.reps[r];
   RepState *S = a.st + r;
@@ -293,21 +330,32 @@ __device__ __forceinline__ void flush_replica(const PassArgs &a, int r, int unit
     if (lane == 0) s_acc[wid] = wa;
   }
   if (MEAS) {
-    const float v = warp_sums(qs);
-    if ((lane & 3) == 0 && lane < 4 * kQ) s_q[wid][lane >> 2] = v;
+    if (low) {
+      const double v = warp_sums(qs, low);
+      if ((lane & 3) == 0 && lane < 4 * kQ) s_long[wid][lane >> 2] = v;
+    } else {
+      const float v = warp_sums(qs);
+      if ((lane & 3) == 0 && lane < 4 * kQ) s_q[wid][lane >> 2] = v;
+    }
   }
   __syncthreads();
   if (MEAS && threadIdx.x < kQ) {
     const int lane_slot = blockIdx.x % kLanes;
     const int q = (!mask && threadIdx.x == 1) ? 0 : threadIdx.x;
-    float v = 0.f;
+    double v = 0.0;
+    if (low) {
+      for (int w2 = 0; w2 < NT / 32; w2++) v += s_long[w2][q];
+    } else {
+      float f = 0.f;
 #pragma unroll
-    for (int w2 = 0; w2 < NT / 32; w2++) v += s_q[w2][q];
+      for (int w2 = 0; w2 < NT / 32; w2++) f += s_q[w2][q];
+      v = f;
+    }
     const unsigned long long slot = MODE == MODE_MEASURE_ONLY ? (unsigned long long)a.ring_cap
                                     : slot_pre >= 0           ? (unsigned long long)slot_pre
                                                               : __ldcg(&S->meas) % (unsigned long long)a.ring_cap;
     double *ring = a.ring + (((size_t)r * (a.ring_cap + 1) + slot) * kLanes + lane_slot) * kQ;
-    atomicAdd(ring + threadIdx.x, (double)v);
+    atomicAdd(ring + threadIdx.x, v);
   }
   __syncwarp();  // warp 0's reads of the ring slot come before its thread 0 can end the sweep
   if (COUNT && threadIdx.x == 0) {

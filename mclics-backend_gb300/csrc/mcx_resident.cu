@@ -137,44 +137,18 @@ struct SplitSums {
   }
 };
 
-// (h, l) + (x, y), the rounding error of the high parts kept
-__device__ __forceinline__ void add_split(float &h, float &l, float x, float y) {
-  const float s = __fadd_rn(h, x), b = __fsub_rn(s, h);
-  l = __fadd_rn(__fadd_rn(l, y), __fadd_rn(__fsub_rn(h, __fsub_rn(s, b)), __fsub_rn(x, b)));
-  h = s;
-}
-
 // The warp's sums (warp_sums): quantity q in lane 4 q.
 template <bool MASKED>
 __device__ __forceinline__ double warp_split_sums(const SplitSums<MASKED> &t) {
-  const int lane = threadIdx.x & 31;
-  float h[8], l[8];
+  float h[kQ], l[kQ];
 #pragma unroll
-  for (int q = 0; q < 8; q++) {
-    h[q] = l[q] = 0.f;
-    if (q < kQ) {
-      const float2 a = unpk(t.hi[q]), b = unpk(t.lo[q]);
-      h[q] = a.x;
-      l[q] = b.x;
-      add_split(h[q], l[q], a.y, b.y);
-    }
+  for (int q = 0; q < kQ; q++) {
+    const float2 a = unpk(t.hi[q]), b = unpk(t.lo[q]);
+    h[q] = a.x;
+    l[q] = b.x;
+    add_split(h[q], l[q], a.y, b.y);
   }
-#pragma unroll
-  for (int w = 4; w > 0; w >>= 1) {
-    const bool up = lane & (4 * w);
-#pragma unroll
-    for (int q = 0; q < w; q++) {
-      const float gh = __shfl_xor_sync(0xffffffffu, up ? h[q] : h[q + w], 4 * w);
-      const float gl = __shfl_xor_sync(0xffffffffu, up ? l[q] : l[q + w], 4 * w);
-      h[q] = up ? h[q + w] : h[q];
-      l[q] = up ? l[q + w] : l[q];
-      add_split(h[q], l[q], gh, gl);
-    }
-  }
-#pragma unroll
-  for (int d = 2; d > 0; d >>= 1)
-    add_split(h[0], l[0], __shfl_xor_sync(0xffffffffu, h[0], d), __shfl_xor_sync(0xffffffffu, l[0], d));
-  return (double)h[0] + (double)l[0];
+  return warp_sums(h, l);
 }
 
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
