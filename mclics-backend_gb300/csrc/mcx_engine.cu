@@ -1627,12 +1627,12 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
   RepState *d_st = nullptr;
   double *d_stats = nullptr, *d_ring = nullptr;
   const size_t ring_n = (size_t)e->nrep * (e->ring_cap + 1) * kLanes * kQ;
-  cudaEvent_t t0, t1;
+  cudaEvent_t t0 = nullptr, t1 = nullptr;
   mcx_status st = MCX_OK;
-  int best_nt = e->march_nt, best_k = e->march_k,
-      best_form = e->resident ? 5 : (e->pmarch ? 3 : (e->tmarch ? 1 : (e->amarch ? 2 : (e->qmarch ? 4 : 0))));
+  const int was_nt = e->march_nt, was_k = e->march_k;
+  const bool was[] = {e->resident, e->pmarch, e->tmarch, e->amarch, e->qmarch};
+  int best_nt = was_nt, best_k = was_k, best_form = 0;
   float best = 1e30f;
-  e->resident = false;
 #define CKA(call)                                                                                    \
   do {                                                                                               \
     cudaError_t _r = (call);                                                                         \
@@ -1653,8 +1653,9 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
     const int nts[3] = {64, 128, 256};
     const int ks[10] = {1, 2, 4, 8, 16, 32, 0, -2, -3, -4};  // fixed depths, then balanced over 1..4 waves
     // forms: 0 the register march, 2 the per-thread prefetch, 4 four sites per
-    // thread (the TMA-staged form, 1, and the persistent one, 3, measured slower
-    // than these on every lattice and are not timed)
+    // thread (the TMA-staged and the persistent form measured slower than these on
+    // every lattice and are not timed), 5 resident
+    e->resident = false;
     for (int form : {0, 2, 4})
     for (int a = 0; a < 3; a++)
       for (int ki = 0; ki < 10; ki++) {
@@ -1698,8 +1699,9 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
           best_form = form;
         }
       }
-    // the resident form at its planned shape (its time includes a run's load
-    // and store of the lattice, over as many sweeps as above)
+    // the resident form at its planned shape, as a run of 32 sweeps: its time
+    // includes the run's launch and its load and store of the lattice, about 12 us
+    // (a march pass takes the same time in a run of any length)
     if (plan_resident(e) > 0.0) {
       PassArgs pa = pass_args(e);
       pa.dir = d_dir;
@@ -1726,21 +1728,23 @@ extern "C" mcx_status mcx_autotune(mcx_engine *e, int *block, int *planes, float
   }
   e->shape_auto = e->form_auto = false;
   e->resident = best_form == 5;
-  e->tmarch = best_form == 1;
   e->amarch = best_form == 2;
-  e->pmarch = best_form == 3;
   e->qmarch = best_form == 4;
   st = apply_march_shape(e, best_nt, best_k);
   if (st == MCX_OK) st = check_err_flag(e);
 done:
 #undef CKA
   cudaStreamSynchronize(e->stream);
+  if (st != MCX_OK) {  // the form and shape of before
+    e->resident = was[0] && e->res[0].c > 0, e->pmarch = was[1], e->tmarch = was[2], e->amarch = was[3], e->qmarch = was[4];
+    apply_march_shape(e, was_nt, was_k);
+  }
   cudaFree(d_dir);
   cudaFree(d_st);
   cudaFree(d_stats);
   cudaFree(d_ring);
-  cudaEventDestroy(t0);
-  cudaEventDestroy(t1);
+  if (t0) cudaEventDestroy(t0);
+  if (t1) cudaEventDestroy(t1);
   if (st == MCX_OK) {
     if (block) *block = best_nt;
     if (planes) *planes = best_k;

@@ -71,3 +71,13 @@ def test_a_shape_from_the_environment_runs_the_march(name, value, monkeypatch):
     monkeypatch.setenv(name, value)
     with mcx.Engine([mcx.replica(nx=16, ny=16, nz=16)]) as eng:
         assert eng.pass_kind == "march"
+
+
+@pytest.mark.parametrize("kind", ["march_persistent", "march_tma", "resident"])
+def test_the_autotuner_leaves_a_form_it_timed(kind):
+    with mcx.Engine([mcx.replica(nx=16, ny=16, nz=16)]) as eng:
+        eng.pass_kind = kind
+        eng.autotune()
+        assert eng.pass_kind in ("march", "march_async", "march_quad", "resident")
+        eng.sweep(20)
+        eng.sync()
