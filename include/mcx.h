@@ -244,11 +244,13 @@ int mcx_get_staged(const mcx_engine *eng);
  *                    in the shared memory of a cluster of 1 to 16 CTAs
  *                    (replicas up to about 40^3; MCX_ERR_UNSUPPORTED
  *                    otherwise).  The default of engines whose replicas are
- *                    small enough that it is estimated faster (and
- *                    have 1,200 active sites or more, 2,200 where
- *                    inactive sites have field energy);
- *                    mcx_set_march_shape returns to MCX_PASS_MARCH, which also
- *                    runs the single passes of mcx_pass_timing.
+ *                    small enough that it is estimated faster, and have
+ *                    1,200 active sites or more (2,200 where inactive sites
+ *                    have field energy); mcx_set_march_shape returns to
+ *                    MCX_PASS_MARCH, which also runs the single passes of
+ *                    mcx_pass_timing.  A run whose CTAs wait for a second in
+ *                    vain ends with MCX_ERR_CUDA from the next call that
+ *                    waits, the replica's state being that before the run.
  * No counterpart in the reference. */
 typedef enum {
   MCX_PASS_MARCH = 0,
@@ -267,15 +269,17 @@ int mcx_get_pass(const mcx_engine *eng);
  * so that the work units fill max(1, -planes) waves of the CTAs the GPU holds
  * at once).  The default is chosen from the batch's potential, masks and size
  * (balanced chunks of 128 or 256 threads; four planes in large masked batches;
- * 128 x 8 where a replica has some hundred active sites). */
+ * 128 x 8 where a replica has some hundred active sites), and again when
+ * mcx_set_mask or mcx_load changes the masks.  MCX_MARCH_NT and MCX_MARCH_K in
+ * the environment of mcx_create ask for a shape like this call. */
 mcx_status mcx_set_march_shape(mcx_engine *eng, int block, int planes);
 /* Autotuner: times the z-march pass (register form and, for unmasked batches,
  * the prefetching and four-site forms) for block sizes {64, 128, 256} and chunk
  * depths {1, 2, 4, ..., 32} (up to the deepest lattice) and balanced chunks
  * over 1 to 4 waves (planes 0, -2, -3, -4), and the resident form where it
  * runs, on a scratch copy of the engine's state (the state itself is
- * untouched), keeps the fastest and reports it (any output may be NULL; the
- * resident form reports the z-march shape that its short runs use).
+ * untouched), keeps the fastest and reports it (any output may be NULL; with
+ * the resident form, the z-march shape that mcx_pass_timing's passes use).
  * Synchronous. */
 mcx_status mcx_autotune(mcx_engine *eng, int *block, int *planes, float *pass_us);
 

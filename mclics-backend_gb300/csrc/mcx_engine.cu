@@ -345,9 +345,14 @@ static int unit_pairs(const mcx_engine *e) { return e->qmarch ? 2 * e->march_nt 
 
 static bool unit_dead(const mcx_engine *e, const int4 &u) { return unit_class(e, u, unit_pairs(e)) == kUnitDead; }
 
-// Flags of the z-march units.
+// Flags of the z-march units and of the learned z-march's units (which only
+// use kUnitDead).
 static void mark_dead_units(mcx_engine *e) {
   for (int4 &u : e->units) u.w = (u.w & (kUnitPlanes | kUnitTiled)) | unit_class(e, u, unit_pairs(e));
+  for (int4 &u : e->lunits) {
+    const int cls = unit_class(e, u, lmarch_block_threads());
+    u.w = (u.w & kUnitPlanes) | (cls == kUnitDead ? kUnitDead : 0);
+  }
 }
 
 // Plane runs of a replica for the z-march's chunks: maximal runs of planes k
@@ -912,13 +917,17 @@ extern "C" mcx_status mcx_set_mask(mcx_engine *e, int r, const int *pt, const fl
     }
   }
   // the z-march's shape and chunks follow the mask: plan them again (in
-  // mcx_create and mcx_load once, after every replica's mask); what only runs of
-  // sweeps need, before the next one (settle)
+  // mcx_create and mcx_load once, after every replica's mask); the form, the
+  // resident cuts and the learned units' depth, which any mask is right with, once
+  // before the next run of sweeps (settle)
   if (e->defer_plan) {
     mark_dead_units(e);
   } else if (mcx_status st = replan_march(e)) {
     return st;
   }
+  if (e->d_lunits && !e->lunits.empty())
+    CK(e, cudaMemcpyAsync(e->d_lunits, e->lunits.data(), sizeof(int4) * e->lunits.size(), cudaMemcpyHostToDevice,
+                          e->stream));
   e->stale = true;
   drop_graphs(e);
   CK(e, cudaStreamSynchronize(e->stream));
@@ -1234,9 +1243,13 @@ static void choose_form(mcx_engine *e) {
   e->resident = t > 0.0 && (!e->form_auto || (t < march_estimate(e) && !tiny_batch(e)));
 }
 
-// Plans again what depends on masks that were set since.
+// Plans again what depends on masks that were set since (not while the caller
+// captures the stream, where nothing can be waited for: the old plans run).
 static mcx_status settle(mcx_engine *e) {
   if (!e->stale) return MCX_OK;
+  cudaStreamCaptureStatus capturing = cudaStreamCaptureStatusNone;
+  CK(e, cudaStreamIsCapturing(e->stream, &capturing));
+  if (capturing != cudaStreamCaptureStatusNone) return MCX_OK;
   CK(e, cudaStreamSynchronize(e->stream));
   choose_form(e);
   if (e->d_lunits) {

@@ -79,3 +79,34 @@ def test_learned_units_follow_the_network_path(monkeypatch):
             eng.mlp_path = "tcgen05"
             assert own.mlp_path == eng.mlp_path == "tcgen05"
             _same(_measured(own, True), _measured(eng, True))
+
+
+@pytest.mark.parametrize("learned", [False, True])
+def test_a_captured_run_after_a_mask(learned):
+    """A caller that captures the engine's stream right after setting a mask: nothing
+    can be planned there, and the plans there are give the same chain."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("needs torch on the GPU")
+    got = []
+    for capture in (False, True):
+        with mcx.Engine(_descs("sphere", 24, 8.0, 2)) as own, mcx.Engine(_descs("custom", 24, 8.0, 2)) as eng:
+            eng.set_mlp(init_weights(3))
+            if learned:
+                eng.set_proposal("vmf_mlp")
+            for q in range(2):
+                eng.init_random(q, 5 + q)
+            eng.sweep(2)
+            for q in range(2):
+                eng.set_mask(q, *own.get_mask(q))
+            if capture:
+                stream = torch.cuda.ExternalStream(mcx.lib().mcx_stream(eng._h))
+                graph = torch.cuda.CUDAGraph()
+                with torch.cuda.graph(graph, stream=stream, capture_error_mode="relaxed"):
+                    eng.sweep(3)
+                graph.replay()
+                torch.cuda.synchronize()
+            else:
+                eng.sweep(3)
+            got.append([eng.get_state(q) for q in range(2)])
+    assert all(np.array_equal(x, y) for x, y in zip(*got))
