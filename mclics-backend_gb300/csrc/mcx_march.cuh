@@ -203,7 +203,14 @@ constexpr int march_min_blocks() {
   // more than the L1 cache holds for 16 warps (8 droplets of 96^3: 65.7 us a
   // pass against 71.4; unmeasured ones spill 120 bytes and are slower at 144 or
   // 168, 52.6 and 55.0 against 51.8)
+  // (LL in 256 threads at 128, two CTAs: 2 x 45x50x41 9.7 us a measured sweep
+  // against 13.5 at 194 registers, 4 slabs of 48x48x40 16.3 against 18.7)
+  if (POT == POT_LL && MASK && MODE == MODE_SWEEP_MEASURE && NT == 256) return 2;
   if (MASK && MODE == MODE_SWEEP_MEASURE) return 65536 / (NT * 168) > 0 ? 65536 / (NT * 168) : 1;
+  // measured LL passes at 128 registers too: at 96 their seven sums leave too few
+  // for loads ahead of the arithmetic (us a measured sweep, 128 against 96: 4 x 64^3
+  // in 128 x 8 19.0, 23.7; 4 x 96^3 in 128 x 8 39.4, 48.1; 16^3 in 64 x 4 7.9, 10.0)
+  if (POT == POT_LL && !MASK && MODE == MODE_SWEEP_MEASURE) return 65536 / (NT * 128);
   return POT == POT_LL && !MASK ? (NT == 64 ? 9 : (NT == 128 ? MCX_MARCH_LL128_BLOCKS : MCX_MARCH_LL256_BLOCKS))
                                 : (MCX_MARCH_MASK_REGS > 0 ? 65536 / (NT * MCX_MARCH_MASK_REGS) : 1);
 }

@@ -99,7 +99,9 @@ __global__ void __launch_bounds__(NT, march_min_blocks<POT, MASK, NT, MODE>()) k
   sums.clear();
   // masked batches' default chunks are not deep: four planes, or balanced ones of
   // at most 300,000 sites
-  LongSums<MODE == MODE_SWEEP_MEASURE && !MASK> all(NT > 128 || (u.w & kUnitPlanes) > kLongPlanes);
+  constexpr bool LONG = MODE == MODE_SWEEP_MEASURE && !MASK;
+  __shared__ float s_part[LONG ? 2 * kQ : 1][NT];
+  LongSums<LONG, NT> all(s_part, NT > 128 || (u.w & kUnitPlanes) > kLongPlanes);
   int slot = -1;  // the sweep's ring slot (measured passes)
   int p = u.y + (int)threadIdx.x;
   bool live = p < R.hp * R.ny;

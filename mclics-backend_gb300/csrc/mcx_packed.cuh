@@ -328,40 +328,34 @@ struct PairSums {
 };
 
 // A thread's sums over a chunk of many planes: every kLongPlanes the FP32 sums so
-// far move into high and low parts in local memory, and the warp's and the CTA's
+// far move into high and low parts, and the warp's and the CTA's
 // sums keep both parts.  Chunks of the default shape are up to a whole lattice
 // deep and 256 threads wide: with FP32 sums alone the energy of a sweep of 16 x
 // LL 96^3 (46 planes to a chunk, 19 CTAs to a replica) was 1.3e-8 of itself off
 // (rms), and 7e-9 on 8 x 64^3, against 2.2e-9 and 3.1e-9 in 128 threads x 8 planes;
 // so 4e-10.  Chunks of at most 128 threads x 8 planes keep the plain sums.
+// They lie in shared memory: stores to local or global memory would make the
+// compiler read the replica's constants again after them.
 constexpr int kLongPlanes = 8;
-template <bool USED>
+template <bool USED, int NT>
 struct LongSums {
-  float part[2 * kQ];
+  float (*part)[NT];  // [2 kQ][NT]
   bool on;
-  __device__ __forceinline__ explicit LongSums(bool deep) : on(USED && deep) {
+  __device__ __forceinline__ LongSums(float (*p)[NT], bool deep) : part(p), on(USED && deep) {
     if (!on) return;
-    float *p = at();
 #pragma unroll
-    for (int q = 0; q < 2 * kQ; q++) p[q] = 0.f;
-  }
-  // in memory, not in the registers that the planes between need
-  __device__ __forceinline__ float *at() {
-    float *p = part;
-    asm volatile("" : "+l"(p)::"memory");
-    return p;
+    for (int q = 0; q < 2 * kQ; q++) part[q][threadIdx.x] = 0.f;
   }
   // before plane `done` of the chunk
   template <class Q>
   __device__ __forceinline__ void plane(int done, Q &sums) {
     if (!USED || done == 0 || done % kLongPlanes != 0) return;
-    float *p = at();
 #pragma unroll
     for (int q = 0; q < kQ; q++) {
-      float h = p[q], l = p[kQ + q];
+      float h = part[q][threadIdx.x], l = part[kQ + q][threadIdx.x];
       add_split(h, l, sums.v[q], 0.f);
-      p[q] = h;
-      p[kQ + q] = l;
+      part[q][threadIdx.x] = h;
+      part[kQ + q][threadIdx.x] = l;
     }
     sums.clear();
   }
@@ -370,12 +364,11 @@ struct LongSums {
   __device__ __forceinline__ void fold(const Q &sums, float qs[kQ], float low[kQ]) {
     sums.fold(qs);
     if (!on) return;
-    const float *p = at();
 #pragma unroll
     for (int q = 0; q < kQ; q++) {
       const float v = qs[q];
-      qs[q] = p[q];
-      low[q] = p[kQ + q];
+      qs[q] = part[q][threadIdx.x];
+      low[q] = part[kQ + q][threadIdx.x];
       add_split(qs[q], low[q], v, 0.f);
     }
   }
