@@ -127,8 +127,16 @@ __device__ __forceinline__ void lds_opair(const float *slot, int nrO, int hs, in
   o.pt = 0x0101;
 }
 
+// Six CTAs of 128 threads per SM for LL (80 registers): the slots bring the rows,
+// so less is held than in k_march (4 x LL 96^3 in 128 x 8: 38.8 us a sweep, 47.7
+// with five)
+template <int POT, int NT>
+constexpr int tmarch_min_blocks() {
+  return POT == POT_LL && NT == 128 ? 6 : march_min_blocks<POT, false, NT>();
+}
+
 template <int POT, bool FIELD, int MODE, int NT, bool PER>
-__global__ void __launch_bounds__(NT, march_min_blocks<POT, false, NT>()) k_tmarch(PassArgs a) {
+__global__ void __launch_bounds__(NT, tmarch_min_blocks<POT, NT>()) k_tmarch(PassArgs a) {
   static_assert(MODE == MODE_SWEEP || MODE == MODE_SWEEP_MEASURE, "sweep modes only");
   extern __shared__ __align__(128) char smem[];
   __shared__ __align__(8) uint64_t bars[2];
