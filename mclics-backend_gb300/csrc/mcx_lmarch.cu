@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
             store_row(X, site_row(lane, 0), rA);  // words 10..15 are zeros that clear_row_tails wrote
             store_row(X, site_row(lane, 1), rB);
             __syncwarp();
-            mlp_warp(W, X, Y);
+            mlp_warp<2>(W, X, Y);
             __syncwarp();
             yA = reinterpret_cast<const float4 *>(Y)[site_row(lane, 0)];
             yB = reinterpret_cast<const float4 *>(Y)[site_row(lane, 1)];

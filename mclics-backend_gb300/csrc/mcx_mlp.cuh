@@ -129,13 +129,19 @@ __device__ __forceinline__ void ldsm_a4(const __nv_bfloat16 *X, int r0, int k0, 
 // kMT 16-row tiles go through the layers together: a weight or bias fragment
 // is read once for all of them, and their GELU chains (six dependent packed
 // operations each) overlap.  Every accumulator starts from the bias fragment
-// as the first MMA's C operand, so no register is filled for it.
-constexpr int kMT = 2;
+// as the first MMA's C operand, so no register is filled for it.  One tile at a
+// time reads two biases instead of their fragment, half the wavefronts.
+template <int kMT>
+__device__ __forceinline__ float4 bias_frag(const uint8_t *W, int c, int b, int nt, int tg) {
+  if (kMT > 1) return reinterpret_cast<const float4 *>(W + c)[nt * 4 + tg];
+  const float2 v = *reinterpret_cast<const float2 *>(W + b + (nt * 8 + 2 * tg) * 4);
+  return make_float4(v.x, v.y, v.x, v.y);
+}
+
+template <int kMT>
 __device__ __forceinline__ void mlp_warp(const uint8_t *W, const __nv_bfloat16 *X, float *Y) {
   const int lane = threadIdx.x & 31, g = lane >> 2, tg = lane & 3;
   const uint8_t *W1 = W + kMlpW1, *W2 = W + kMlpW2, *W3 = W + kMlpW3;
-  const float4 *c1 = reinterpret_cast<const float4 *>(W + kMlpC1) + tg;
-  const float4 *c2 = reinterpret_cast<const float4 *>(W + kMlpC2) + tg;
   const float *b3 = reinterpret_cast<const float *>(W + kMlpB3);
 #pragma unroll 1
   for (int mt = 0; mt < 4; mt += kMT) {
@@ -149,7 +155,8 @@ __device__ __forceinline__ void mlp_warp(const uint8_t *W, const __nv_bfloat16 *
       // layer 1: 2 k-tiles x 8 n-tiles
 #pragma unroll
       for (int q = 0; q < 4; q++) {
-        const float4 ca = c1[(2 * q) * 4], cb = c1[(2 * q + 1) * 4];
+        const float4 ca = bias_frag<kMT>(W, kMlpC1, kMlpB1, 2 * q, tg);
+        const float4 cb = bias_frag<kMT>(W, kMlpC1, kMlpB1, 2 * q + 1, tg);
         uint32_t bf[2][4];
         ldsm_b2(W1, kW1s, 16 * q, 0, bf[0]);
         ldsm_b2(W1, kW1s, 16 * q, 16, bf[1]);
@@ -175,7 +182,8 @@ __device__ __forceinline__ void mlp_warp(const uint8_t *W, const __nv_bfloat16 *
       for (int r = 0; r < 4; r++) y[t][r] = 0.f;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
-      const float4 ca = c2[(2 * q) * 4], cb = c2[(2 * q + 1) * 4];
+      const float4 ca = bias_frag<kMT>(W, kMlpC2, kMlpB2, 2 * q, tg);
+      const float4 cb = bias_frag<kMT>(W, kMlpC2, kMlpB2, 2 * q + 1, tg);
       float h[kMT][2][4];
 #pragma unroll
       for (int kt = 0; kt < 4; kt++) {

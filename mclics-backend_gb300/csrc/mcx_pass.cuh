@@ -789,7 +789,9 @@ __device__ __forceinline__ void compute_pair_learned(const PassArgs &a, int c, i
   write_features(X, site_row(lane, 0), nbA, wA, T, g.valid);
   write_features(X, site_row(lane, 1), nbB, wB, T, g.valid && g.hasB);
   __syncwarp();
-  mlp_warp(W, X, Y);
+  // two row tiles at a time spill here (44 to 112 bytes; 4 x LL 64^3 86.3 us a sweep
+  // against 85.5, a field droplet batch 137 against 132)
+  mlp_warp<1>(W, X, Y);
   __syncwarp();
   if (!g.valid) return;
   const float4 y0 = reinterpret_cast<const float4 *>(Y)[site_row(lane, 0)];

@@ -90,7 +90,7 @@ __global__ void __launch_bounds__(kTcThreads) k_mlp_warp(const uint8_t *mlp, con
       store_row(X, site_row(lane, h), w);
     }
     __syncwarp();
-    mlp_warp(W, X, Y);
+    mlp_warp<2>(W, X, Y);
     __syncwarp();
 #pragma unroll
     for (int h = 0; h < 2; h++) {
