@@ -58,14 +58,15 @@ struct Hood {
   uint8_t pex;
 };
 
-template <bool MASK>
+// CARRY: om and o0 are there already (the plane before's o0 and op).
+template <bool MASK, bool CARRY = false>
 __device__ __forceinline__ void load_hood(const March &m, int up, int down, bool zp, bool zm, Hood &h) {
   const int dx = m.s ? m.dx1 : m.dx0;
-  load_opair_at<MASK>(m, m.off, m.offp, true, h.o0);
+  if (!CARRY) load_opair_at<MASK>(m, m.off, m.offp, true, h.o0);
   load_opair_at<MASK>(m, m.off + m.dyp, m.offp + m.dypp, true, h.yp);
   load_opair_at<MASK>(m, m.off + m.dym, m.offp + m.dymp, true, h.ym);
   load_opair_at<MASK>(m, m.off + up * m.dz, m.offp + up * m.dzp, zp, h.op);
-  load_opair_at<MASK>(m, m.off - down * m.dz, m.offp - down * m.dzp, zm, h.om);
+  if (!CARRY) load_opair_at<MASK>(m, m.off - down * m.dz, m.offp - down * m.dzp, zm, h.om);
   h.ex[0] = ldo1(m.O0 + m.off + dx);
   h.ex[1] = ldo1(m.O1 + m.off + dx);
   h.ex[2] = ldo1(m.O2 + m.off + dx);
@@ -204,6 +205,12 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
   } else {
     const unsigned long long sw = S->sweep;
     const float T = S->T, invT = 1.0f / S->T;
+    Hood h;
+    if (TC) {
+      const int down = kb > 0 ? 1 : 1 - nz;
+      load_opair_at<MASK>(m, m.off - down * m.dz, m.offp - down * m.dzp, kb > 0 || zper, h.om);
+      load_opair_at<MASK>(m, m.off, m.offp, true, h.o0);
+    }
 #pragma unroll 1
     for (int k = kb; k < ke; k++) {
       const bool zp = k + 1 < nz || zper, zm = k > 0 || zper;
@@ -217,8 +224,7 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
       if (!(idle && (MODE == MODE_SWEEP || (c == 0 && !(FIELD && a.idle_in_pass))))) {
         float4 yA = make_float4(0.f, 0.f, 0.f, 0.f), yB = yA;
         if (!idle) {
-          Hood h;
-          load_hood<MASK>(m, up, down, zp, zm, h);
+          load_hood<MASK, TC>(m, up, down, zp, zm, h);
           const PairSlots sl = hood_slots<MASK, PER>(m, h, pself, zp, zm);
           uint32_t rA[16], rB[16];
           pair_features(sl, T, valid, valid && (PER || m.hasB), rA, rB);
@@ -245,10 +251,12 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
           }
         }
         if (valid) {
-          // the neighbourhood again: held in registers across the network it
-          // would cost the network its second row tile (spills)
-          Hood h;
-          load_hood<MASK>(m, up, down, zp, zm, h);
+          // the neighbourhood again: held in registers across the warp's network
+          // it would cost the network its second row tile (spills).  The tensor
+          // cores' network needs few registers, and its CTAs have 168 per thread:
+          // held there, with the z reuse of the march (4 x LL 96^3 at one shape 259 us
+          // a sweep; 317 with the second reading)
+          if (!TC) load_hood<MASK>(m, up, down, zp, zm, h);
           float2 ax = *reinterpret_cast<const float2 *>(m.A0 + m.off);
           float2 ay = *reinterpret_cast<const float2 *>(m.A1 + m.off);
           float2 az = *reinterpret_cast<const float2 *>(m.A2 + m.off);
@@ -260,6 +268,10 @@ __global__ void __launch_bounds__(kLPB, TC ? 3 : MCX_LMARCH_MIN_BLOCKS) k_lmarch
           *reinterpret_cast<float2 *>(m.A1 + m.off) = ay;
           *reinterpret_cast<float2 *>(m.A2 + m.off) = az;
         }
+      }
+      if (TC) {
+        h.om = h.o0;
+        h.o0 = h.op;
       }
       m.off += m.dz;
       m.offp += m.dzp;
@@ -312,6 +324,21 @@ int lmarch_block_threads() { return kLPB; }
 
 int lmarch_blocks_per_sm(const Variant &v, bool tc) {
   int n = 0;
+  if (tc) {
+    // the occupancy call answers 1 for a kernel that allocates tensor memory;
+    // registers, shared memory and TMEM columns hold three such CTAs
+    cudaFuncAttributes f;
+    int dev = 0, smem = 0, regs = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || cudaFuncGetAttributes(&f, lmarch_kernel(v, MODE_SWEEP, tc)) != cudaSuccess ||
+        cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&regs, cudaDevAttrMaxRegistersPerMultiprocessor, dev) != cudaSuccess)
+      return 0;
+    const int per_cta = (f.numRegs + 7) / 8 * 8 * kLPB;  // registers come in blocks of 8 a thread
+    n = smem / (lmarch_smem(tc) + (int)f.sharedSizeBytes + 1024);  // 1 KB of each CTA's is the system's
+    if (regs / per_cta < n) n = regs / per_cta;
+    if (512 / (int)kLmarchTcCols < n) n = 512 / (int)kLmarchTcCols;
+    return n;
+  }
   if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, lmarch_kernel(v, MODE_SWEEP, tc), kLPB, lmarch_smem(tc)) !=
       cudaSuccess)
     return 0;
