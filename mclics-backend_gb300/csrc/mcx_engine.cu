@@ -71,6 +71,11 @@ struct mcx_engine {
   // both come back under one wait
   double *h_out = nullptr;
   std::mutex out_mutex;
+  // a replica's directors or normals and point types on their way to a
+  // checkpoint: kept, because fresh memory of that size costs more in page
+  // faults than the copies (2 droplets of 96^3: 11.6 ms a save against 1.7)
+  std::vector<float> save_ni;
+  std::vector<int> save_pt;
   // learned proposal
   int proposal = MCX_PROPOSAL_PLAIN;
   uint8_t *d_mlp = nullptr;
@@ -2091,14 +2096,16 @@ extern "C" mcx_status mcx_save(mcx_engine *e, const char *path) {
   for (int r = 0; r < e->nrep && ok; r++) {
     const RepDev &R = e->rep[r];
     CkptState cs{st[r].T, st[r].ang_var, st[r].sweep, st[r].meas, st[r].frozen, 0u};
-    std::vector<float> ni(3 * (size_t)R.ntot);
+    std::vector<float> &ni = e->save_ni;
+    ni.resize(3 * (size_t)R.ntot);
     if (mcx_status s2 = mcx_get_state(e, r, ni.data())) return s2;
     ok = fwrite(&e->desc[r], sizeof(mcx_replica_desc), 1, fc.f) == 1 && fwrite(&cs, sizeof cs, 1, fc.f) == 1 &&
          fwrite(stats.data() + (size_t)kStats * r, sizeof(double), kStats, fc.f) == (size_t)kStats &&
          fwrite(ni.data(), sizeof(float), ni.size(), fc.f) == ni.size();
     if (ok && e->var.mask) {
-      std::vector<int> pt(R.ntot);
-      std::vector<float> ns(3 * (size_t)R.ntot);
+      std::vector<int> &pt = e->save_pt;
+      std::vector<float> &ns = e->save_ni;  // the directors are written
+      pt.resize(R.ntot);
       if (mcx_status s2 = mcx_get_mask(e, r, pt.data(), ns.data())) return s2;
       ok = fwrite(pt.data(), sizeof(int), pt.size(), fc.f) == pt.size() &&
            fwrite(ns.data(), sizeof(float), ns.size(), fc.f) == ns.size();
