@@ -1189,6 +1189,7 @@ static double plan_resident(mcx_engine *e) {
   double best[2] = {1e30, 1e30};
   std::vector<int> cut, keep[2];
   for (auto &r : e->res) r.c = 0;
+  if (!resident_prepare(e->var)) return 0.0;
   for (int C : {1, 2, 4, 8, 16}) {
     if (C > minz) break;  // a CTA's rows span at least one plane
     long long smem = 0;
@@ -1244,8 +1245,10 @@ static double plan_resident(mcx_engine *e) {
 // the z-march.  A form that was asked for stays, with cuts for the present masks.
 static void choose_form(mcx_engine *e) {
   if (!e->march || e->staged || !(e->form_auto || e->resident)) return;
+  e->resident = !(e->form_auto && tiny_batch(e));
+  if (!e->resident) return;
   const double t = plan_resident(e);
-  e->resident = t > 0.0 && (!e->form_auto || (t < march_estimate(e) && !tiny_batch(e)));
+  e->resident = t > 0.0 && (!e->form_auto || t < march_estimate(e));
 }
 
 // Plans again what depends on masks that were set since (not while the caller

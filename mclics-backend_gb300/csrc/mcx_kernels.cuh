@@ -147,6 +147,7 @@ cudaError_t launch_pmarch(const Variant &v, int mode, const PassArgs &a, int nt,
 long long resident_smem_bytes(const RepDev &R, bool mask, int n);
 int resident_max_threads(bool mask, int mode);
 constexpr int kResidentSmem = 220 * 1024;  // dynamic shared memory of a CTA, below the 227 KB limit
+bool resident_prepare(const Variant &v);  // before the two below
 int resident_clusters(const Variant &v, int mode, int C, int nt, int smem);
 // limit: nanoseconds a wait may take; extra: bytes that each sweep waits for in
 // vain (a test of the limit).

@@ -593,18 +593,29 @@ static void res_config(cudaLaunchConfig_t &cfg, cudaLaunchAttribute &at, int nre
   cfg.numAttrs = 1;
 }
 
+// Sets the kernels' attributes: the largest values any engine uses, because they
+// belong to the kernel.
+bool resident_prepare(const Variant &v) {
+  for (int mode : {MODE_SWEEP, MODE_SWEEP_MEASURE}) {
+    const void *fn = res_kernel(v, mode);
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem) != cudaSuccess ||
+        cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+  }
+  return true;
+}
+
 // Clusters of C CTAs of nt threads with smem bytes the GPU holds at once (0:
-// the shape cannot run); sets the kernel's attributes.
+// the shape cannot run).
 int resident_clusters(const Variant &v, int mode, int C, int nt, int smem) {
   const void *fn = res_kernel(v, mode);
-  // the largest values any engine uses: the attributes belong to the kernel
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute at;
   res_config(cfg, at, 1, C, nt, smem, nullptr);
   int n = 0;
-  if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kResidentSmem) != cudaSuccess ||
-      cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+  if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
     cudaGetLastError();
     return 0;
   }
