@@ -10,10 +10,12 @@
 // so the bond sums, the rotation and the energy change take half the
 // instructions.  Measured per pass, scalar -> packed: LL 128^3 10.0 -> 8.95 us
 // (autotuned shape), 16 x LL 96^3 59.3 -> 55.8 us, 48 GHRL slabs of 16^3 to
-// 64^3 35.2 -> 26.4 us, 8 droplets of 96^3 67.3 -> 61.4 us.  Each half of a packed operation is rounded as the scalar
-// operation (round to nearest even, denormals kept), so with the operations
-// of site_update (mcx_pass.cuh) in their order the results are the same bits;
-// the direct pass keeps the scalar form and the tests compare the two bit for
+// 64^3 35.2 -> 26.4 us, 8 droplets of 96^3 67.3 -> 61.4 us.
+//
+// Each half of a packed operation is rounded as the scalar operation (round to
+// nearest even, denormals kept), so with the operations of site_update
+// (mcx_pass.cuh) in their order the results are the same bits; the direct pass
+// keeps the scalar form and the tests compare the two bit for
 // bit.
 #pragma once
 #include <cuda_runtime.h>
